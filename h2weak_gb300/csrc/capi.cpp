@@ -86,6 +86,17 @@ template <class T> struct GmbStore {
 
 inline int64_t pad4(int64_t x) { return (x + 3) & ~int64_t(3); }
 
+// A single-vector target stream on the device, as sv.cu's launch takes it
+struct SvStream {
+    DBuf<SvHdr> hdr;
+    DBuf<uint32_t> idx, cons;
+    DBuf<uint2> grp;
+    DBuf<int32_t> cnt, rem, ctr;
+    int32_t list[3][2] = {{0, 0}, {0, 0}, {0, 0}};  // target ranges of the three lists
+    int32_t share = 0, ngrp = 0;                    // list 0's part of lists 0 and 1, thousandths
+    SvConf f64, f32;
+};
+
 constexpr int XW_CAP = 4096;          // gathered source width per target (elements)
 constexpr int64_t ROW_SPLIT = 16384;  // rows * width above which a target is split (load balance)
 constexpr int64_t MR_ROWS = 64;      // rows per target of the multi-vector stream (its result tile)
@@ -119,6 +130,7 @@ struct h2w_handle {
     double diag_im = 0;
     DBuf<double2> c_V, c_w, c_r, c_ax, c_part, c_h, c_y;  // complex GMRES state
     int64_t nv() const { return cplx ? 2 * tree.N : tree.N; }  // doubles per vector
+    int64_t xoff() const { return pad4(ws_n); }  // the input in leaf order behind the workspace rows
     // device state
     DBuf<double> d_pts;
     DBuf<int32_t> d_perm;
@@ -132,13 +144,17 @@ struct h2w_handle {
     DBuf<float> d_op32m;
     DBuf<int64_t> d_blob_mw, d_mslices;
     int64_t op32m_n = 0;
-    // the same for the single-vector stream's FP32 products: each (target, panel)
-    // slice of the FP32 operator contiguous at its padded height, so that a row
-    // chunk of a block streams whole sectors (made on the first FP32 product)
+    // the single-vector dataflow launch: its stream and its operator copies (each target's
+    // panels side by side as one contiguous matrix at its padded height; FP64 made with
+    // the operator, FP32 on the first product of that precision)
     DBuf<float> d_op32s;
-    DBuf<int64_t> d_blob_s, d_sslices;
-    int64_t op32s_n = 0;
-    bool op32s_ready = false;
+    DBuf<double> d_op64s;
+    DBuf<int64_t> d_sslices;
+    int64_t ops_n = 0;
+    bool op32s_ready = false, op64s_ready = false;
+    SvStream sv;
+    int32_t sv_split = 0;   // list 0: end of the upward passes
+    bool fused_sv = true;
     bool op32m_ready = false;
     DBuf<int32_t> d_mctr;                           // its per-phase target counters
     std::vector<Phase> mphases;
@@ -199,8 +215,6 @@ struct h2w_handle {
     bool producer_warp = true;  // the FP32 dataflow product's warp-specialised form (H2W_OPT_PRODUCER_WARP)
     DBuf<int32_t> d_mdep0, d_mdep, d_mcidx;
     DBuf<int64_t> d_mcoff;
-    DBuf<int32_t> d_sdep0, d_sdep, d_scidx, d_sctr;  // the same for the single-vector stream
-    DBuf<int64_t> d_scoff;
     int64_t mflow_edges = 0;
     // multi-vector plan: targets, panels, operator entries per column, entries
     // the kernel multiplies (rows to warp granularity, each panel's columns to
@@ -1244,6 +1258,7 @@ struct PlanBuilder {
     // row chunks of max(min_rows, row_split / width) rows (multiples of 4)
     int64_t row_split = ROW_SPLIT;
     int64_t min_rows = 4;
+    int64_t max_rows = INT32_MAX;
     int64_t xw_cap = XW_CAP;  // gathered columns per target before a column split
     bool fused = true;        // no leaf (scatter) target was column-split
 
@@ -1318,7 +1333,7 @@ struct PlanBuilder {
         logical.push_back({dst, nrows, flags, panels, lo, hi});
     }
     // Realise the logical targets with the given split parameters into T/P/S/win.
-    void realize(int64_t rs, int64_t mr, int64_t cap) {
+    void realize(int64_t rs, int64_t mr, int64_t cap, int64_t rows_cap = INT32_MAX) {
         T.clear();
         P.clear();
         S.clear();
@@ -1326,6 +1341,7 @@ struct PlanBuilder {
         row_split = rs;
         min_rows = mr;
         xw_cap = cap;
+        max_rows = rows_cap;
         fused = true;
         for (const LTarget &l : logical) {
             lo = l.lo;
@@ -1344,7 +1360,7 @@ struct PlanBuilder {
             // row chunks are multiples of 4 rows so the kernel's 16-byte column loads stay aligned
             int64_t rows_per =
                 std::max<int64_t>(min_rows, (row_split / std::max<int64_t>(xw, 1)) & ~int64_t(3));
-            rows_per = std::min<int64_t>(rows_per, nrows);
+            rows_per = std::min<int64_t>(std::min(rows_per, max_rows), nrows);
             for (int64_t r0 = 0; r0 < nrows; r0 += rows_per) {
                 int32_t nr = (int32_t)std::min<int64_t>(rows_per, nrows - r0);
                 Target tg{};
@@ -1375,10 +1391,15 @@ struct PlanBuilder {
             }
             return;
         }
-        // column split, atomically accumulated sub-targets: whole panels in
-        // groups of <= xw_cap gathered columns (as many groups as the width
-        // needs, filled evenly), panels wider than xw_cap in chunks of xw_cap
+        // column split, atomically accumulated sub-targets
         if (flags & T_SCATTER) fused = false;
+        for (const auto &part : column_parts(panels)) split(dst, nrows, T_ATOMIC, part);
+    }
+    // The panels in groups of at most xw_cap gathered columns: whole panels (as many
+    // groups as the width needs, filled evenly), panels wider than xw_cap in
+    // chunks of xw_cap
+    std::vector<std::vector<PanelSpec>> column_parts(const std::vector<PanelSpec> &panels) const {
+        std::vector<std::vector<PanelSpec>> out;
         int64_t narrow = 0;
         for (auto &p : panels)
             if (pad4(p.w) <= xw_cap) narrow += pad4(p.w);
@@ -1389,14 +1410,14 @@ struct PlanBuilder {
             for (auto &p : panels) {
                 if (pad4(p.w) > xw_cap) continue;
                 if (!grp.empty() && (gw + pad4(p.w) > xw_cap || gw >= share)) {
-                    split(dst, nrows, T_ATOMIC, grp);
+                    out.push_back(grp);
                     grp.clear();
                     gw = 0;
                 }
                 grp.push_back(p);
                 gw += pad4(p.w);
             }
-            if (!grp.empty()) split(dst, nrows, T_ATOMIC, grp);
+            if (!grp.empty()) out.push_back(grp);
         }
         for (auto &p : panels) {
             if (pad4(p.w) <= xw_cap) continue;
@@ -1416,9 +1437,10 @@ struct PlanBuilder {
                     ns.xoff = (int32_t)(lo - c0);
                     q.segs.push_back(ns);
                 }
-                split(dst, nrows, T_ATOMIC, {q});
+                out.push_back({q});
             }
         }
+        return out;
     }
 };
 
@@ -1700,6 +1722,317 @@ void build_deps(const PlanBuilder &pb, int64_t ws_n, std::vector<int32_t> &cnt, 
         for (int32_t u : prod[t]) cidx[(size_t)fill[(size_t)u]++] = (int32_t)t;
 }
 
+// The panels of a record stream moved to slices of their own: the panels of a
+// target one after another, each column-major at pad4(nrows), so a target is one
+// contiguous matrix. Rewrites the records; appends the slices to copy (6 words
+// each: source offset, lda, rows, width, offset, lda) and returns the end offset.
+int64_t slice_records(const std::vector<int64_t> &roff, std::vector<int64_t> &blob, std::vector<int64_t> &sl, int64_t off) {
+    for (size_t t = 0; t + 1 < roff.size(); ++t) {
+        const size_t o = (size_t)roff[t];
+        const int64_t nrows = blob[o + 1] & 0xffffffff, np = blob[o + 2] & 0xffffffff, ld = pad4(nrows);
+        for (int64_t q = 0; q < np; ++q) {
+            const size_t wa = o + 3 + 3 * (size_t)q, wl = wa + 1;
+            const int64_t a = blob[wa], lda = blob[wl] & 0xffffffff, w = blob[wl] >> 32;
+            sl.insert(sl.end(), {a, lda, nrows, w, off, ld});
+            blob[wa] = off;
+            blob[wl] = (int64_t)(uint32_t)ld | (w << 32);
+            off += ld * w;
+        }
+    }
+    return off;
+}
+
+// The dataflow stream of one operator's single-vector product (sv.cu) on the host:
+// its targets in dependency order, with the list, deadline and work that order them
+// in a launch, and its groups.
+struct SvHost {
+    std::vector<SvHdr> hdr;
+    std::vector<int32_t> list, key;  // key: deadline, then the place among the parts of a block row
+    std::vector<double> work;        // elements of the target's block row
+    std::vector<uint32_t> idx, cons;
+    std::vector<uint2> grp;
+    std::vector<int32_t> cnt;
+    std::vector<int64_t> slices;  // operator pieces to copy (slice_records)
+    int64_t opn = 0;
+    int max_w = 1;
+    bool fused = true;  // the leaf pass writes the result itself
+};
+
+// Producers of the groups, in their order: as build_deps, with all targets of a group
+// taken together and no atomic writers. parts[g]: targets of group g.
+void group_deps(const std::vector<PlanBuilder::LTarget> &groups, const std::vector<int32_t> &parts, int64_t ws_n,
+                SvHost &out) {
+    const size_t ng = groups.size();
+    std::vector<int32_t> last((size_t)ws_n, -1);
+    std::vector<std::vector<int32_t>> rd((size_t)ws_n), prod(ng);
+    std::vector<int32_t> deps;
+    std::vector<uint32_t> ncons(ng, 0);
+    out.cnt.assign(ng, 0);
+    for (size_t g = 0; g < ng; ++g) {
+        const PlanBuilder::LTarget &l = groups[g];
+        const bool scatter = l.flags & T_SCATTER, accum = l.flags & T_ACCUM;
+        deps.clear();
+        auto for_reads = [&](auto &&f) {
+            for (const PlanBuilder::PanelSpec &pn : l.panels)
+                for (const Seg &sg : pn.segs)
+                    if (!(sg.flags & S_GATHER))
+                        for (int64_t r = sg.src; r < sg.src + sg.len; ++r) f((size_t)r);
+            if (accum)
+                for (int64_t r = l.dst; r < l.dst + l.nrows; ++r) f((size_t)r);
+        };
+        auto add = [&](int32_t u) {
+            if (u >= 0 && (deps.empty() || deps.back() != u)) deps.push_back(u);
+        };
+        for_reads([&](size_t r) { add(last[r]); });
+        if (!scatter)
+            for (int64_t r = l.dst; r < l.dst + l.nrows; ++r) {
+                add(last[(size_t)r]);
+                for (int32_t u : rd[(size_t)r]) add(u);
+            }
+        std::sort(deps.begin(), deps.end());
+        deps.erase(std::unique(deps.begin(), deps.end()), deps.end());
+        prod[g] = deps;
+        for_reads([&](size_t r) {
+            if (rd[r].empty() || rd[r].back() != (int32_t)g) rd[r].push_back((int32_t)g);
+        });
+        if (!scatter)
+            for (int64_t r = l.dst; r < l.dst + l.nrows; ++r) {
+                last[(size_t)r] = (int32_t)g;
+                rd[(size_t)r].clear();
+            }
+        for (int32_t u : prod[g]) {
+            out.cnt[g] += parts[(size_t)u];
+            ++ncons[(size_t)u];
+        }
+    }
+    out.grp.resize(ng);
+    uint32_t at = 0;
+    for (size_t g = 0; g < ng; ++g) {
+        out.grp[g] = make_uint2(at, 0);
+        at += ncons[g];
+    }
+    out.cons.resize(at);
+    for (size_t g = 0; g < ng; ++g)
+        for (int32_t u : prod[g]) out.cons[out.grp[(size_t)u].x + out.grp[(size_t)u].y++] = (uint32_t)g;
+}
+
+// Cut the logical targets for the dataflow launch. Each pass is cut for the whole
+// chip: its elements over SV_CUT_CTAS, at most row_split and at least SV_CUT_MIN a
+// target, so that a pass of a few large blocks near the root is not left to a few SMs
+// (an FP64 target of 16384 elements takes one SM's FP64 pipe 4 us). Large operators
+// have whole rows to spare and keep at least 8, 16 or 32 rows a target: its sources are
+// gathered once for all its rows (3D semi-nested, 2e8 entries, FP32: 262 us at 4 rows,
+// 196 at 16, 166 at 32). A block row wider than XW_CAP is cut into column parts, each
+// adding to the rows of the one before: the sums come in the same order on every run.
+constexpr int64_t SV_CUT_CTAS = 608, SV_CUT_MIN = 2048;
+void sv_build(h2w_handle *h, int64_t row_split, int32_t pid, int64_t ws0, int64_t x0, int64_t xoff, SvHost &out) {
+    auto bad = [](const char *what) { throw ApiError(H2W_ERR_STATE, std::string("internal: single-vector stream: ") + what); };
+    PlanBuilder &pb = *h->plan;
+    const int last = h->nph_total - 1;
+    // list 0: the passes that depend on one another; 1: near field and pair rows, from the input alone;
+    // 2: the leaf pass
+    auto list_of = [&](const PlanBuilder::LTarget &l) { return l.lo == last ? 2 : (l.lo == 0 && l.hi == last - 1) ? 1 : 0; };
+    auto elems = [](const PlanBuilder::LTarget &l) {
+        double w = 0;
+        for (const auto &p : l.panels) w += p.w;
+        return w * l.nrows;
+    };
+    pb.T.clear();
+    pb.P.clear();
+    pb.S.clear();
+    pb.win.clear();
+    pb.fused = true;
+    pb.xw_cap = XW_CAP;
+    pb.max_rows = SV_MAX_ROWS;
+    std::vector<PlanBuilder::LTarget> groups;
+    struct Key { int list, hi, part; double work; };
+    std::vector<Key> key;
+    double pass[3][2 * 64] = {}, all = 0;
+    for (const auto &l : pb.logical) {
+        int64_t xw = 0;
+        for (const auto &p : l.panels) xw += pad4(p.w);
+        if (xw == 0 || l.nrows <= 0) continue;
+        const double w = elems(l);
+        const int ls = list_of(l);
+        all += w;
+        pass[ls][std::min(l.hi, 127)] += w;
+        if (ls == 1)
+            for (const auto &p : l.panels)
+                for (const Seg &sg : p.segs)
+                    if (!(sg.flags & S_GATHER)) bad("a free target reads the workspace");
+        if (xw <= XW_CAP) {
+            groups.push_back(l);
+            key.push_back({ls, l.hi, 0, w});
+            continue;
+        }
+        const auto parts = pb.column_parts(l.panels);
+        for (size_t i = 0; i < parts.size(); ++i) {
+            groups.push_back({l.dst, l.nrows, i + 1 < parts.size() ? (int32_t)T_ACCUM : l.flags, parts[i], l.lo, l.hi});
+            key.push_back({ls, l.hi, (int)i, w});
+        }
+    }
+    {
+        std::vector<size_t> ord(groups.size());
+        for (size_t i = 0; i < ord.size(); ++i) ord[i] = i;
+        std::stable_sort(ord.begin(), ord.end(), [&](size_t a, size_t b) {
+            const Key &p = key[a], &q = key[b];
+            if (p.list != q.list) return p.list < q.list;
+            if (p.hi != q.hi) return p.hi < q.hi;
+            if (p.part != q.part) return p.part < q.part;
+            return p.work > q.work;
+        });
+        std::vector<PlanBuilder::LTarget> g2;
+        std::vector<Key> k2;
+        for (size_t i : ord) {
+            g2.push_back(std::move(groups[i]));
+            k2.push_back(key[i]);
+        }
+        groups.swap(g2);
+        key.swap(k2);
+    }
+    const int64_t rows_min = all >= 128e6 ? 32 : all >= 64e6 ? 16 : all >= 16e6 ? 8 : 4;
+    std::vector<int32_t> parts(groups.size());
+    int64_t covered = 0;
+    for (const auto &l : groups)
+        if (l.flags & T_SCATTER) covered += l.nrows;
+    out.fused = covered == h->nv();  // else an explicit scatter follows
+    for (size_t g = 0; g < groups.size(); ++g) {
+        auto &l = groups[g];
+        if (!out.fused && (l.flags & T_SCATTER)) l.flags = T_ACCUM;
+        const int64_t share = (int64_t)(pass[key[g].list][std::min(l.hi, 127)] / SV_CUT_CTAS);
+        pb.row_split = std::min(row_split, std::max(SV_CUT_MIN, share));
+        pb.min_rows = rows_min;
+        const size_t t0 = pb.T.size();
+        pb.split(l.dst, l.nrows, l.flags, l.panels);
+        parts[g] = (int32_t)(pb.T.size() - t0);
+        for (size_t t = t0; t < pb.T.size(); ++t) {
+            out.list.push_back(key[g].list);
+            out.key.push_back(l.hi * 4096 + std::min(key[g].part, 4095));
+            out.work.push_back(key[g].work);
+            SvHdr d{};
+            d.grp = (uint32_t)g;
+            d.pid = (uint32_t)pid;
+            out.hdr.push_back(d);
+        }
+    }
+    validate_plan(pb, h, {});
+    std::vector<int64_t> roff, blob, pstart;
+    pack_records(pb, {}, roff, blob, pstart);
+    first_writers_overwrite(roff, blob, h->ws_n, h->fly_active ? &h->fly_rows : nullptr);
+    group_deps(groups, parts, h->ws_n, out);
+    out.opn = slice_records(roff, blob, out.slices, 0);
+    // headers; targets of a group that read the same sources share the list of rows.
+    // Every value the kernel indexes with is checked against its field.
+    std::vector<uint32_t> rows, prev;
+    uint32_t prev0 = 0;
+    for (size_t t = 0; t + 1 < roff.size(); ++t) {
+        const size_t o = (size_t)roff[t];
+        const int64_t nrows = blob[o + 1] & 0xffffffff, fl = blob[o + 1] >> 32;
+        const int64_t np = blob[o + 2] & 0xffffffff, ns = blob[o + 2] >> 32;
+        if (np < 1 || nrows < 1 || nrows > SV_MAX_ROWS) bad("target shape");
+        SvHdr &d = out.hdr[t];
+        d.a = blob[o + 3];
+        d.dst = (uint32_t)(ws0 + blob[o]);
+        d.nrows = (uint16_t)nrows;
+        if (fl & T_ATOMIC) bad("an atomic target");
+        d.flags = (uint16_t)(fl & (T_ACCUM | T_SCATTER));
+        rows.clear();
+        int64_t W = 0, e = 0;
+        for (int64_t q = 0; q < np; ++q) {  // padded panel offsets become columns of the one matrix
+            const int64_t w = blob[o + 4 + 3 * (size_t)q] >> 32, px = blob[o + 5 + 3 * (size_t)q];
+            if (blob[o + 3 + 3 * (size_t)q] != d.a + W * pad4(nrows)) bad("panels not contiguous");
+            int64_t c = 0;
+            for (; e < ns; ++e) {
+                const size_t sw = o + 3 + 3 * (size_t)np + 2 * (size_t)e;
+                const int64_t src = blob[sw], len = blob[sw + 1] & 0xffffffff, code = blob[sw + 1] >> 32;
+                if ((code >> 1) >= px + w) break;  // the next panel's
+                if ((code >> 1) != px + c || len < 0 || c + len > w) bad("segments do not cover the columns in order");
+                const int64_t row = (code & 1) ? xoff + x0 + src : ws0 + src;
+                if (row < 0 || row + len > (int64_t)UINT32_MAX) bad("source rows out of range");
+                for (int64_t i = 0; i < len; ++i) rows.push_back((uint32_t)(row + i));
+                c += len;
+            }
+            if (c != w) bad("columns without a source");
+            W += w;
+        }
+        if (W < 1 || W > BRG_XS_ELEMS || ws0 + blob[o] + nrows > (int64_t)UINT32_MAX) bad("target out of range");
+        if (rows != prev) {
+            prev0 = (uint32_t)out.idx.size();
+            if (out.idx.size() + rows.size() > (size_t)UINT32_MAX) bad("too many sources");
+            out.idx.insert(out.idx.end(), rows.begin(), rows.end());
+            prev.swap(rows);
+        }
+        d.idx0 = prev0;
+        d.W = (uint16_t)W;
+        out.max_w = std::max(out.max_w, (int)W);
+    }
+    pb.T = std::vector<Target>();
+    pb.P = std::vector<Panel>();
+    pb.S = std::vector<Seg>();
+}
+
+// Streams of one or several operators (the problems of a batch, their deadlines
+// aligned at the leaf pass by shift) as one on the device: targets by list, deadline
+// and work, which keeps each operator's own dependency order.
+void sv_upload(std::vector<SvHost> &v, const std::vector<int> &shift, SvStream &d, cudaStream_t st) {
+    struct Ref { int32_t list, key; double work; int32_t p, t; };
+    std::vector<Ref> ref;
+    SvHost all;
+    std::vector<uint32_t> g0(v.size()), i0(v.size());
+    std::vector<int64_t> a0(v.size());
+    double work[3] = {0, 0, 0};
+    for (size_t p = 0; p < v.size(); ++p) {
+        SvHost &s = v[p];
+        if (all.idx.size() + s.idx.size() > (size_t)UINT32_MAX || all.cons.size() + s.cons.size() > (size_t)UINT32_MAX)
+            throw ApiError(H2W_ERR_STATE, "internal: single-vector stream too large");
+        g0[p] = (uint32_t)all.grp.size();
+        i0[p] = (uint32_t)all.idx.size();
+        a0[p] = all.opn;
+        const uint32_t c0 = (uint32_t)all.cons.size();
+        for (const uint2 &g : s.grp) all.grp.push_back(make_uint2(g.x + c0, g.y));
+        for (uint32_t c : s.cons) all.cons.push_back(c + g0[p]);
+        all.idx.insert(all.idx.end(), s.idx.begin(), s.idx.end());
+        all.cnt.insert(all.cnt.end(), s.cnt.begin(), s.cnt.end());
+        all.opn += s.opn;
+        all.max_w = std::max(all.max_w, s.max_w);
+        for (size_t t = 0; t < s.hdr.size(); ++t) {
+            ref.push_back({s.list[t], s.key[t] + 4096 * shift[p], s.work[t], (int32_t)p, (int32_t)t});
+            work[s.list[t]] += (double)s.hdr[t].nrows * s.hdr[t].W;
+        }
+    }
+    if (ref.size() >= (size_t)INT32_MAX || all.grp.size() >= (size_t)INT32_MAX)
+        throw ApiError(H2W_ERR_STATE, "internal: too many single-vector targets");
+    std::stable_sort(ref.begin(), ref.end(), [](const Ref &a, const Ref &b) {
+        if (a.list != b.list) return a.list < b.list;
+        if (a.key != b.key) return a.key < b.key;
+        return a.work > b.work;
+    });
+    for (int l = 0; l < 3; ++l) d.list[l][0] = d.list[l][1] = 0;
+    for (const Ref &r : ref) {
+        SvHdr h = v[(size_t)r.p].hdr[(size_t)r.t];
+        h.a += a0[(size_t)r.p];
+        h.grp += g0[(size_t)r.p];
+        h.idx0 += i0[(size_t)r.p];
+        all.hdr.push_back(h);
+        ++d.list[r.list][1];
+    }
+    for (int l = 1; l < 3; ++l) {
+        d.list[l][0] = d.list[l - 1][1];
+        d.list[l][1] += d.list[l][0];
+    }
+    d.share = (int32_t)(1000.0 * work[0] / std::max(1.0, work[0] + work[1]));
+    d.ngrp = (int32_t)all.grp.size();
+    d.hdr.upload(all.hdr, st);
+    d.idx.upload(all.idx, st);
+    d.cons.upload(all.cons, st);
+    d.grp.upload(all.grp, st);
+    d.cnt.upload(all.cnt, st);
+    d.rem.alloc(all.cnt.size());
+    if (!d.ctr.p) d.ctr.alloc(SV_CTRS);
+    CK(sv_configure(all.max_w, d.f64, d.f32));
+    CK(cudaStreamSynchronize(st));  // the host arrays end here
+}
+
 // for the profiling statistics.
 void realize_single(h2w_handle *h, int64_t row_split) {
     if (!h->plan) throw ApiError(H2W_ERR_STATE, "operator not assembled");
@@ -1727,30 +2060,6 @@ void realize_single(h2w_handle *h, int64_t row_split) {
     pack_records(pb, h->phases, roff, blob, pstart);
     first_writers_overwrite(roff, blob, h->ws_n, h->fly_active ? &h->fly_rows : nullptr);
     check_phase_writers(roff, blob, h->phases);
-    {
-        // FP32 records on the slice-contiguous copy: panel q of target t reads its
-        // rows from slice (a', pad4(nrows)) instead of (a, lda); slices 16-byte aligned
-        std::vector<int64_t> bs(blob), sl;
-        int64_t off = 0;
-        for (size_t t = 0; t + 1 < roff.size(); ++t) {
-            const int64_t o = roff[t];
-            const int64_t nrows = bs[(size_t)o + 1] & 0xffffffff, np = bs[(size_t)o + 2] & 0xffffffff;
-            const int64_t ld = pad4(nrows);
-            for (int64_t q = 0; q < np; ++q) {
-                const size_t wa = (size_t)(o + 3 + 3 * q), wl = wa + 1;
-                const int64_t a = bs[wa], lda = bs[wl] & 0xffffffff, w = bs[wl] >> 32;
-                sl.insert(sl.end(), {a, lda, nrows, w, off, ld});
-                bs[wa] = off;
-                bs[wl] = (int64_t)(uint32_t)ld | (w << 32);
-                off += pad4(ld * w);
-            }
-        }
-        h->d_blob_s.upload(bs, h->stream);
-        h->d_sslices.upload(sl, h->stream);
-        h->op32s_n = off;
-        h->op32s_ready = false;
-        h->d_op32s.reset();
-    }
     // the far M2L kernel runs between the upward passes (logical phases <= L)
     // and the downward ones (>= L + 1)
     h->fly_split = (int)h->phases.size();
@@ -1759,16 +2068,6 @@ void realize_single(h2w_handle *h, int64_t row_split) {
             h->fly_split = (int)q;
             break;
         }
-    {
-        std::vector<int32_t> cnt, cidx;
-        std::vector<int64_t> coff;
-        build_deps(pb, h->ws_n, cnt, coff, cidx);
-        h->d_sdep0.upload(cnt, h->stream);
-        h->d_sdep.alloc(cnt.size());
-        h->d_scoff.upload(coff, h->stream);
-        h->d_scidx.upload(cidx, h->stream);
-        if (!h->d_sctr.p) h->d_sctr.alloc(1);
-    }
     cudaStream_t st = h->stream;
     h->d_roff.upload(roff, st);
     h->d_blob.upload(blob, st);
@@ -1777,6 +2076,33 @@ void realize_single(h2w_handle *h, int64_t row_split) {
     pb.T = std::vector<Target>();
     pb.P = std::vector<Panel>();
     pb.S = std::vector<Seg>();
+    {
+        std::vector<SvHost> sv(1);
+        sv_build(h, row_split, 0, 0, 0, h->xoff(), sv[0]);
+        h->fused_sv = sv[0].fused;
+        h->ops_n = sv[0].opn;
+        // in a product with the far field on the fly, list 0 from the passes after the upward ones
+        h->sv_split = (int32_t)std::count_if(sv[0].hdr.begin(), sv[0].hdr.end(), [&](const SvHdr &d) {
+            const size_t t = (size_t)(&d - sv[0].hdr.data());
+            return sv[0].list[t] == 0 && sv[0].key[t] < 4096 * h->tree.nL;
+        });
+        h->d_sslices.upload(sv[0].slices, st);
+        h->op32s_ready = h->op64s_ready = false;
+        h->d_op32s.reset();
+        sv_upload(sv, {0}, h->sv, st);
+        // The FP64 copy is made with the operator, a second one in memory: only where that
+        // leaves the room of the FP32 copies and of a double-FP32 one (three times as much
+        // again); else FP64 products stay on the packed operator and the cooperative launch.
+        size_t fr = 0, tot = 0;
+        const size_t need = (size_t)std::max<int64_t>(h->ops_n, 4) * 8;
+        if (h->d_op64s.n * 8 != need) h->d_op64s.reset();
+        CK(cudaMemGetInfo(&fr, &tot));
+        if (h->d_op64s.p || fr / 4 >= need) {
+            if (!h->d_op64s.p) h->d_op64s.alloc(need / 8);
+            CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 6, h->d_op64s.p, st));
+            h->op64s_ready = true;
+        }
+    }
     CK(cudaStreamSynchronize(st));
 }
 
@@ -2409,7 +2735,7 @@ void build_plan(h2w_handle *h) {
         realize_single(h, h->row_split);
         realize_multi(h, h->mr_xw);
     }
-    h->d_ws.alloc((size_t)h->ws_n);
+    h->d_ws.alloc((size_t)(h->xoff() + h->nv()));
     h->d_ctr.alloc(h->phases.size() + 1);
     h->d_err.alloc(1);
     CK(cudaMemsetAsync(h->d_err.p, 0, 4, st));
@@ -2533,6 +2859,69 @@ void prof_launch(h2w_handle *h, int prec, int phase, cudaStream_t st, F &&launch
     h->prof_recs.push_back(r);
 }
 
+// the slice-contiguous FP32 operator of the single-vector stream
+void ensure_f32s(h2w_handle *h) {
+    if (h->op32s_ready) return;
+    h->d_op32s.reset();
+    h->d_op32s.alloc((size_t)std::max<int64_t>(h->ops_n, 4));
+    CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 6, h->d_op32s.p, h->stream));
+    CK(cudaStreamSynchronize(h->stream));  // products may run on a caller's stream
+    h->op32s_ready = true;
+}
+
+// The arguments of a dataflow launch of h's stream, all of it
+template <class T>
+SvArgs<T> sv_args(h2w_handle *h, const T *A, T *ws, const double *dx, double *dy, const int32_t *perm) {
+    SvArgs<T> a{};
+    a.hdr = h->sv.hdr.p;
+    a.idx = h->sv.idx.p;
+    a.cons = h->sv.cons.p;
+    a.grp = h->sv.grp.p;
+    for (int l = 0; l < 3; ++l) {
+        a.l0[l] = h->sv.list[l][0];
+        a.l1[l] = h->sv.list[l][1];
+    }
+    a.na = h->sv.share;
+    a.ngrp = h->sv.ngrp;
+    a.A = A;
+    a.ws = ws;
+    a.nzero = a.xoff = h->xoff();
+    a.nx = h->nv();
+    a.xin = dx;
+    a.perm = perm;
+    a.yout = dy;
+    a.cnt = h->sv.cnt.p;
+    a.rem = h->sv.rem.p;
+    a.ctr = h->sv.ctr.p;
+    a.bar = h->d_bar.p;
+    a.err = h->d_err.p;
+    a.prep = 1;
+    return a;
+}
+inline cudaError_t sv_run(h2w_handle *h, const SvArgs<double> &a, cudaStream_t st) { return launch_sv(a, h->sv.f64, st); }
+inline cudaError_t sv_run(h2w_handle *h, const SvArgs<float> &a, cudaStream_t st) { return launch_sv(a, h->sv.f32, st); }
+
+// The stored passes of a product on the dataflow launch; with the far field on
+// the fly, far(st) between the upward passes (and the near field) and the others
+template <class T, class F>
+void sv_product(h2w_handle *h, int prec, SvArgs<T> a, cudaStream_t st, F &&far) {
+    const int nph = (int)h->phases.size();
+    if (!h->fly_active) {
+        prof_launch(h, prec, nph, st, [&] { return sv_run(h, a, st); });
+        return;
+    }
+    SvArgs<T> up = a;
+    up.l1[0] = up.l0[0] + h->sv_split;
+    up.l1[2] = up.l0[2];
+    prof_launch(h, prec, nph, st, [&] { return sv_run(h, up, st); });
+    far();
+    a.l0[0] += h->sv_split;
+    a.l1[1] = a.l0[1];
+    a.ctr += 3;
+    a.prep = 0;
+    prof_launch(h, prec, nph, st, [&] { return sv_run(h, a, st); });
+}
+
 // y = A x. permuted: x and y in leaf order (GMRES works there: no gather or
 // scatter per product); otherwise original point order.
 // df: with the far field on the fly, its M2L in double-FP32 arithmetic
@@ -2542,27 +2931,8 @@ void run_matvec_f64(h2w_handle *h, const double *dx, double *dy, cudaStream_t st
                     bool df = false) {
     const int32_t *perm = permuted ? nullptr : h->d_perm.p;
     const int nph = (int)h->phases.size();
-    CK(cudaMemsetAsync(h->d_ws.p, 0, (size_t)h->ws_n * 8, st));
-    if (h->fly_active) {
-        // stored passes up to the upward ones, the far M2L kernel, the rest
-        auto stored = [&](int a, int b) {
-            if (b <= a) return;
-            if (h->coop) {
-                prof_launch(h, H2W_PREC_FP64, nph, st, [&] {
-                    return launch_coop_f64(h->d_roff.p, h->d_blob.p, h->d_pstart.p + a, b - a, h->d_op.p, h->d_ws.p,
-                                           dx, dy, perm, h->d_bar.p, h->d_err.p, st, h->spin_limit);
-                });
-            } else {
-                for (int q = a; q < b; ++q) {
-                    const Phase &ph = h->phases[(size_t)q];
-                    prof_launch(h, H2W_PREC_FP64, q, st, [&] {
-                        return launch_brg_f64(h->d_roff.p, h->d_blob.p, ph.t0, ph.t1, h->d_op.p, h->d_ws.p, dx, dy,
-                                              perm, st);
-                    });
-                }
-            }
-        };
-        stored(0, h->fly_split);
+    const bool flow = h->coop && h->dataflow && h->op64s_ready;
+    auto far = [&] {
         prof_launch(h, df ? H2W_PREC_DF64 : H2W_PREC_FP64, FLY_PHASE, st, [&] {
             if (df)
                 return launch_fly_df64(h->d_fly_items.p, (int64_t)h->d_fly_items.n, h->d_fly_ctr.p, h->d_fly_rowpid.p,
@@ -2571,28 +2941,34 @@ void run_matvec_f64(h2w_handle *h, const double *dx, double *dy, cudaStream_t st
             return launch_fly_f64(h->d_fly_items.p, (int64_t)h->d_fly_items.n, h->d_fly_ctr.p, h->d_fly_rowpid.p,
                                   h->d_fly_cpid.p, h->d_fly_cws.p, h->d_ws.p, h->kparams(), st);
         });
-        stored(h->fly_split, nph);
-    } else if (h->coop && h->dataflow) {
-        CK(cudaMemcpyAsync(h->d_sdep.p, h->d_sdep0.p, h->d_sdep0.n * 4, cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemsetAsync(h->d_sctr.p, 0, 4, st));
-        prof_launch(h, H2W_PREC_FP64, nph, st, [&] {
-            return launch_brg_flow_f64(h->d_roff.p, h->d_blob.p, 0, (int64_t)h->d_roff.n - 1, h->d_sctr.p, h->d_sdep.p,
-                                       h->d_scoff.p, h->d_scidx.p, h->d_op.p, h->d_ws.p, dx, dy, perm, h->d_err.p, st);
-        });
-    } else if (h->coop) {
-        prof_launch(h, H2W_PREC_FP64, nph, st, [&] {
-            return launch_coop_f64(h->d_roff.p, h->d_blob.p, h->d_pstart.p, nph, h->d_op.p, h->d_ws.p, dx, dy, perm,
-                                   h->d_bar.p, h->d_err.p, st, h->spin_limit);
-        });
+    };
+    if (flow) {
+        sv_product(h, H2W_PREC_FP64, sv_args<double>(h, h->d_op64s.p, h->d_ws.p, dx, dy, perm), st, far);
     } else {
-        for (size_t q = 0; q < h->phases.size(); ++q) {
-            const Phase &ph = h->phases[q];
-            prof_launch(h, H2W_PREC_FP64, (int)q, st, [&] {
-                return launch_brg_f64(h->d_roff.p, h->d_blob.p, ph.t0, ph.t1, h->d_op.p, h->d_ws.p, dx, dy, perm, st);
-            });
+        CK(cudaMemsetAsync(h->d_ws.p, 0, (size_t)h->ws_n * 8, st));
+        auto stored = [&](int a, int b) {  // phases [a, b)
+            if (b > a && h->coop) {
+                prof_launch(h, H2W_PREC_FP64, nph, st, [&] {
+                    return launch_coop_f64(h->d_roff.p, h->d_blob.p, h->d_pstart.p + a, b - a, h->d_op.p, h->d_ws.p,
+                                           dx, dy, perm, h->d_bar.p, h->d_err.p, st, h->spin_limit);
+                });
+                return;
+            }
+            for (int q = a; q < b; ++q) {
+                const Phase &ph = h->phases[(size_t)q];
+                prof_launch(h, H2W_PREC_FP64, q, st, [&] {
+                    return launch_brg_f64(h->d_roff.p, h->d_blob.p, ph.t0, ph.t1, h->d_op.p, h->d_ws.p, dx, dy, perm, st);
+                });
+            }
+        };
+        const int split = h->fly_active ? h->fly_split : nph;
+        stored(0, split);
+        if (h->fly_active) {
+            far();
+            stored(split, nph);
         }
     }
-    if (!h->fused_scatter) {
+    if (!(flow ? h->fused_sv : h->fused_scatter)) {
         if (permuted)
             CK(cudaMemcpyAsync(dy, h->d_ws.p + h->yperm_off, (size_t)h->nv() * 8, cudaMemcpyDeviceToDevice, st));
         else
@@ -2604,7 +2980,6 @@ void ensure_f32(h2w_handle *h) {
     if (h->d_op32.p) return;
     h->d_op32.alloc((size_t)h->op_n);
     CK(launch_convert_f32(h->d_op.p, h->d_op32.p, h->op_n, h->stream));
-    h->d_ws32.alloc((size_t)h->ws_n);
     CK(cudaStreamSynchronize(h->stream));
 }
 
@@ -2619,71 +2994,50 @@ void ensure_f32m(h2w_handle *h) {
     h->op32m_ready = true;
 }
 
-// the slice-contiguous FP32 operator of the single-vector stream
-void ensure_f32s(h2w_handle *h) {
-    ensure_f32(h);
-    if (h->op32s_ready) return;
-    h->d_op32s.reset();
-    h->d_op32s.alloc((size_t)std::max<int64_t>(h->op32s_n, 4));
-    CK(launch_slice_copy_f32(h->d_op32.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 6, h->d_op32s.p, h->stream));
-    CK(cudaStreamSynchronize(h->stream));  // products may run on a caller's stream
-    h->op32s_ready = true;
-}
-
 // FP32 operator and workspace; x and y stay FP64 in original order (the
 // conversions happen in the kernel's gather and scatter).
 void run_matvec_f32(h2w_handle *h, const double *dx, double *dy, cudaStream_t st, bool permuted = false) {
-    ensure_f32s(h);
     const int32_t *perm = permuted ? nullptr : h->d_perm.p;
     const int nph = (int)h->phases.size();
-    CK(cudaMemsetAsync(h->d_ws32.p, 0, (size_t)h->ws_n * 4, st));
-    if (h->fly_active) {
-        auto stored = [&](int a, int b) {
-            if (b <= a) return;
-            if (h->coop) {
-                prof_launch(h, H2W_PREC_FP32, nph, st, [&] {
-                    return launch_coop_f32(h->d_roff.p, h->d_blob_s.p, h->d_pstart.p + a, b - a, h->d_op32s.p,
-                                           h->d_ws32.p, dx, dy, perm, h->d_bar.p, h->d_err.p, st, h->spin_limit);
-                });
-            } else {
-                for (int q = a; q < b; ++q) {
-                    const Phase &ph = h->phases[(size_t)q];
-                    prof_launch(h, H2W_PREC_FP32, q, st, [&] {
-                        return launch_brg_f32(h->d_roff.p, h->d_blob_s.p, ph.t0, ph.t1, h->d_op32s.p, h->d_ws32.p, dx, dy,
-                                              perm, st);
-                    });
-                }
-            }
-        };
-        stored(0, h->fly_split);
+    const bool flow = h->coop && h->dataflow;
+    if (h->d_ws32.n < (size_t)(h->xoff() + h->nv())) h->d_ws32.alloc((size_t)(h->xoff() + h->nv()));
+    auto far = [&] {
         prof_launch(h, H2W_PREC_FP32, FLY_PHASE, st, [&] {
             return launch_fly_f32(h->d_fly_items.p, (int64_t)h->d_fly_items.n, h->d_fly_ctr.p, h->d_fly_rowpid.p,
                                   h->d_fly_cpid.p, h->d_fly_cws.p, h->d_pts4.p, h->d_ws32.p, h->kparams(), h->k32, st);
         });
-        stored(h->fly_split, nph);
-    } else if (h->coop && h->dataflow) {
-        CK(cudaMemcpyAsync(h->d_sdep.p, h->d_sdep0.p, h->d_sdep0.n * 4, cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemsetAsync(h->d_sctr.p, 0, 4, st));
-        prof_launch(h, H2W_PREC_FP32, nph, st, [&] {
-            return launch_brg_flow_f32(h->d_roff.p, h->d_blob_s.p, 0, (int64_t)h->d_roff.n - 1, h->d_sctr.p, h->d_sdep.p,
-                                       h->d_scoff.p, h->d_scidx.p, h->d_op32s.p, h->d_ws32.p, dx, dy, perm, h->d_err.p,
-                                       st);
-        });
-    } else if (h->coop) {
-        prof_launch(h, H2W_PREC_FP32, nph, st, [&] {
-            return launch_coop_f32(h->d_roff.p, h->d_blob_s.p, h->d_pstart.p, nph, h->d_op32s.p, h->d_ws32.p, dx, dy,
-                                   perm, h->d_bar.p, h->d_err.p, st, h->spin_limit);
-        });
+    };
+    if (flow) {
+        if (!h->fly_active) ensure_f32(h);  // h2w_matvec_static runs on the packed copy
+        ensure_f32s(h);
+        sv_product(h, H2W_PREC_FP32, sv_args<float>(h, h->d_op32s.p, h->d_ws32.p, dx, dy, perm), st, far);
     } else {
-        for (size_t q = 0; q < h->phases.size(); ++q) {
-            const Phase &ph = h->phases[q];
-            prof_launch(h, H2W_PREC_FP32, (int)q, st, [&] {
-                return launch_brg_f32(h->d_roff.p, h->d_blob_s.p, ph.t0, ph.t1, h->d_op32s.p, h->d_ws32.p, dx, dy, perm,
-                                      st);
-            });
+        ensure_f32(h);
+        CK(cudaMemsetAsync(h->d_ws32.p, 0, (size_t)h->ws_n * 4, st));
+        auto stored = [&](int a, int b) {
+            if (b > a && h->coop) {
+                prof_launch(h, H2W_PREC_FP32, nph, st, [&] {
+                    return launch_coop_f32(h->d_roff.p, h->d_blob.p, h->d_pstart.p + a, b - a, h->d_op32.p, h->d_ws32.p,
+                                           dx, dy, perm, h->d_bar.p, h->d_err.p, st, h->spin_limit);
+                });
+                return;
+            }
+            for (int q = a; q < b; ++q) {
+                const Phase &ph = h->phases[(size_t)q];
+                prof_launch(h, H2W_PREC_FP32, q, st, [&] {
+                    return launch_brg_f32(h->d_roff.p, h->d_blob.p, ph.t0, ph.t1, h->d_op32.p, h->d_ws32.p, dx, dy,
+                                          perm, st);
+                });
+            }
+        };
+        const int split = h->fly_active ? h->fly_split : nph;
+        stored(0, split);
+        if (h->fly_active) {
+            far();
+            stored(split, nph);
         }
     }
-    if (!h->fused_scatter) {
+    if (!(flow ? h->fused_sv : h->fused_scatter)) {
         if (permuted) CK(vec_f32_to_f64(h->d_ws32.p + h->yperm_off, dy, h->tree.N, st));
         else CK(launch_scatter_f32(h->d_ws32.p + h->yperm_off, dy, h->d_perm.p, h->tree.N, st));
     }
@@ -3228,7 +3582,6 @@ int gmres_run(h2w_handle *h, const double *db, double *dx, int max_iter, double 
     }
     // graph path: the Arnoldi steps as one while-loop graph launch
     if (h->use_graphs && !h->graph_failed && !h->prof) {
-        if (prec == H2W_PREC_FP32) ensure_f32(h);
         gmres_prepare();
         // before a capture, one product outside it makes its buffers and launch
         // attributes (the step recomputes w)

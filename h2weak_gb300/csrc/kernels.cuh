@@ -65,15 +65,61 @@ cudaError_t launch_brg_f64(const int64_t *roff, const int64_t *blob, int64_t t0,
                            double *ws, const double *xin, double *yout, const int32_t *perm, cudaStream_t st);
 cudaError_t launch_brg_f32(const int64_t *roff, const int64_t *blob, int64_t t0, int64_t t1, const float *A,
                            float *ws, const double *xin, double *yout, const int32_t *perm, cudaStream_t st);
-// Dataflow form of the single-vector product (see launch_mr_f32_flow):
-// targets [t0, nt) in stored order, ctr a zeroed claim counter, rem the producer
-// counts (reset before every launch), consumers in cidx[coff[t] .. coff[t+1])
-cudaError_t launch_brg_flow_f64(const int64_t *roff, const int64_t *blob, int64_t t0, int64_t nt, int32_t *ctr, int32_t *rem,
-                                const int64_t *coff, const int32_t *cidx, const double *A, double *ws,
-                                const double *xin, double *yout, const int32_t *perm, int32_t *err, cudaStream_t st);
-cudaError_t launch_brg_flow_f32(const int64_t *roff, const int64_t *blob, int64_t t0, int64_t nt, int32_t *ctr, int32_t *rem,
-                                const int64_t *coff, const int32_t *cidx, const float *A, float *ws, const double *xin,
-                                double *yout, const int32_t *perm, int32_t *err, cudaStream_t st);
+// Dataflow form of the single-vector product (sv.cu). A target in 32 bytes: its
+// matrix (nrows x W, column-major at pad4(nrows), at A + a), destination rows,
+// the rows of its W sources (idx[idx0 ..]), its group and its problem.
+constexpr int SV_MAX_ROWS = 256;  // rows per target
+constexpr int SV_CTRS = 12;       // claim counters (three per launch of a product)
+struct alignas(16) SvHdr {
+    int64_t a;
+    uint32_t dst, idx0, grp, pid;
+    uint16_t nrows, W, flags, pad;
+};
+// The targets cut from one block row form a group: they wait for the same
+// producers, counted in rem[group], and their ends are counted by the groups in
+// cons[grp[g].x .. + grp[g].y). Three lists of targets: [0] the passes that depend
+// on one another, in the order of their deadlines, [1] work that depends on the
+// input alone, [2] the leaf pass. The first na CTAs take [0], then [1], the others [1],
+// then [0]; all end with [2].
+// Sources are rows of ws: [0, xoff) the workspace, from xoff the input in leaf
+// order. prep: the launch zeroes ws[0, nzero), resets the counts (rem from cnt, all
+// ngrp of them, and all SV_CTRS claim counters, the first three of which are ctr) and
+// writes the nx input values (through perm when given) first; without it the counts and
+// the workspace are those that the launch of an earlier range left, and ctr are three
+// counters of this launch's own. na: list 0's part of the work of lists 0 and 1, in
+// thousandths. perm also gives the output position of a leaf row. Batches: active[p] != -1 a problem to
+// skip, vshift[p] its workspace offset minus its vector offset (may be NULL).
+template <class T> struct SvArgs {
+    const SvHdr *hdr;
+    const uint32_t *idx, *cons;
+    const uint2 *grp;
+    const int32_t *active;
+    const int64_t *vshift;
+    int32_t l0[3], l1[3], na, ngrp;
+    const T *A;
+    T *ws;
+    int64_t nzero, xoff, nx;
+    const double *xin;
+    const int32_t *perm;
+    double *yout;
+    const int32_t *cnt;
+    int32_t *rem, *ctr;
+    unsigned *bar;
+    int32_t *err;
+    int prep;
+};
+// Launch shape for a stream whose widest target gathers max_w columns: found
+// once per stream (the launch itself makes no queries)
+struct SvConf {
+    int max_w = 0, nslots = 0, nst = 0, ctas = 0, cw = 4, sms = 1;
+    size_t smem = 0;
+};
+cudaError_t sv_configure(int max_w, SvConf &f64, SvConf &f32);
+cudaError_t launch_sv(const SvArgs<double> &a, const SvConf &c, cudaStream_t st);
+cudaError_t launch_sv(const SvArgs<float> &a, const SvConf &c, cudaStream_t st);
+// the slices of an FP64 operator (as launch_slice_copy_f32) copied or converted
+cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, double *dst, cudaStream_t st);
+cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, float *dst, cudaStream_t st);
 // The whole matvec as one cooperative launch: phase p covers targets
 // [pstart[p], pstart[p+1]); bar (2 unsigned, zero) is the grid barrier state;
 // spin bounds each grid-barrier wait in polls (<= 0: the built-in limit).
