@@ -3399,7 +3399,7 @@ int gmres_batch_run(h2w_handle *h, const double *bi, double *xi, int rp, int nrh
 // --------------------------------------------------------------- GMRES ---
 GmresDev gmres_state(h2w_handle *h, int m) {
     const int64_t N = h->tree.N;
-    const int nblk = (int)std::max<int64_t>(1, std::min<int64_t>(2 * 152, (N + 1023) / 1024));
+    const int nblk = gmres_blocks(N);
     if (h->g_m != m) {
         h->g_V.alloc((size_t)N * (size_t)(m + 1));
         h->g_w.alloc((size_t)N);
@@ -3411,7 +3411,7 @@ GmresDev gmres_state(h2w_handle *h, int m) {
         h->g_part.alloc((size_t)3 * nblk * (size_t)(m + 1));
         h->g_scal.alloc(8);
         h->g_iter.alloc(2);
-        h->g_tmp.alloc((size_t)N);
+        h->g_tmp.alloc((size_t)m + 1);
         h->g_r.alloc((size_t)N);
         h->g_m = m;
     }
@@ -3426,19 +3426,26 @@ GmresDev gmres_state(h2w_handle *h, int m) {
     g.part = h->g_part.p;
     g.scal = h->g_scal.p;
     g.iter = h->g_iter.p;
+    g.bar = h->d_bar.p;
+    g.err = h->d_err.p;
     g.N = N;
     g.m = m;
     g.nblk = nblk;
     return g;
 }
 
-double dnorm(h2w_handle *h, const double *x) {
-    if (!h->g_npart.p) h->g_npart.alloc(256);
+// Norms of one or two vectors, one wait for both
+void dnorms(h2w_handle *h, const double *x, const double *y, double *out) {
+    if (!h->g_npart.p) h->g_npart.alloc(512);
     if (!h->g_scal.p) h->g_scal.alloc(8);
     CK(vec_norm(x, h->tree.N, h->g_npart.p, 256, h->g_scal.p + 4, h->stream));
-    double v;
-    CK(cudaMemcpyAsync(&v, h->g_scal.p + 4, 8, cudaMemcpyDeviceToHost, h->stream));
+    if (y) CK(vec_norm(y, h->tree.N, h->g_npart.p + 256, 256, h->g_scal.p + 5, h->stream));
+    CK(cudaMemcpyAsync(out, h->g_scal.p + 4, y ? 16 : 8, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+}
+double dnorm(h2w_handle *h, const double *x) {
+    double v;
+    dnorms(h, x, nullptr, &v);
     return v;
 }
 
@@ -3519,113 +3526,62 @@ double fp32_error_multi(h2w_handle *h, const GmbT<T> &g, int rp, cudaStream_t st
     return eta;
 }
 
-// Solve the upper-triangular least-squares system H(0:k,0:k) y = s(0:k) on
-// the host, as Update does (*/codes/gmres.hpp:77-90), then x += V y.
-void gmres_xupdate(h2w_handle *h, const GmresDev &g, double *dx, int k) {
-    const int m = g.m;
-    std::vector<double> H((size_t)(m + 1) * (size_t)(k + 1)), s((size_t)k + 1);
-    CK(cudaMemcpyAsync(H.data(), g.H, H.size() * 8, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaMemcpyAsync(s.data(), g.s, s.size() * 8, cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    auto Hc = [&](int r, int c) { return H[(size_t)r + (size_t)c * (size_t)(m + 1)]; };
-    std::vector<double> y = s;
-    for (int i = k; i >= 0; --i) {
-        y[(size_t)i] /= Hc(i, i);
-        for (int j = i - 1; j >= 0; --j) y[(size_t)j] -= Hc(j, i) * y[(size_t)i];
-    }
-    CK(cudaMemcpyAsync(h->g_tmp.p, y.data(), y.size() * 8, cudaMemcpyHostToDevice, h->stream));
-    CK(gmres_update(g, dx, h->g_tmp.p, k, h->stream));
-}
-
-// All max_iter steps taken without meeting the tolerance: x += V y over all
-// columns, then the true relative residual.
-int gmres_unconverged(h2w_handle *h, const GmresDev &g, const double *db, double *dx, int max_iter, double tol,
-                      int prec, double normb, int *iters, double *resid) {
-    cudaStream_t st = h->stream;
-    gmres_xupdate(h, g, dx, max_iter - 1);
-    if (prec == H2W_PREC_FP32) run_matvec_f32(h, dx, h->g_r.p, st, true);
-    else run_matvec_f64(h, dx, h->g_r.p, st, true);
-    CK(vec_axpby(1.0, db, -1.0, h->g_r.p, h->g_r.p, h->tree.N, st));
-    *resid = dnorm(h, h->g_r.p) / normb;
-    *iters = max_iter;
-    return *resid < tol ? H2W_OK : H2W_ERR_NOT_CONVERGED;
-}
-
 // FP64 GMRES on device vectors in leaf order (the operator is applied as
 // P A P^T, which leaves GMRES unchanged up to rounding); matvec precision
-// chosen by prec.
+// chosen by prec. One read of the result: the start's test, the steps, the
+// back substitution and the update all run on the device.
 int gmres_run(h2w_handle *h, const double *db, double *dx, int max_iter, double tol, int prec, int *iters,
               double *resid, bool x0_zero = false) {
     GmresDev g = gmres_state(h, max_iter);
     cudaStream_t st = h->stream;
-    const int64_t N = h->tree.N;
-    CK(cudaMemcpyAsync(g.scal + 6, &tol, 8, cudaMemcpyHostToDevice, st));  // read by the Givens step
-    auto A = [&](const double *in, double *out) {
-        if (prec == H2W_PREC_FP32) run_matvec_f32(h, in, out, st, true);
-        else run_matvec_f64(h, in, out, st, true);
+    CK(cudaMemcpyAsync(g.scal + 6, &tol, 8, cudaMemcpyHostToDevice, st));  // read by the start and the steps
+    auto A = [&](const double *in, double *out, cudaStream_t s) {
+        if (prec == H2W_PREC_FP32) run_matvec_f32(h, in, out, s, true);
+        else run_matvec_f64(h, in, out, s, true);
     };
-    double normb = dnorm(h, db);
-    if (normb == 0.0) normb = 1;
-    if (x0_zero) {
-        CK(gmres_start(g, db, nullptr, normb, st));
-    } else {
-        A(dx, h->g_r.p);
-        CK(gmres_start(g, db, h->g_r.p, normb, st));
-    }
+    if (!x0_zero) A(dx, h->g_r.p, st);
+    CK(gmres_start(g, db, x0_zero ? nullptr : h->g_r.p, st));
     double sc[4];
-    CK(cudaMemcpyAsync(sc, g.scal, 32, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    *resid = sc[1];
-    if (sc[1] <= tol) {
-        *iters = 0;
-        return H2W_OK;
-    }
+    int32_t it2[2];
+    auto read = [&] {
+        CK(cudaMemcpyAsync(sc, g.scal, 32, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(it2, g.iter, 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+    };
+    cudaGraphExec_t ex = nullptr;
+    int64_t kps = 0;
     // graph path: the Arnoldi steps as one while-loop graph launch
     if (h->use_graphs && !h->graph_failed && !h->prof) {
         gmres_prepare();
         // before a capture, one product outside it makes its buffers and launch
         // attributes (the step recomputes w)
-        if (!loop_graph_cached(h, 0, prec, max_iter, 1, 1)) A(g.vcur, g.w);
-        int64_t kps = 0;
-        cudaGraphExec_t ex = loop_graph(h, 0, prec, max_iter, 1, 1, kps, [&](cudaStream_t s, cudaGraphConditionalHandle c) {
-            if (prec == H2W_PREC_FP32) run_matvec_f32(h, g.vcur, g.w, s, true);
-            else run_matvec_f64(h, g.vcur, g.w, s, true);
-            CK(gmres_cgs2(g, s));
-            CK(gmres_finish_iter(g, s));
-            CK(gmres_loop_cond(g, c, s));
+        if (!loop_graph_cached(h, 0, prec, max_iter, 1, 1)) A(g.vcur, g.w, st);
+        ex = loop_graph(h, 0, prec, max_iter, 1, 1, kps, [&](cudaStream_t s, cudaGraphConditionalHandle c) {
+            A(g.vcur, g.w, s);
+            CK(gmres_step(g, &c, s));
         });
-        if (ex) {
-            CK(cudaGraphLaunch(ex, st));
-            int32_t it2[2];
-            CK(cudaMemcpyAsync(sc, g.scal, 32, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(it2, g.iter, 8, cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            count_launch(kps * it2[1]);
-            *resid = sc[1];
-            if (sc[2] != 0.0) {
-                gmres_xupdate(h, g, dx, it2[0]);
-                CK(cudaStreamSynchronize(st));
-                *iters = it2[1];
-                return H2W_OK;
-            }
-            return gmres_unconverged(h, g, db, dx, max_iter, tol, prec, normb, iters, resid);
+    }
+    if (ex) {
+        CK(cudaGraphLaunch(ex, st));
+    } else {
+        read();
+        for (int i = 0; i < max_iter && sc[2] == 0.0; ++i) {
+            A(g.vcur, g.w, st);
+            CK(gmres_step(g, nullptr, st));
+            read();
         }
     }
-    for (int i = 0; i < max_iter; ++i) {
-        A(g.vcur, g.w);
-        CK(gmres_cgs2(g, st));
-        CK(gmres_finish_iter(g, st));
-        CK(cudaMemcpyAsync(sc, g.scal, 32, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        *resid = sc[1];
-        if (sc[2] != 0.0) {
-            gmres_xupdate(h, g, dx, i);
-            CK(cudaStreamSynchronize(st));
-            *iters = i + 1;
-            return H2W_OK;
-        }
-    }
-    return gmres_unconverged(h, g, db, dx, max_iter, tol, prec, normb, iters, resid);
+    CK(gmres_update(g, dx, h->g_tmp.p, st));
+    read();
+    if (ex) count_launch(kps * std::max(it2[1], 1));
+    *resid = sc[1];
+    *iters = it2[1];
+    if (sc[2] != 0.0) return H2W_OK;
+    // all max_iter steps taken without meeting the tolerance: the true relative residual
+    A(dx, h->g_r.p, st);
+    CK(vec_axpby(1.0, db, -1.0, h->g_r.p, h->g_r.p, h->tree.N, st));
+    *resid = dnorm(h, h->g_r.p) / sc[0];
+    return *resid < tol ? H2W_OK : H2W_ERR_NOT_CONVERGED;
 }
 
 // Device-side failure flag of the cooperative matvec (a grid barrier whose
@@ -4630,7 +4586,6 @@ int h2w_gmres(h2w_handle *h, const double *b, double *x, int max_iter, int tol_p
         int rc = h->cplx ? cgmres_run(h, bp.p, xp.p, max_iter, tol, iters, resid)
                          : gmres_run(h, bp.p, xp.p, max_iter, tol, H2W_PREC_FP64, iters, resid);
         CK(launch_scatter_f64(xp.p, dx, h->d_perm.p, N, h->stream));
-        CK(cudaStreamSynchronize(h->stream));
         check_device_error(h);
         if (where == H2W_HOST) {
             CK(cudaMemcpyAsync(x, h->d_x.p, (size_t)N * 8, cudaMemcpyDeviceToHost, h->stream));
@@ -4671,9 +4626,10 @@ int h2w_gmres_ir(h2w_handle *h, const double *b, double *x, int max_outer, int i
         double *dx_user = dx;
         db = bp.p;
         dx = xp.p;
-        double normb = dnorm(h, db);
-        if (normb == 0.0) normb = 1;
-        const bool x0_zero = dnorm(h, dx) == 0.0;
+        double nbx[2];
+        dnorms(h, db, dx, nbx);
+        const double normb = nbx[0] == 0.0 ? 1 : nbx[0];
+        const bool x0_zero = nbx[1] == 0.0;
         *inner_total = 0;
         *outer_iters = 0;
         int rc = H2W_ERR_NOT_CONVERGED;

@@ -849,106 +849,11 @@ cudaError_t launch_dense_matvec(const KParams &kp, int64_t N, const double *x, d
 
 // --------------------------------------------------------------- GMRES ---
 // Classical Gram-Schmidt with one reorthogonalisation (CGS2), FP64, on a
-// device-resident Krylov basis. Block b owns rows [b*chunk, (b+1)*chunk);
-// per-block partial sums go through three buffers so that no block
-// overwrites a partial another block still reads.
+// device-resident Krylov basis. CTA b owns rows [b*chunk, (b+1)*chunk).
 __device__ __forceinline__ void gm_rows(int64_t N, int nblk, int64_t &r0, int64_t &r1) {
     int64_t chunk = (N + nblk - 1) / nblk;
-    r0 = (int64_t)blockIdx.x * chunk;
+    r0 = (int64_t)blockIdx.x * chunk < N ? (int64_t)blockIdx.x * chunk : N;
     r1 = r0 + chunk < N ? r0 + chunk : N;
-}
-
-// out[b*(m+1)+k] = sum_{t in block b} V[t,k] w[t], k <= i
-__device__ void gm_block_dots(const GmresDev &g, int i, int64_t r0, int64_t r1, double *red, double *out) {
-    const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int k = 0; k <= i; ++k) {
-        const double *Vk = g.V + (size_t)k * g.N;
-        double acc = 0.0;
-        for (int64_t t = r0 + threadIdx.x; t < r1; t += blockDim.x) acc += Vk[t] * g.w[t];
-        acc = warp_sum(acc);
-        if (lane == 0) red[k * nw + warp] = acc;
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k <= i; k += blockDim.x) {
-        double s = 0.0;
-        for (int q = 0; q < nw; ++q) s += red[k * nw + q];
-        out[(size_t)blockIdx.x * (g.m + 1) + k] = s;
-    }
-}
-
-__global__ void gm_dots(GmresDev g) {
-    extern __shared__ double red[];
-    const int i = *g.iter;
-    int64_t r0, r1;
-    gm_rows(g.N, g.nblk, r0, r1);
-    gm_block_dots(g, i, r0, r1, red, g.part);
-}
-
-// h = sum_b in; w -= V h; H(:,i) (=|+=) h; out <- new dots (pass 0) or ||w||^2 partials (pass 1)
-__global__ void gm_update(GmresDev g, int pass) {
-    extern __shared__ double shm[];
-    double *h = shm;
-    double *red = shm + (g.m + 1);
-    const double *in = g.part + (size_t)pass * g.nblk * (g.m + 1);
-    double *out = g.part + (size_t)(pass + 1) * g.nblk * (g.m + 1);
-    const int i = *g.iter;
-    for (int k = threadIdx.x; k <= i; k += blockDim.x) {
-        double s = 0.0;
-        for (int b = 0; b < g.nblk; ++b) s += in[(size_t)b * (g.m + 1) + k];
-        h[k] = s;
-    }
-    __syncthreads();
-    if (blockIdx.x == 0)
-        for (int k = threadIdx.x; k <= i; k += blockDim.x) {
-            double *Hk = g.H + (size_t)i * (g.m + 1) + k;
-            *Hk = pass == 0 ? h[k] : *Hk + h[k];
-        }
-    int64_t r0, r1;
-    gm_rows(g.N, g.nblk, r0, r1);
-    for (int64_t t = r0 + threadIdx.x; t < r1; t += blockDim.x) {
-        double v = g.w[t];
-        for (int k = 0; k <= i; ++k) v -= g.V[(size_t)k * g.N + t] * h[k];
-        g.w[t] = v;
-    }
-    __syncthreads();
-    if (pass == 0) {
-        gm_block_dots(g, i, r0, r1, red, out);
-    } else {
-        const int nw = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        double acc = 0.0;
-        for (int64_t t = r0 + threadIdx.x; t < r1; t += blockDim.x) acc += g.w[t] * g.w[t];
-        acc = warp_sum(acc);
-        if (lane == 0) red[warp] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0.0;
-            for (int q = 0; q < nw; ++q) s += red[q];
-            out[(size_t)blockIdx.x * (g.m + 1)] = s;
-        }
-    }
-}
-
-// H(i+1,i) = ||w||; V[:,i+1] = vcur = (1/H(i+1,i)) w
-__global__ void gm_normalise(GmresDev g) {
-    __shared__ double hn;
-    const double *in = g.part + (size_t)2 * g.nblk * (g.m + 1);
-    const int i = *g.iter;
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < g.nblk; ++b) s += in[(size_t)b * (g.m + 1)];
-        hn = sqrt(s);
-        if (blockIdx.x == 0) g.H[(size_t)i * (g.m + 1) + i + 1] = hn;
-    }
-    __syncthreads();
-    const double ih = 1.0 / hn;
-    int64_t r0, r1;
-    gm_rows(g.N, g.nblk, r0, r1);
-    double *Vn = g.V + (size_t)(i + 1) * g.N;
-    for (int64_t t = r0 + threadIdx.x; t < r1; t += blockDim.x) {
-        double v = ih * g.w[t];
-        Vn[t] = v;
-        g.vcur[t] = v;
-    }
 }
 
 __device__ void gm_apply(double &dx, double &dy, double cs, double sn) {
@@ -957,32 +862,173 @@ __device__ void gm_apply(double &dx, double &dy, double cs, double sn) {
     dx = temp;
 }
 
-// Givens rotations on column i (*/codes/gmres.hpp:30-75,156-162); resid = |s(i+1)| / ||b||.
-__global__ void gm_givens(GmresDev g) {
-    const int i = *g.iter;
-    const double tol = g.scal[6];
-    double *Hc = g.H + (size_t)i * (g.m + 1);
-    if (g.scal[2] != 0.0) return;  // already converged: leave state untouched
-    for (int k = 0; k < i; ++k) gm_apply(Hc[k], Hc[k + 1], g.cs[k], g.sn[k]);
-    double dx = Hc[i], dy = Hc[i + 1], cs, sn;
-    if (dy == 0.0) { cs = 1.0; sn = 0.0; }
-    else if (fabs(dy) > fabs(dx)) {
-        double temp = dx / dy;
-        sn = 1.0 / sqrt(1.0 + temp * temp);
-        cs = temp * sn;
-    } else {
-        double temp = dy / dx;
-        cs = 1.0 / sqrt(1.0 + temp * temp);
-        sn = temp * cs;
+// One Arnoldi step after the product w = A v_i: two Gram-Schmidt passes, the norm, the
+// next basis vector, the Givens rotations of column i, the convergence test and (cond)
+// the loop condition of the captured step, as one cooperative launch with three grid
+// barriers. A CTA keeps its rows of w in shared memory (ws_rows > 0; else in g.w), and
+// those of the first vcap basis vectors, which the first pass reads from memory
+// and the other three sweeps from there. Dots: a warp per basis vector (and row share,
+// while there are fewer vectors than warps), whose lanes stride the rows: with few rows a
+// CTA the shuffles of a warp sum cost the FP64 pipe as much as the multiply-adds, so
+// there is one sum a vector, not one a vector and warp. Every CTA then sums the
+// partials of all CTAs itself, a warp a vector. What bounds it: latency, the barriers and
+// the chains of reads between them; past 1e5 rows, the FP64 pipe. A 7-step solve of 32768
+// rows: 29 us a step (cold caches), where five launches, whose CTAs each summed the
+// partials in one thread, took 54.
+constexpr int GMS_THREADS = 512, GMS_WARPS = GMS_THREADS / 32;
+
+// A CTA's rows of basis vector k
+struct GmCols {
+    const double *V;  // this CTA's rows of vector 0
+    int64_t N;
+    double *vsh;      // copies of the first vcap
+    int rows, vcap;
+    __device__ __forceinline__ const double *col(int k) const { return k < vcap ? vsh + (size_t)k * rows : V + (size_t)k * N; }
+};
+
+// out[k] = sum over this CTA's rows of V[., k] w, k <= i, then over all CTAs in h[k];
+// first: the copies are made
+__device__ void gm_dots_all(const GmresDev &g, const GmCols &C, int i, bool first, const double *w, double *red,
+                            double *part, double *h) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nk = i + 1, S = nk < GMS_WARPS ? GMS_WARPS / nk : 1, rows = C.rows;
+    __syncthreads();  // w is written
+    for (int e = warp; e < nk * S; e += GMS_WARPS) {
+        const int k = e % nk, sl = e / nk;
+        const double *v = first ? C.V + (size_t)k * C.N : C.col(k);
+        double *to = first && k < C.vcap ? C.vsh + (size_t)k * rows : nullptr;
+        double acc = 0.0;
+#pragma unroll 4
+        for (int t = sl * 32 + lane; t < rows; t += 32 * S) {
+            const double x = v[t];
+            if (to) to[t] = x;
+            acc = fma(x, w[t], acc);
+        }
+        acc = warp_sum(acc);
+        if (lane == 0) red[e] = acc;
     }
-    g.cs[i] = cs;
-    g.sn[i] = sn;
-    gm_apply(Hc[i], Hc[i + 1], cs, sn);
-    gm_apply(g.s[i], g.s[i + 1], cs, sn);
-    double resid = fabs(g.s[i + 1]) / g.scal[0];
-    g.scal[1] = resid;
-    if (resid < tol) g.scal[2] = 1.0;
-    else if (i + 1 < g.m) *g.iter = i + 1;
+    __syncthreads();
+    for (int k = threadIdx.x; k < nk; k += GMS_THREADS) {
+        double s = 0.0;
+        for (int sl = 0; sl < S; ++sl) s += red[sl * nk + k];
+        part[(size_t)k * g.nblk + blockIdx.x] = s;
+    }
+    grid_barrier(g.bar, gridDim.x, g.err);
+    for (int k = warp; k < nk; k += GMS_WARPS) {
+        double s = 0.0;
+        for (int b = lane; b < g.nblk; b += 32) s += __ldcg(part + (size_t)k * g.nblk + b);
+        s = warp_sum(s);
+        if (lane == 0) h[k] = s;
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(GMS_THREADS)
+    gm_step(GmresDev g, int ws_rows, int vcap, cudaGraphConditionalHandle hnd, int cond) {
+    extern __shared__ double gsh[];
+    __shared__ double s_hn, sh[32];
+    double *h1 = gsh, *h2 = h1 + g.m + 1, *red = h2 + g.m + 1, *wsh = red + g.m + 1 + GMS_WARPS;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int i = *g.iter;
+    const bool done = g.scal[2] != 0.0;  // CTA 0 changes these two only after the last barrier
+    if (done) {
+        if (cond && blockIdx.x == 0 && tid == 0) cudaGraphSetConditional(hnd, 0u);
+        return;
+    }
+    int64_t r0, r1;
+    gm_rows(g.N, g.nblk, r0, r1);
+    const int rows = (int)(r1 - r0);
+    double *w = ws_rows > 0 ? wsh : g.w + r0;
+    const GmCols C{g.V + r0, g.N, wsh + ws_rows, rows, vcap};
+    if (ws_rows > 0)
+        for (int t = tid; t < rows; t += GMS_THREADS) w[t] = g.w[r0 + t];
+    const size_t ps = (size_t)g.nblk * (g.m + 1);
+    double nrm = 0.0;
+    for (int pass = 0; pass < 2; ++pass) {
+        double *h = pass == 0 ? h1 : h2;
+        gm_dots_all(g, C, i, pass == 0, w, red, g.part + pass * ps, h);
+        nrm = 0.0;
+        for (int t = tid; t < rows; t += GMS_THREADS) {
+            double x = w[t];
+#pragma unroll 4
+            for (int k = 0; k <= i; ++k) x -= C.col(k)[t] * h[k];
+            w[t] = x;
+            nrm = fma(x, x, nrm);
+        }
+    }
+    nrm = block_sum(nrm, sh);
+    if (tid == 0) g.part[2 * ps + blockIdx.x] = nrm;
+    grid_barrier(g.bar, gridDim.x, g.err);
+    if (warp == 0) {
+        double s = 0.0;
+        for (int b = lane; b < g.nblk; b += 32) s += __ldcg(g.part + 2 * ps + b);
+        s = warp_sum(s);
+        if (lane == 0) s_hn = sqrt(s);
+    }
+    __syncthreads();
+    const double hn = s_hn;
+    // the first warp of CTA 0 does the rotations meanwhile
+    const bool rot = blockIdx.x == 0 && warp == 0;
+    if (!rot) {
+        const double ih = 1.0 / hn;
+        const int first = blockIdx.x == 0 ? 32 : 0;
+        double *Vn = g.V + (size_t)(i + 1) * g.N + r0;
+        for (int t = tid - first; t < rows; t += GMS_THREADS - first) {
+            const double v = ih * w[t];
+            Vn[t] = v;
+            g.vcur[r0 + t] = v;
+        }
+        return;
+    }
+    // Givens rotations on column i (*/codes/gmres.hpp:30-75,156-162); resid = |s(i+1)| / ||b||.
+    // h1: the column; red and h2: the earlier rotations
+    for (int k = lane; k <= i; k += 32) {
+        h1[k] += h2[k];
+        if (k < i) {
+            red[k] = g.cs[k];
+            h2[k] = g.sn[k];
+        }
+    }
+    __syncwarp();
+    if (lane == 0) {
+        double next = hn;
+        for (int k = 0; k < i; ++k) gm_apply(h1[k], h1[k + 1], red[k], h2[k]);
+        double dx = h1[i], dy = next, cs, sn;
+        if (dy == 0.0) { cs = 1.0; sn = 0.0; }
+        else if (fabs(dy) > fabs(dx)) {
+            double temp = dx / dy;
+            sn = 1.0 / sqrt(1.0 + temp * temp);
+            cs = temp * sn;
+        } else {
+            double temp = dy / dx;
+            cs = 1.0 / sqrt(1.0 + temp * temp);
+            sn = temp * cs;
+        }
+        g.cs[i] = cs;
+        g.sn[i] = sn;
+        gm_apply(h1[i], next, cs, sn);
+        g.H[(size_t)i * (g.m + 1) + i + 1] = next;
+        gm_apply(g.s[i], g.s[i + 1], cs, sn);
+        const double resid = fabs(g.s[i + 1]) / g.scal[0];
+        g.scal[1] = resid;
+        if (resid < g.scal[6]) g.scal[2] = 1.0;
+        else if (i + 1 < g.m) *g.iter = i + 1;
+        const int c = ++g.iter[1];
+        if (cond) cudaGraphSetConditional(hnd, (!(resid < g.scal[6]) && c < g.m) ? 1u : 0u);
+    }
+    __syncwarp();
+    for (int k = lane; k <= i; k += 32) g.H[(size_t)i * (g.m + 1) + k] = h1[k];
+}
+
+__global__ void gm_backsub(GmresDev g, double *__restrict__ y);
+
+int gmres_blocks(int64_t N) {
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // one CTA an SM at most, and at least a row a thread: more CTAs only add partials to sum
+    const int64_t want = (N + GMS_THREADS - 1) / GMS_THREADS;
+    return (int)(want < 1 ? 1 : want < sms ? want : sms > 0 ? sms : 1);
 }
 
 // One-time function attributes of the Arnoldi kernels (done before any
@@ -990,61 +1036,75 @@ __global__ void gm_givens(GmresDev g) {
 void gmres_prepare() {
     static bool cfg = false;
     if (!cfg) {
-        cudaFuncSetAttribute(gm_dots, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(gm_update, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(gm_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+        cudaFuncSetAttribute(gm_backsub, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cfg = true;
     }
 }
 
-cudaError_t gmres_cgs2(const GmresDev &g, cudaStream_t st) {
-    const int nw = GM_THREADS / 32;
-    size_t sm_dots = (size_t)(g.m + 1) * nw * sizeof(double);
-    size_t sm_upd = (size_t)(g.m + 1) * (nw + 1) * sizeof(double);
+cudaError_t gmres_step(const GmresDev &g, const cudaGraphConditionalHandle *hnd, cudaStream_t st) {
     gmres_prepare();
-    gm_dots<<<g.nblk, GM_THREADS, sm_dots, st>>>(g);
-    gm_update<<<g.nblk, GM_THREADS, sm_upd, st>>>(g, 0);
-    gm_update<<<g.nblk, GM_THREADS, sm_upd, st>>>(g, 1);
-    count_launch(3); return cudaGetLastError();
+    const int64_t chunk = (g.N + g.nblk - 1) / g.nblk;
+    const size_t head = ((size_t)3 * (g.m + 1) + GMS_WARPS) * sizeof(double), most = 200 * 1024;
+    if (head > most) return cudaErrorInvalidValue;
+    int ws_rows = head + (size_t)chunk * 8 <= most ? (int)chunk : 0;
+    const size_t left = ws_rows > 0 ? (most - head) / 8 - (size_t)chunk : 0;
+    int vcap = (int)(left / (size_t)chunk < (size_t)g.m + 1 ? left / (size_t)chunk : (size_t)g.m + 1);
+    const size_t smem = head + ((size_t)ws_rows + (size_t)vcap * chunk) * 8;
+    GmresDev ga = g;
+    cudaGraphConditionalHandle h = hnd ? *hnd : cudaGraphConditionalHandle{};
+    int cond = hnd ? 1 : 0;
+    void *args[] = {(void *)&ga, (void *)&ws_rows, (void *)&vcap, (void *)&h, (void *)&cond};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)gm_step, dim3(g.nblk), dim3(GMS_THREADS), args, smem, st);
+    count_launch();
+    return e;
 }
 
-cudaError_t gmres_finish_iter(const GmresDev &g, cudaStream_t st) {
-    gm_normalise<<<g.nblk, GM_THREADS, 0, st>>>(g);
-    gm_givens<<<1, 1, 0, st>>>(g);
-    count_launch(2); return cudaGetLastError();
-}
-
-// r = b - Ax (Ax NULL: r = b); beta = ||r||; V[:,0] = vcur = r / beta; s = beta e1; iter = 0
+// r = b - Ax (Ax NULL: r = b); beta = ||r||; V[:,0] = vcur = r / beta; s = beta e1; iter = 0;
+// normb = ||b|| (1 if b = 0); converged (scal[2] = 2) if beta / normb <= tol
 __global__ void gm_resid_part(GmresDev g, const double *__restrict__ b, const double *__restrict__ Ax) {
     __shared__ double sh[32];
     int64_t r0, r1;
     gm_rows(g.N, g.nblk, r0, r1);
-    double acc = 0.0;
+    double acc = 0.0, bb = 0.0;
     for (int64_t t = r0 + threadIdx.x; t < r1; t += blockDim.x) {
-        double r = Ax ? b[t] - Ax[t] : b[t];  // Ax == NULL: x0 = 0
+        const double v = b[t], r = Ax ? v - Ax[t] : v;  // Ax == NULL: x0 = 0
         g.w[t] = r;
         acc += r * r;
+        bb += v * v;
     }
     acc = block_sum(acc, sh);
-    if (threadIdx.x == 0) g.part[blockIdx.x] = acc;
-}
-__global__ void gm_start_fin(GmresDev g, double normb) {
-    __shared__ double beta;
+    bb = block_sum(bb, sh);
     if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (int b = 0; b < g.nblk; ++b) s += g.part[b];
-        beta = sqrt(s);
-        if (blockIdx.x == 0) {
-            for (int k = 0; k <= g.m; ++k) { g.s[k] = 0.0; g.cs[k] = 0.0; g.sn[k] = 0.0; }
-            g.s[0] = beta;
+        g.part[blockIdx.x] = acc;
+        g.part[g.nblk + blockIdx.x] = bb;
+    }
+}
+__global__ void gm_start_fin(GmresDev g) {
+    __shared__ double sh[32];
+    double r2 = 0.0, b2 = 0.0;
+    for (int b = threadIdx.x; b < g.nblk; b += blockDim.x) {
+        r2 += g.part[b];
+        b2 += g.part[g.nblk + b];
+    }
+    const double beta = sqrt(block_sum(r2, sh));
+    double normb = sqrt(block_sum(b2, sh));
+    if (normb == 0.0) normb = 1.0;
+    if (blockIdx.x == 0) {
+        for (int k = threadIdx.x; k <= g.m; k += blockDim.x) {
+            g.s[k] = k == 0 ? beta : 0.0;
+            g.cs[k] = 0.0;
+            g.sn[k] = 0.0;
+        }
+        if (threadIdx.x == 0) {
             g.scal[0] = normb;
             g.scal[1] = beta / normb;
-            g.scal[2] = 0.0;
+            g.scal[2] = beta / normb <= g.scal[6] ? 2.0 : 0.0;
             g.scal[3] = beta;
             g.iter[0] = 0;
-            g.iter[1] = 0;  // Arnoldi steps taken (graph loop counter)
+            g.iter[1] = 0;  // Arnoldi steps taken
         }
     }
-    __syncthreads();
     const double ib = 1.0 / beta;
     int64_t r0, r1;
     gm_rows(g.N, g.nblk, r0, r1);
@@ -1054,35 +1114,48 @@ __global__ void gm_start_fin(GmresDev g, double normb) {
         g.vcur[t] = v;
     }
 }
-// Loop condition of the graph-captured Arnoldi step: run another step while
-// not converged and fewer than m steps were taken.
-__global__ void gm_loop_cond(GmresDev g, cudaGraphConditionalHandle hnd) {
-    const int c = ++g.iter[1];
-    cudaGraphSetConditional(hnd, (g.scal[2] == 0.0 && c < g.m) ? 1u : 0u);
-}
-cudaError_t gmres_loop_cond(const GmresDev &g, cudaGraphConditionalHandle hnd, cudaStream_t st) {
-    gm_loop_cond<<<1, 1, 0, st>>>(g, hnd);
-    count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t gmres_start(const GmresDev &g, const double *b, const double *Ax, double normb, cudaStream_t st) {
+cudaError_t gmres_start(const GmresDev &g, const double *b, const double *Ax, cudaStream_t st) {
     gm_resid_part<<<g.nblk, GM_THREADS, 0, st>>>(g, b, Ax);
-    gm_start_fin<<<g.nblk, GM_THREADS, 0, st>>>(g, normb);
+    gm_start_fin<<<g.nblk, GM_THREADS, 0, st>>>(g);
     count_launch(2); return cudaGetLastError();
 }
 
-// x += sum_{j<=k} V[:,j] y[j]  (y precomputed by the back-substitution, in g.s)
-__global__ void gm_xupdate(GmresDev g, double *__restrict__ x, const double *__restrict__ y, int k) {
+// The triangular least-squares system H(0:k,0:k) y = s(0:k), k the last column
+// (*/codes/gmres.hpp:77-90), into y; nothing if converged at the start. One CTA: a
+// column's updates in parallel, the columns in turn, each entry's operations in
+// the order of the plain double loop.
+__global__ void gm_backsub(GmresDev g, double *__restrict__ y) {
+    extern __shared__ double ysh[];
+    if (g.scal[2] == 2.0) return;
+    const int k = g.iter[0];
+    for (int j = threadIdx.x; j <= k; j += blockDim.x) ysh[j] = g.s[j];
+    for (int i = k; i >= 0; --i) {
+        const double *Hc = g.H + (size_t)i * (g.m + 1);
+        __syncthreads();
+        const double yi = ysh[i] / Hc[i];
+        __syncthreads();
+        for (int j = threadIdx.x; j < i; j += blockDim.x) ysh[j] = __dsub_rn(ysh[j], __dmul_rn(Hc[j], yi));
+        if (threadIdx.x == 0) ysh[i] = yi;
+    }
+    __syncthreads();
+    for (int j = threadIdx.x; j <= k; j += blockDim.x) y[j] = ysh[j];
+}
+// x += sum_{j<=k} V[:,j] y[j]
+__global__ void gm_xupdate(GmresDev g, double *__restrict__ x, const double *__restrict__ y) {
+    if (g.scal[2] == 2.0) return;
+    const int k = g.iter[0];
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < g.N; t += (int64_t)gridDim.x * blockDim.x) {
         double v = x[t];
+#pragma unroll 4
         for (int j = 0; j <= k; ++j) v += g.V[(size_t)j * g.N + t] * y[j];
         x[t] = v;
     }
 }
-cudaError_t gmres_update(const GmresDev &g, double *x, const double *y, int k, cudaStream_t st) {
-    gm_xupdate<<<g.nblk, GM_THREADS, 0, st>>>(g, x, y, k);
-    count_launch(); return cudaGetLastError();
+cudaError_t gmres_update(const GmresDev &g, double *x, double *y, cudaStream_t st) {
+    gm_backsub<<<1, 128, (size_t)(g.m + 1) * sizeof(double), st>>>(g, y);
+    const int64_t nb = (g.N + GM_THREADS - 1) / GM_THREADS;
+    gm_xupdate<<<(unsigned)(nb < 1216 ? nb : 1216), GM_THREADS, 0, st>>>(g, x, y);
+    count_launch(2); return cudaGetLastError();
 }
 
 __global__ void norm_part(const double *__restrict__ x, int64_t n, double *part) {
@@ -1094,13 +1167,15 @@ __global__ void norm_part(const double *__restrict__ x, int64_t n, double *part)
     if (threadIdx.x == 0) part[blockIdx.x] = acc;
 }
 __global__ void norm_fin(const double *part, int nblk, double *out) {
+    __shared__ double sh[32];
     double s = 0.0;
-    for (int b = 0; b < nblk; ++b) s += part[b];
-    *out = sqrt(s);
+    for (int b = threadIdx.x; b < nblk; b += blockDim.x) s += part[b];
+    s = block_sum(s, sh);
+    if (threadIdx.x == 0) *out = sqrt(s);
 }
 cudaError_t vec_norm(const double *x, int64_t n, double *part, int nblk, double *out, cudaStream_t st) {
     norm_part<<<nblk, GM_THREADS, 0, st>>>(x, n, part);
-    norm_fin<<<1, 1, 0, st>>>(part, nblk, out);
+    norm_fin<<<1, GM_THREADS, 0, st>>>(part, nblk, out);
     count_launch(2); return cudaGetLastError();
 }
 

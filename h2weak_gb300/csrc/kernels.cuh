@@ -204,19 +204,21 @@ cudaError_t launch_dense_rows(const KParams &kp, int64_t N, const double *x, con
 struct GmresDev {
     double *V, *w, *vcur, *H, *cs, *sn, *s;  // V: N x (m+1); H: (m+1) x m column-major
     double *part;                             // 3 * nblk * (m+1) partial sums
-    double *scal;                             // [0] ||b||, [1] resid, [2] converged flag, [3] beta,
-                                              // [6] stopping tolerance (read by the Givens step)
+    double *scal;                             // [0] ||b||, [1] resid, [2] 0 running, 1 converged, 2 at the start,
+                                              // [3] beta, [6] stopping tolerance
     int32_t *iter;                            // [0] current Arnoldi column i, [1] steps taken
+    unsigned *bar;                            // grid barrier state (2, zero) and error word of the step
+    int32_t *err;
     int64_t N;
     int m, nblk;
 };
+int gmres_blocks(int64_t N);                                      // nblk
 void gmres_prepare();                                             // one-time kernel attributes
-cudaError_t gmres_cgs2(const GmresDev &g, cudaStream_t st);      // orthogonalise w against V[:, 0..i], H column
-cudaError_t gmres_finish_iter(const GmresDev &g, cudaStream_t st);  // normalise, Givens, residual (tol: scal[6])
-cudaError_t gmres_start(const GmresDev &g, const double *b, const double *Ax, double normb, cudaStream_t st);
-cudaError_t gmres_update(const GmresDev &g, double *x, const double *y, int k, cudaStream_t st);
-// last node of a graph-captured Arnoldi step: sets the while-loop condition
-cudaError_t gmres_loop_cond(const GmresDev &g, cudaGraphConditionalHandle hnd, cudaStream_t st);
+// one Arnoldi step on w = A v_i; hnd (may be NULL): the while condition of a captured step
+cudaError_t gmres_step(const GmresDev &g, const cudaGraphConditionalHandle *hnd, cudaStream_t st);
+cudaError_t gmres_start(const GmresDev &g, const double *b, const double *Ax, cudaStream_t st);
+// x += V y, y the solved least-squares system of the columns so far (m + 1 doubles)
+cudaError_t gmres_update(const GmresDev &g, double *x, double *y, cudaStream_t st);
 cudaError_t vec_norm(const double *x, int64_t n, double *part, int nblk, double *out, cudaStream_t st);
 cudaError_t vec_axpby(double a, const double *x, double b, const double *y, double *z, int64_t n, cudaStream_t st);
 cudaError_t vec_f64_to_f32(const double *x, float *y, int64_t n, cudaStream_t st);
