@@ -9,6 +9,7 @@
 #include <complex>
 #include <cstdio>
 #include <cstring>
+#include <deque>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -151,7 +152,7 @@ struct h2w_handle {
     DBuf<double> d_op64s;
     DBuf<int64_t> d_sslices;
     int64_t ops_n = 0;
-    bool op32s_ready = false, op64s_ready = false;
+    bool op32s_ready = false;
     SvStream sv;
     int32_t sv_split = 0;   // list 0: end of the upward passes
     bool fused_sv = true;
@@ -1759,48 +1760,44 @@ struct SvHost {
 };
 
 // Producers of the groups, in their order: as build_deps, with all targets of a group
-// taken together and no atomic writers. parts[g]: targets of group g.
-void group_deps(const std::vector<PlanBuilder::LTarget> &groups, const std::vector<int32_t> &parts, int64_t ws_n,
+// taken together and no atomic writers. parts[g]: targets of group g. The tree passes
+// write every row to the end before anything gathers it, so the writers of a row order
+// its readers and no write has to wait for a read; a plan that did otherwise is refused.
+void group_deps(const std::vector<const PlanBuilder::LTarget *> &groups, const std::vector<int32_t> &parts, int64_t ws_n,
                 SvHost &out) {
     const size_t ng = groups.size();
-    std::vector<int32_t> last((size_t)ws_n, -1);
-    std::vector<std::vector<int32_t>> rd((size_t)ws_n), prod(ng);
-    std::vector<int32_t> deps;
+    std::vector<int32_t> last((size_t)ws_n, -1), deps;
+    std::vector<uint8_t> gathered((size_t)ws_n, 0);
+    std::vector<int32_t> prod;  // producers of all groups, group g's from first[g]
+    std::vector<size_t> first(ng + 1, 0);
     std::vector<uint32_t> ncons(ng, 0);
     out.cnt.assign(ng, 0);
     for (size_t g = 0; g < ng; ++g) {
-        const PlanBuilder::LTarget &l = groups[g];
-        const bool scatter = l.flags & T_SCATTER, accum = l.flags & T_ACCUM;
+        const PlanBuilder::LTarget &l = *groups[g];
         deps.clear();
-        auto for_reads = [&](auto &&f) {
-            for (const PlanBuilder::PanelSpec &pn : l.panels)
-                for (const Seg &sg : pn.segs)
-                    if (!(sg.flags & S_GATHER))
-                        for (int64_t r = sg.src; r < sg.src + sg.len; ++r) f((size_t)r);
-            if (accum)
-                for (int64_t r = l.dst; r < l.dst + l.nrows; ++r) f((size_t)r);
+        auto rows = [&](int64_t r0, int64_t n) {
+            for (int64_t r = r0; r < r0 + n; ++r) {
+                const int32_t u = last[(size_t)r];
+                if (u >= 0 && (deps.empty() || deps.back() != u)) deps.push_back(u);
+            }
         };
-        auto add = [&](int32_t u) {
-            if (u >= 0 && (deps.empty() || deps.back() != u)) deps.push_back(u);
-        };
-        for_reads([&](size_t r) { add(last[r]); });
-        if (!scatter)
+        for (const PlanBuilder::PanelSpec &pn : l.panels)
+            for (const Seg &sg : pn.segs)
+                if (!(sg.flags & S_GATHER)) {
+                    rows(sg.src, sg.len);
+                    std::memset(gathered.data() + sg.src, 1, (size_t)sg.len);
+                }
+        if (!(l.flags & T_SCATTER) || (l.flags & T_ACCUM)) rows(l.dst, l.nrows);
+        if (!(l.flags & T_SCATTER))
             for (int64_t r = l.dst; r < l.dst + l.nrows; ++r) {
-                add(last[(size_t)r]);
-                for (int32_t u : rd[(size_t)r]) add(u);
+                if (gathered[(size_t)r]) throw ApiError(H2W_ERR_STATE, "internal: a row is written after it was read");
+                last[(size_t)r] = (int32_t)g;
             }
         std::sort(deps.begin(), deps.end());
         deps.erase(std::unique(deps.begin(), deps.end()), deps.end());
-        prod[g] = deps;
-        for_reads([&](size_t r) {
-            if (rd[r].empty() || rd[r].back() != (int32_t)g) rd[r].push_back((int32_t)g);
-        });
-        if (!scatter)
-            for (int64_t r = l.dst; r < l.dst + l.nrows; ++r) {
-                last[(size_t)r] = (int32_t)g;
-                rd[(size_t)r].clear();
-            }
-        for (int32_t u : prod[g]) {
+        prod.insert(prod.end(), deps.begin(), deps.end());
+        first[g + 1] = prod.size();
+        for (int32_t u : deps) {
             out.cnt[g] += parts[(size_t)u];
             ++ncons[(size_t)u];
         }
@@ -1813,19 +1810,23 @@ void group_deps(const std::vector<PlanBuilder::LTarget> &groups, const std::vect
     }
     out.cons.resize(at);
     for (size_t g = 0; g < ng; ++g)
-        for (int32_t u : prod[g]) out.cons[out.grp[(size_t)u].x + out.grp[(size_t)u].y++] = (uint32_t)g;
+        for (size_t e = first[g]; e < first[g + 1]; ++e) {
+            uint2 &u = out.grp[(size_t)prod[e]];
+            out.cons[u.x + u.y++] = (uint32_t)g;
+        }
 }
 
 // Cut the logical targets for the dataflow launch. Each pass is cut for the whole
-// chip: its elements over SV_CUT_CTAS, at most row_split and at least SV_CUT_MIN a
+// chip (a batch's problem for its part of it): its elements over `ctas`, at most row_split and at least SV_CUT_MIN a
 // target, so that a pass of a few large blocks near the root is not left to a few SMs
 // (an FP64 target of 16384 elements takes one SM's FP64 pipe 4 us). Large operators
 // have whole rows to spare and keep at least 8, 16 or 32 rows a target: its sources are
 // gathered once for all its rows (3D semi-nested, 2e8 entries, FP32: 262 us at 4 rows,
 // 196 at 16, 166 at 32). A block row wider than XW_CAP is cut into column parts, each
 // adding to the rows of the one before: the sums come in the same order on every run.
-constexpr int64_t SV_CUT_CTAS = 608, SV_CUT_MIN = 2048;
-void sv_build(h2w_handle *h, int64_t row_split, int32_t pid, int64_t ws0, int64_t x0, int64_t xoff, SvHost &out) {
+constexpr int SV_CUT_CTAS = 608;
+constexpr int64_t SV_CUT_MIN = 2048;
+void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t ws0, int64_t x0, int64_t xoff, SvHost &out) {
     auto bad = [](const char *what) { throw ApiError(H2W_ERR_STATE, std::string("internal: single-vector stream: ") + what); };
     PlanBuilder &pb = *h->plan;
     const int last = h->nph_total - 1;
@@ -1844,7 +1845,8 @@ void sv_build(h2w_handle *h, int64_t row_split, int32_t pid, int64_t ws0, int64_
     pb.fused = true;
     pb.xw_cap = XW_CAP;
     pb.max_rows = SV_MAX_ROWS;
-    std::vector<PlanBuilder::LTarget> groups;
+    std::vector<const PlanBuilder::LTarget *> groups;
+    std::deque<PlanBuilder::LTarget> cut;  // the column parts and what changes its flags
     struct Key { int list, hi, part; double work; };
     std::vector<Key> key;
     double pass[3][2 * 64] = {}, all = 0;
@@ -1861,13 +1863,14 @@ void sv_build(h2w_handle *h, int64_t row_split, int32_t pid, int64_t ws0, int64_
                 for (const Seg &sg : p.segs)
                     if (!(sg.flags & S_GATHER)) bad("a free target reads the workspace");
         if (xw <= XW_CAP) {
-            groups.push_back(l);
+            groups.push_back(&l);
             key.push_back({ls, l.hi, 0, w});
             continue;
         }
         const auto parts = pb.column_parts(l.panels);
         for (size_t i = 0; i < parts.size(); ++i) {
-            groups.push_back({l.dst, l.nrows, i + 1 < parts.size() ? (int32_t)T_ACCUM : l.flags, parts[i], l.lo, l.hi});
+            cut.push_back({l.dst, l.nrows, i + 1 < parts.size() ? (int32_t)T_ACCUM : l.flags, parts[i], l.lo, l.hi});
+            groups.push_back(&cut.back());
             key.push_back({ls, l.hi, (int)i, w});
         }
     }
@@ -1881,10 +1884,10 @@ void sv_build(h2w_handle *h, int64_t row_split, int32_t pid, int64_t ws0, int64_
             if (p.part != q.part) return p.part < q.part;
             return p.work > q.work;
         });
-        std::vector<PlanBuilder::LTarget> g2;
+        std::vector<const PlanBuilder::LTarget *> g2;
         std::vector<Key> k2;
         for (size_t i : ord) {
-            g2.push_back(std::move(groups[i]));
+            g2.push_back(groups[i]);
             k2.push_back(key[i]);
         }
         groups.swap(g2);
@@ -1893,13 +1896,17 @@ void sv_build(h2w_handle *h, int64_t row_split, int32_t pid, int64_t ws0, int64_
     const int64_t rows_min = all >= 128e6 ? 32 : all >= 64e6 ? 16 : all >= 16e6 ? 8 : 4;
     std::vector<int32_t> parts(groups.size());
     int64_t covered = 0;
-    for (const auto &l : groups)
-        if (l.flags & T_SCATTER) covered += l.nrows;
+    for (const auto *l : groups)
+        if (l->flags & T_SCATTER) covered += l->nrows;
     out.fused = covered == h->nv();  // else an explicit scatter follows
     for (size_t g = 0; g < groups.size(); ++g) {
-        auto &l = groups[g];
-        if (!out.fused && (l.flags & T_SCATTER)) l.flags = T_ACCUM;
-        const int64_t share = (int64_t)(pass[key[g].list][std::min(l.hi, 127)] / SV_CUT_CTAS);
+        if (!out.fused && (groups[g]->flags & T_SCATTER)) {
+            cut.push_back(*groups[g]);
+            cut.back().flags = T_ACCUM;
+            groups[g] = &cut.back();
+        }
+        const auto &l = *groups[g];
+        const int64_t share = (int64_t)(pass[key[g].list][std::min(l.hi, 127)] / ctas);
         pb.row_split = std::min(row_split, std::max(SV_CUT_MIN, share));
         pb.min_rows = rows_min;
         const size_t t0 = pb.T.size();
@@ -1973,13 +1980,13 @@ void sv_build(h2w_handle *h, int64_t row_split, int32_t pid, int64_t ws0, int64_
 
 // Streams of one or several operators (the problems of a batch, their deadlines
 // aligned at the leaf pass by shift) as one on the device: targets by list, deadline
-// and work, which keeps each operator's own dependency order.
+// and work, which keeps each operator's own dependency order. Matrix offsets stay each
+// operator's own.
 void sv_upload(std::vector<SvHost> &v, const std::vector<int> &shift, SvStream &d, cudaStream_t st) {
     struct Ref { int32_t list, key; double work; int32_t p, t; };
     std::vector<Ref> ref;
     SvHost all;
     std::vector<uint32_t> g0(v.size()), i0(v.size());
-    std::vector<int64_t> a0(v.size());
     double work[3] = {0, 0, 0};
     for (size_t p = 0; p < v.size(); ++p) {
         SvHost &s = v[p];
@@ -1987,13 +1994,11 @@ void sv_upload(std::vector<SvHost> &v, const std::vector<int> &shift, SvStream &
             throw ApiError(H2W_ERR_STATE, "internal: single-vector stream too large");
         g0[p] = (uint32_t)all.grp.size();
         i0[p] = (uint32_t)all.idx.size();
-        a0[p] = all.opn;
         const uint32_t c0 = (uint32_t)all.cons.size();
         for (const uint2 &g : s.grp) all.grp.push_back(make_uint2(g.x + c0, g.y));
         for (uint32_t c : s.cons) all.cons.push_back(c + g0[p]);
         all.idx.insert(all.idx.end(), s.idx.begin(), s.idx.end());
         all.cnt.insert(all.cnt.end(), s.cnt.begin(), s.cnt.end());
-        all.opn += s.opn;
         all.max_w = std::max(all.max_w, s.max_w);
         for (size_t t = 0; t < s.hdr.size(); ++t) {
             ref.push_back({s.list[t], s.key[t] + 4096 * shift[p], s.work[t], (int32_t)p, (int32_t)t});
@@ -2010,7 +2015,6 @@ void sv_upload(std::vector<SvHost> &v, const std::vector<int> &shift, SvStream &
     for (int l = 0; l < 3; ++l) d.list[l][0] = d.list[l][1] = 0;
     for (const Ref &r : ref) {
         SvHdr h = v[(size_t)r.p].hdr[(size_t)r.t];
-        h.a += a0[(size_t)r.p];
         h.grp += g0[(size_t)r.p];
         h.idx0 += i0[(size_t)r.p];
         all.hdr.push_back(h);
@@ -2078,7 +2082,7 @@ void realize_single(h2w_handle *h, int64_t row_split) {
     pb.S = std::vector<Seg>();
     {
         std::vector<SvHost> sv(1);
-        sv_build(h, row_split, 0, 0, 0, h->xoff(), sv[0]);
+        sv_build(h, row_split, SV_CUT_CTAS, 0, 0, 0, h->xoff(), sv[0]);
         h->fused_sv = sv[0].fused;
         h->ops_n = sv[0].opn;
         // in a product with the far field on the fly, list 0 from the passes after the upward ones
@@ -2087,7 +2091,7 @@ void realize_single(h2w_handle *h, int64_t row_split) {
             return sv[0].list[t] == 0 && sv[0].key[t] < 4096 * h->tree.nL;
         });
         h->d_sslices.upload(sv[0].slices, st);
-        h->op32s_ready = h->op64s_ready = false;
+        h->op32s_ready = false;
         h->d_op32s.reset();
         sv_upload(sv, {0}, h->sv, st);
         // The FP64 copy is made with the operator, a second one in memory: only where that
@@ -2095,12 +2099,11 @@ void realize_single(h2w_handle *h, int64_t row_split) {
         // again); else FP64 products stay on the packed operator and the cooperative launch.
         size_t fr = 0, tot = 0;
         const size_t need = (size_t)std::max<int64_t>(h->ops_n, 4) * 8;
-        if (h->d_op64s.n * 8 != need) h->d_op64s.reset();
+        h->d_op64s.reset();
         CK(cudaMemGetInfo(&fr, &tot));
-        if (h->d_op64s.p || fr / 4 >= need) {
-            if (!h->d_op64s.p) h->d_op64s.alloc(need / 8);
+        if (fr / 4 >= need) {
+            h->d_op64s.alloc(need / 8);
             CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 6, h->d_op64s.p, st));
-            h->op64s_ready = true;
         }
     }
     CK(cudaStreamSynchronize(st));
@@ -2931,7 +2934,7 @@ void run_matvec_f64(h2w_handle *h, const double *dx, double *dy, cudaStream_t st
                     bool df = false) {
     const int32_t *perm = permuted ? nullptr : h->d_perm.p;
     const int nph = (int)h->phases.size();
-    const bool flow = h->coop && h->dataflow && h->op64s_ready;
+    const bool flow = h->coop && h->dataflow && h->d_op64s.p;
     auto far = [&] {
         prof_launch(h, df ? H2W_PREC_DF64 : H2W_PREC_FP64, FLY_PHASE, st, [&] {
             if (df)
@@ -3049,6 +3052,51 @@ void run_matvec_f32(h2w_handle *h, const double *dx, double *dy, cudaStream_t st
 // (kind, precision, m, rp, nrhs, tol) and rebuilt when any device buffer was
 // reallocated since the capture. Returns nullptr when capture is unavailable
 // (the caller then runs the host loop). kps: kernels one step launches.
+// A graph whose one node runs body(s, cond), one step, while the condition is set.
+// kps: kernels a step launches. False when capture is unavailable.
+template <class F>
+bool capture_loop(cudaStream_t st, cudaGraph_t &graph, cudaGraphExec_t &exec, int64_t &kps, F &&body) {
+    graph = nullptr;
+    exec = nullptr;
+    const int64_t c0 = launch_count();
+    bool capturing = false;
+    try {
+        CK(cudaGraphCreate(&graph, 0));
+        cudaGraphConditionalHandle cond;
+        CK(cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault));
+        // zero-initialised storage (the struct's union has no default constructor in C++)
+        alignas(cudaGraphNodeParams) unsigned char npbuf[sizeof(cudaGraphNodeParams)] = {};
+        cudaGraphNodeParams *np = reinterpret_cast<cudaGraphNodeParams *>(npbuf);
+        np->type = cudaGraphNodeTypeConditional;
+        np->conditional.handle = cond;
+        np->conditional.type = cudaGraphCondTypeWhile;
+        np->conditional.size = 1;
+        cudaGraphNode_t node;
+        CK(cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, np));
+        cudaGraph_t bodyg = np->conditional.phGraph_out[0];
+        CK(cudaStreamBeginCaptureToGraph(st, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+        capturing = true;
+        body(st, cond);
+        cudaGraph_t out = nullptr;
+        capturing = false;
+        CK(cudaStreamEndCapture(st, &out));
+        CK(cudaGraphInstantiate(&exec, graph, 0));
+    } catch (const std::exception &) {
+        if (capturing) {
+            cudaGraph_t out = nullptr;
+            cudaStreamEndCapture(st, &out);
+        }
+        cudaGetLastError();
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+        count_launch(c0 - launch_count());
+        return false;
+    }
+    kps = launch_count() - c0;
+    count_launch(-kps);  // the captured launches run when the graph does
+    return true;
+}
+
 // Whether loop_graph holds a valid captured step for this key (no capture needed).
 bool loop_graph_cached(h2w_handle *h, int kind, int prec, int m, int rp, int nrhs) {
     if (!h->use_graphs || h->graph_failed || h->prof) return false;
@@ -3077,43 +3125,10 @@ cudaGraphExec_t loop_graph(h2w_handle *h, int kind, int prec, int m, int rp, int
     }
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    const int64_t c0 = launch_count();
-    bool capturing = false;
-    try {
-        CK(cudaGraphCreate(&graph, 0));
-        cudaGraphConditionalHandle cond;
-        CK(cudaGraphConditionalHandleCreate(&cond, graph, 1, cudaGraphCondAssignDefault));
-        // zero-initialised storage (the struct's union has no default constructor in C++)
-        alignas(cudaGraphNodeParams) unsigned char npbuf[sizeof(cudaGraphNodeParams)] = {};
-        cudaGraphNodeParams *np = reinterpret_cast<cudaGraphNodeParams *>(npbuf);
-        np->type = cudaGraphNodeTypeConditional;
-        np->conditional.handle = cond;
-        np->conditional.type = cudaGraphCondTypeWhile;
-        np->conditional.size = 1;
-        cudaGraphNode_t node;
-        CK(cudaGraphAddNode(&node, graph, nullptr, nullptr, 0, np));
-        cudaGraph_t bodyg = np->conditional.phGraph_out[0];
-        CK(cudaStreamBeginCaptureToGraph(h->stream, bodyg, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        capturing = true;
-        body(h->stream, cond);
-        cudaGraph_t out = nullptr;
-        capturing = false;
-        CK(cudaStreamEndCapture(h->stream, &out));
-        CK(cudaGraphInstantiate(&exec, graph, 0));
-    } catch (const std::exception &) {
-        if (capturing) {
-            cudaGraph_t out = nullptr;
-            cudaStreamEndCapture(h->stream, &out);
-        }
-        cudaGetLastError();
-        if (exec) cudaGraphExecDestroy(exec);
-        if (graph) cudaGraphDestroy(graph);
-        count_launch(c0 - launch_count());
+    if (!capture_loop(h->stream, graph, exec, kps, body)) {
         h->graph_failed = true;
         return nullptr;
     }
-    kps = launch_count() - c0;
-    count_launch(-kps);  // the captured launches run when the graph does
     h->loops.push_back({kind, prec, m, rp, nrhs, gen, graph, exec, kps});
     return exec;
 }
@@ -3618,11 +3633,30 @@ struct h2w_batch {
     int64_t Ntot = 0;
     std::vector<int64_t> off, wsoff;        // P+1: vector and workspace offsets
     std::vector<int> unfused;               // problems whose leaf rows need an explicit scatter
+    // one dataflow stream of all problems' targets (sv.cu) on their operator copies
+    SvStream sv;
+    DBuf<int64_t> vshift;                   // per problem: workspace offset minus vector offset
+    DBuf<int32_t> perm32;                   // perm_all for the kernel
+    DBuf<const double *> A64;
+    DBuf<const float *> A32;
+    std::vector<std::unique_ptr<DBuf<double>>> op64;  // made with the batch
+    std::vector<std::unique_ptr<DBuf<float>>> op32;   // made on the first FP32 product
+    std::vector<DBuf<int64_t>> slices;
+    std::vector<int64_t> opn;
+    int64_t xoff = 0;                       // the input in leaf order behind the workspace rows
+    // the FP64 products of a batch whose copies had no room: one launch with grid barriers
+    // on the packed operators
     DBuf<int64_t> roff, blob, pstart;
     int nphase = 0;
-    DBuf<BatchProb> tab64_orig, tab64_leaf, tab32_orig, tab32_leaf;
+    std::vector<int> unfused_ph;
+    DBuf<BatchProb> tab64_orig, tab64_leaf;
     DBuf<double> ws64;
     DBuf<float> ws32;
+    // the Arnoldi loop as a graph, per (precision, m)
+    struct Loop { int prec, m; uint64_t gen; cudaGraph_t graph; cudaGraphExec_t exec; int64_t kps; };
+    std::vector<Loop> loops;
+    bool graph_failed = false;
+    DBuf<double> tol;
     DBuf<unsigned> bar;
     DBuf<int32_t> errf;
     DBuf<int64_t> perm_all;                 // global leaf position -> global original position
@@ -3667,8 +3701,40 @@ void batch_check_error(h2w_batch *b) {
     if (e) {
         CK(cudaMemsetAsync(b->errf.p, 0, 4, b->stream));
         CK(cudaMemsetAsync(b->bar.p, 0, 8, b->stream));
-        throw ApiError(H2W_ERR_CUDA, "batch matvec: a grid-barrier wait ran out (device error flag)");
+        throw ApiError(H2W_ERR_CUDA, "batch matvec: a wait on the device ran out (device error flag " + std::to_string(e) + ")");
     }
+}
+
+template <class T>
+cudaError_t batch_sv(h2w_batch *b, const T *const *A, T *ws, const SvConf &conf, const double *x, double *y, bool leaf,
+                     const int32_t *active) {
+    SvArgs<T> a{};
+    a.hdr = b->sv.hdr.p;
+    a.idx = b->sv.idx.p;
+    a.cons = b->sv.cons.p;
+    a.grp = b->sv.grp.p;
+    a.active = active;
+    a.vshift = b->vshift.p;
+    a.Ap = A;
+    for (int l = 0; l < 3; ++l) {
+        a.l0[l] = b->sv.list[l][0];
+        a.l1[l] = b->sv.list[l][1];
+    }
+    a.na = b->sv.share;
+    a.ngrp = b->sv.ngrp;
+    a.ws = ws;
+    a.nzero = a.xoff = b->xoff;
+    a.nx = b->Ntot;
+    a.xin = x;
+    a.perm = leaf ? nullptr : b->perm32.p;
+    a.yout = y;
+    a.cnt = b->sv.cnt.p;
+    a.rem = b->sv.rem.p;
+    a.ctr = b->sv.ctr.p;
+    a.bar = b->bar.p;
+    a.err = b->errf.p;
+    a.prep = 1;
+    return launch_sv(a, conf, b->stream);
 }
 
 // y = A x for every problem: x, y concatenated, leaf order (leaf) or each
@@ -3677,27 +3743,33 @@ void run_batch(h2w_batch *b, int prec, const double *x, double *y, bool leaf, co
     cudaStream_t st = b->stream;
     const bool f32 = prec == H2W_PREC_FP32;
     const int P = (int)b->hs.size();
-    if (f32 && !b->tab32_orig.p) {
-        if (!b->ws32.p) b->ws32.alloc((size_t)b->wsoff[(size_t)P]);
-        std::vector<BatchProb> to(P), tl(P);
+    if (f32 && b->op32.empty()) {
+        std::vector<std::unique_ptr<DBuf<float>>> op((size_t)P);
+        std::vector<const float *> tab((size_t)P);
         for (int p = 0; p < P; ++p) {
-            ensure_f32(b->hs[(size_t)p]);
-            to[(size_t)p] = {b->hs[(size_t)p]->d_op32.p, b->ws32.p + b->wsoff[(size_t)p], b->hs[(size_t)p]->d_perm.p,
-                             b->off[(size_t)p]};
-            tl[(size_t)p] = to[(size_t)p];
-            tl[(size_t)p].perm = nullptr;
+            op[(size_t)p].reset(new DBuf<float>());
+            op[(size_t)p]->alloc((size_t)std::max<int64_t>(b->opn[(size_t)p], 4));
+            CK(launch_sv_slices(b->hs[(size_t)p]->d_op.p, b->slices[(size_t)p].p, (int64_t)b->slices[(size_t)p].n / 6,
+                                op[(size_t)p]->p, st));
+            tab[(size_t)p] = op[(size_t)p]->p;
         }
-        b->tab32_orig.upload(to, st);
-        b->tab32_leaf.upload(tl, st);
+        b->ws32.alloc((size_t)(b->xoff + b->Ntot));
+        b->A32.upload(tab, st);
+        CK(cudaStreamSynchronize(st));
+        b->op32.swap(op);
     }
-    const BatchProb *tab = f32 ? (leaf ? b->tab32_leaf.p : b->tab32_orig.p) : (leaf ? b->tab64_leaf.p : b->tab64_orig.p);
-    if (f32) CK(cudaMemsetAsync(b->ws32.p, 0, (size_t)b->wsoff[(size_t)P] * 4, st));
-    else CK(cudaMemsetAsync(b->ws64.p, 0, (size_t)b->wsoff[(size_t)P] * 8, st));
-    if (f32)
-        CK(launch_brgb_f32(b->roff.p, b->blob.p, b->pstart.p, b->nphase, tab, active, x, y, b->bar.p, b->errf.p, st));
-    else
-        CK(launch_brgb_f64(b->roff.p, b->blob.p, b->pstart.p, b->nphase, tab, active, x, y, b->bar.p, b->errf.p, st));
-    for (int p : b->unfused) {
+    const std::vector<int> *unfused = &b->unfused;
+    if (f32) {
+        CK(batch_sv<float>(b, b->A32.p, b->ws32.p, b->sv.f32, x, y, leaf, active));
+    } else if (b->A64.p) {
+        CK(batch_sv<double>(b, b->A64.p, b->ws64.p, b->sv.f64, x, y, leaf, active));
+    } else {
+        CK(cudaMemsetAsync(b->ws64.p, 0, (size_t)b->wsoff[(size_t)P] * 8, st));
+        CK(launch_brgb_f64(b->roff.p, b->blob.p, b->pstart.p, b->nphase, leaf ? b->tab64_leaf.p : b->tab64_orig.p,
+                           active, x, y, b->bar.p, b->errf.p, st));
+        unfused = &b->unfused_ph;
+    }
+    for (int p : *unfused) {
         h2w_handle *h = b->hs[(size_t)p];
         const int64_t N = h->tree.N, o = b->off[(size_t)p], w0 = b->wsoff[(size_t)p] + h->yperm_off;
         if (f32) {
@@ -3708,6 +3780,73 @@ void run_batch(h2w_batch *b, int prec, const double *x, double *y, bool leaf, co
             else CK(launch_scatter_f64(b->ws64.p + w0, y + o, h->d_perm.p, N, st));
         }
     }
+}
+
+// The merged stream of a batch's FP64 products by phases: records with the problem
+// index in the flags, phases aligned at the leaf end.
+void batch_phased(h2w_batch *b) {
+    const int P = (int)b->hs.size();
+    struct Rec { int slot; double size; std::vector<int64_t> words; };
+    std::vector<std::vector<Rec>> per((size_t)P);
+    size_t maxph = 0;
+    std::vector<size_t> nph((size_t)P);
+    for (int p = 0; p < P; ++p) {
+        h2w_handle *h = b->hs[(size_t)p];
+        PlanBuilder &pb = *h->plan;
+        std::vector<Phase> ph;
+        bool fused = true;
+        pb.realize(h->row_split, 4, XW_CAP);
+        assign_phases(h, pb, h->nph_total, ph, fused);
+        validate_plan(pb, h, ph);
+        if (!fused) b->unfused_ph.push_back(p);
+        for (Target &t : pb.T) t.flags |= (p << 8);
+        std::vector<int64_t> ro, bl, ps;
+        pack_records(pb, ph, ro, bl, ps);
+        first_writers_overwrite(ro, bl, h->ws_n);
+        nph[(size_t)p] = ph.size();
+        maxph = std::max(maxph, ph.size());
+        for (size_t j = 0; j < ph.size(); ++j)
+            for (int64_t t = ph[j].t0; t < ph[j].t1; ++t) {
+                const Target &tg = pb.T[(size_t)t];
+                Rec r;
+                r.slot = (int)j;
+                r.size = (double)tg.nrows * (double)tg.xw;
+                r.words.assign(bl.begin() + ro[(size_t)t], bl.begin() + ro[(size_t)t + 1]);
+                per[(size_t)p].push_back(std::move(r));
+            }
+        pb.T = std::vector<Target>();
+        pb.P = std::vector<Panel>();
+        pb.S = std::vector<Seg>();
+    }
+    // merged phases, aligned at the leaf end; heaviest first within a phase
+    std::vector<std::vector<std::pair<double, const Rec *>>> slots(maxph);
+    for (int p = 0; p < P; ++p)
+        for (const Rec &r : per[(size_t)p])
+            slots[(size_t)r.slot + (maxph - nph[(size_t)p])].push_back({r.size, &r});
+    std::vector<int64_t> roff{0}, blob, pstart;
+    for (auto &sl : slots) {
+        std::stable_sort(sl.begin(), sl.end(), [](const auto &a, const auto &c) { return a.first > c.first; });
+        pstart.push_back((int64_t)roff.size() - 1);
+        for (auto &e : sl) {
+            blob.insert(blob.end(), e.second->words.begin(), e.second->words.end());
+            roff.push_back((int64_t)blob.size());
+        }
+    }
+    pstart.push_back((int64_t)roff.size() - 1);
+    b->nphase = (int)maxph;
+    cudaStream_t st = b->stream;
+    b->roff.upload(roff, st);
+    b->blob.upload(blob, st);
+    b->pstart.upload(pstart, st);
+    std::vector<BatchProb> to((size_t)P), tl((size_t)P);
+    for (int p = 0; p < P; ++p) {
+        h2w_handle *h = b->hs[(size_t)p];
+        to[(size_t)p] = {h->d_op.p, b->ws64.p + b->wsoff[(size_t)p], h->d_perm.p, b->off[(size_t)p]};
+        tl[(size_t)p] = to[(size_t)p];
+        tl[(size_t)p].perm = nullptr;
+    }
+    b->tab64_orig.upload(to, st);
+    b->tab64_leaf.upload(tl, st);
 }
 
 GmresSeg gms_state(h2w_batch *b, int m) {
@@ -3724,6 +3863,7 @@ GmresSeg gms_state(h2w_batch *b, int m) {
         b->part.alloc((size_t)b->nblk * (m + 1));
         b->hsum.alloc((size_t)P * (m + 1));
         b->y.alloc((size_t)P * (m + 1));
+        if (!b->tol.p) b->tol.alloc(1);
         b->g_m = m;
     }
     GmresSeg g;
@@ -3744,6 +3884,7 @@ GmresSeg gms_state(h2w_batch *b, int m) {
     g.bprob = b->bprob.p;
     g.brow = b->brow.p;
     g.pblk = b->pblk.p;
+    g.tolp = b->tol.p;
     g.Ntot = N;
     g.m = m;
     g.P = P;
@@ -3759,6 +3900,7 @@ int gms_run(h2w_batch *b, const double *bl, double *xl, int max_iter, double tol
     const int P = (int)b->hs.size();
     GmresSeg g = gms_state(b, max_iter);
     cudaStream_t st = b->stream;
+    CK(cudaMemcpyAsync(b->tol.p, &tol, 8, cudaMemcpyHostToDevice, st));  // read by the steps
     CK(gms_norms(g, bl, g.normb, 1, st));
     if (x0_zero) {
         CK(gms_start(g, bl, nullptr, tol, st));
@@ -3774,13 +3916,50 @@ int gms_run(h2w_batch *b, const double *bl, double *xl, int max_iter, double tol
             if (conv[(size_t)p] == -1) return false;
         return true;
     };
-    bool done = read_conv();
     int last = -1;
-    for (int i = 0; i < max_iter && !done; ++i) {
-        run_batch(b, prec, g.vcur, g.w, true, g.conv);  // converged problems are skipped
-        CK(gms_arnoldi(g, tol, st));
-        last = i;
-        done = read_conv();
+    // the steps as one while-loop graph launch (as loop_graph for one operator); problems
+    // that have converged are skipped by every kernel of a step
+    h2w_batch::Loop *loop = nullptr;
+    for (size_t i = 0; i < b->loops.size(); ++i) {
+        h2w_batch::Loop &L = b->loops[i];
+        if (L.prec != prec || L.m != max_iter) continue;
+        if (L.gen == g_alloc_gen.load()) {
+            loop = &L;
+        } else {  // a buffer was reallocated since the capture
+            cudaGraphExecDestroy(L.exec);
+            cudaGraphDestroy(L.graph);
+            b->loops.erase(b->loops.begin() + (long)i);
+        }
+        break;
+    }
+    if (!loop && !b->graph_failed) {
+        run_batch(b, prec, g.vcur, g.w, true, g.conv);  // its buffers, outside the capture
+        h2w_batch::Loop L{prec, max_iter, g_alloc_gen.load(), nullptr, nullptr, 0};
+        if (capture_loop(st, L.graph, L.exec, L.kps, [&](cudaStream_t, cudaGraphConditionalHandle c) {
+                run_batch(b, prec, g.vcur, g.w, true, g.conv);
+                CK(gms_arnoldi(g, &c, st));
+            })) {
+            b->loops.push_back(L);
+            loop = &b->loops.back();
+        } else {
+            b->graph_failed = true;
+        }
+    }
+    if (loop) {
+        CK(cudaGraphLaunch(loop->exec, st));
+        int32_t it2[2];
+        CK(cudaMemcpyAsync(it2, g.iter, 8, cudaMemcpyDeviceToHost, st));
+        read_conv();
+        count_launch(loop->kps * it2[1]);
+        last = it2[1] - 1;
+    } else {
+        bool done = read_conv();
+        for (int i = 0; i < max_iter && !done; ++i) {
+            run_batch(b, prec, g.vcur, g.w, true, g.conv);
+            CK(gms_arnoldi(g, nullptr, st));
+            last = i;
+            done = read_conv();
+        }
     }
     int kmax = -1;
     for (int p = 0; p < P; ++p) {
@@ -5017,6 +5196,8 @@ int h2w_batch_create(h2w_handle *const *handles, int n, h2w_batch **out) {
     b->device = b->hs[0]->cfg.device;
     int rc = bguarded(b, [&] {
         CK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
+        const char *eg = getenv("H2W_GRAPH");
+        if (eg && std::string(eg) == "0") b->graph_failed = true;
         const int P = n;
         b->off.assign((size_t)P + 1, 0);
         b->wsoff.assign((size_t)P + 1, 0);
@@ -5025,86 +5206,70 @@ int h2w_batch_create(h2w_handle *const *handles, int n, h2w_batch **out) {
             b->wsoff[(size_t)p + 1] = b->wsoff[(size_t)p] + b->hs[(size_t)p]->ws_n;
         }
         b->Ntot = b->off[(size_t)P];
-        // per problem: its single-vector stream with the problem index in the flags
-        struct Rec { int slot; double size; std::vector<int64_t> words; };
-        std::vector<std::vector<Rec>> per((size_t)P);
-        size_t maxph = 0;
-        std::vector<size_t> nph((size_t)P);
-        for (int p = 0; p < P; ++p) {
-            h2w_handle *h = b->hs[(size_t)p];
-            PlanBuilder &pb = *h->plan;
-            std::vector<Phase> ph;
-            bool fused = true;
-            pb.realize(h->row_split, 4, XW_CAP);
-            assign_phases(h, pb, h->nph_total, ph, fused);
-            validate_plan(pb, h, ph);
-            if (!fused) b->unfused.push_back(p);
-            for (Target &t : pb.T) t.flags |= (p << 8);
-            std::vector<int64_t> ro, bl, ps;
-            pack_records(pb, ph, ro, bl, ps);
-            first_writers_overwrite(ro, bl, h->ws_n);
-            nph[(size_t)p] = ph.size();
-            maxph = std::max(maxph, ph.size());
-            for (size_t j = 0; j < ph.size(); ++j)
-                for (int64_t t = ph[j].t0; t < ph[j].t1; ++t) {
-                    const Target &tg = pb.T[(size_t)t];
-                    Rec r;
-                    r.slot = (int)j;
-                    r.size = (double)tg.nrows * (double)tg.xw;
-                    r.words.assign(bl.begin() + ro[(size_t)t], bl.begin() + ro[(size_t)t + 1]);
-                    per[(size_t)p].push_back(std::move(r));
-                }
-            pb.T = std::vector<Target>();
-            pb.P = std::vector<Panel>();
-            pb.S = std::vector<Seg>();
-        }
-        // merged phases, aligned at the leaf end; heaviest first within a phase
-        std::vector<std::vector<std::pair<double, const Rec *>>> slots(maxph);
-        for (int p = 0; p < P; ++p)
-            for (const Rec &r : per[(size_t)p])
-                slots[(size_t)r.slot + (maxph - nph[(size_t)p])].push_back({r.size, &r});
-        std::vector<int64_t> roff{0}, blob, pstart;
-        for (auto &sl : slots) {
-            std::stable_sort(sl.begin(), sl.end(), [](const auto &a, const auto &c) { return a.first > c.first; });
-            pstart.push_back((int64_t)roff.size() - 1);
-            for (auto &e : sl) {
-                blob.insert(blob.end(), e.second->words.begin(), e.second->words.end());
-                roff.push_back((int64_t)blob.size());
-            }
-        }
-        pstart.push_back((int64_t)roff.size() - 1);
-        b->nphase = (int)maxph;
         cudaStream_t st = b->stream;
-        b->roff.upload(roff, st);
-        b->blob.upload(blob, st);
-        b->pstart.upload(pstart, st);
-        b->ws64.alloc((size_t)b->wsoff[(size_t)P]);
-        std::vector<BatchProb> to((size_t)P), tl((size_t)P);
-        for (int p = 0; p < P; ++p) {
-            h2w_handle *h = b->hs[(size_t)p];
-            to[(size_t)p] = {h->d_op.p, b->ws64.p + b->wsoff[(size_t)p], h->d_perm.p, b->off[(size_t)p]};
-            tl[(size_t)p] = to[(size_t)p];
-            tl[(size_t)p].perm = nullptr;
+        b->xoff = pad4(b->wsoff[(size_t)P]);
+        if (b->xoff + b->Ntot >= (int64_t)UINT32_MAX || b->Ntot >= (int64_t)INT32_MAX)
+            throw ApiError(H2W_ERR_ARG, "batch too large (2^32 workspace rows and points at most)");
+        {
+            std::vector<SvHost> sv((size_t)P);
+            std::vector<int> shift((size_t)P);
+            int most = 0;
+            for (h2w_handle *h : b->hs) most = std::max(most, h->nph_total);
+            b->slices = std::vector<DBuf<int64_t>>((size_t)P);
+            std::vector<int64_t> vs((size_t)P);
+            for (int p = 0; p < P; ++p) {
+                h2w_handle *h = b->hs[(size_t)p];
+                sv_build(h, h->row_split, std::max(1, SV_CUT_CTAS / P), p, b->wsoff[(size_t)p], b->off[(size_t)p], b->xoff, sv[(size_t)p]);
+                shift[(size_t)p] = most - h->nph_total;
+                if (!sv[(size_t)p].fused) b->unfused.push_back(p);
+                b->slices[(size_t)p].upload(sv[(size_t)p].slices, st);
+                b->opn.push_back(sv[(size_t)p].opn);
+                vs[(size_t)p] = b->wsoff[(size_t)p] - b->off[(size_t)p];
+            }
+            sv_upload(sv, shift, b->sv, st);
+            b->vshift.upload(vs, st);
+            CK(cudaStreamSynchronize(st));
         }
-        b->tab64_orig.upload(to, st);
-        b->tab64_leaf.upload(tl, st);
+        b->ws64.alloc((size_t)(b->xoff + b->Ntot));
+        // FP64 copies where they leave the room of the FP32 ones and as much again
+        size_t fr = 0, tot = 0;
+        int64_t all = 0;
+        for (int64_t v : b->opn) all += std::max<int64_t>(v, 4);
+        CK(cudaMemGetInfo(&fr, &tot));
+        if (fr / 2 >= (size_t)all * 8) {
+            std::vector<const double *> tab((size_t)P);
+            for (int p = 0; p < P; ++p) {
+                b->op64.emplace_back(new DBuf<double>());
+                b->op64.back()->alloc((size_t)std::max<int64_t>(b->opn[(size_t)p], 4));
+                CK(launch_sv_slices(b->hs[(size_t)p]->d_op.p, b->slices[(size_t)p].p, (int64_t)b->slices[(size_t)p].n / 6,
+                                    b->op64.back()->p, st));
+                tab[(size_t)p] = b->op64.back()->p;
+            }
+            b->A64.upload(tab, st);
+            CK(cudaStreamSynchronize(st));
+        } else {
+            batch_phased(b);
+        }
         std::vector<int64_t> pa((size_t)b->Ntot);
         for (int p = 0; p < P; ++p) {
             const auto &pm = b->hs[(size_t)p]->tree.perm;
             for (size_t t = 0; t < pm.size(); ++t) pa[(size_t)b->off[(size_t)p] + t] = b->off[(size_t)p] + pm[t];
         }
         b->perm_all.upload(pa, st);
+        const std::vector<int32_t> pa32(pa.begin(), pa.end());
+        b->perm32.upload(pa32, st);
         b->bar.alloc(2);
         CK(cudaMemsetAsync(b->bar.p, 0, 8, st));
         b->errf.alloc(1);
         CK(cudaMemsetAsync(b->errf.p, 0, 4, st));
         for (DBuf<double> *v : {&b->sx, &b->sy, &b->bl, &b->xl, &b->r, &b->d}) v->alloc((size_t)b->Ntot);
-        // segmented GMRES blocks: about 2048 rows each, never across problems
+        // segmented GMRES blocks: about 512 rows each, never across problems (2048 left two
+        // thirds of the SMs without rows in a batch of 1e5)
         std::vector<int32_t> bprob, pblk{0};
         std::vector<int64_t> brow{0};
         for (int p = 0; p < P; ++p) {
             const int64_t Np = b->hs[(size_t)p]->tree.N;
-            const int64_t nb = std::max<int64_t>(1, (Np + 2047) / 2048);
+            const int64_t nb = std::max<int64_t>(1, (Np + 511) / 512);
             for (int64_t q = 0; q < nb; ++q) {
                 bprob.push_back(p);
                 brow.push_back(b->off[(size_t)p] + std::min(Np, (q + 1) * ((Np + nb - 1) / nb)));
@@ -5134,6 +5299,10 @@ int h2w_batch_destroy(h2w_batch *b) {
     if (!b) return H2W_OK;
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
+    for (auto &L : b->loops) {
+        cudaGraphExecDestroy(L.exec);
+        cudaGraphDestroy(L.graph);
+    }
     cudaStream_t st = b->stream;
     delete b;
     if (st) cudaStreamDestroy(st);

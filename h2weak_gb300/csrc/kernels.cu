@@ -769,12 +769,6 @@ cudaError_t launch_brgb_f64(const int64_t *roff, const int64_t *blob, const int6
                             unsigned *bar, int32_t *err, cudaStream_t st) {
     return launch_brgb_t<double>(roff, blob, pstart, nphase, probs, active, xin, yout, bar, err, st);
 }
-cudaError_t launch_brgb_f32(const int64_t *roff, const int64_t *blob, const int64_t *pstart, int nphase,
-                            const BatchProb *probs, const int32_t *active, const double *xin, double *yout,
-                            unsigned *bar, int32_t *err, cudaStream_t st) {
-    return launch_brgb_t<float>(roff, blob, pstart, nphase, probs, active, xin, yout, bar, err, st);
-}
-
 cudaError_t launch_brg_f64(const int64_t *roff, const int64_t *blob, int64_t t0, int64_t t1, const double *A,
                            double *ws, const double *xin, double *yout, const int32_t *perm, cudaStream_t st) {
     return launch_brg_t<double>(roff, blob, t0, t1, A, ws, xin, yout, perm, st);
@@ -926,7 +920,7 @@ __device__ void gm_dots_all(const GmresDev &g, const GmCols &C, int i, bool firs
 __global__ void __launch_bounds__(GMS_THREADS)
     gm_step(GmresDev g, int ws_rows, int vcap, cudaGraphConditionalHandle hnd, int cond) {
     extern __shared__ double gsh[];
-    __shared__ double s_hn, sh[32];
+    __shared__ double s_hn, s_ih, sh[32];
     double *h1 = gsh, *h2 = h1 + g.m + 1, *red = h2 + g.m + 1, *wsh = red + g.m + 1 + GMS_WARPS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int i = *g.iter;
@@ -963,14 +957,17 @@ __global__ void __launch_bounds__(GMS_THREADS)
         double s = 0.0;
         for (int b = lane; b < g.nblk; b += 32) s += __ldcg(g.part + 2 * ps + b);
         s = warp_sum(s);
-        if (lane == 0) s_hn = sqrt(s);
+        if (lane == 0) {
+            s_hn = sqrt(s);
+            s_ih = 1.0 / s_hn;
+        }
     }
     __syncthreads();
     const double hn = s_hn;
     // the first warp of CTA 0 does the rotations meanwhile
     const bool rot = blockIdx.x == 0 && warp == 0;
     if (!rot) {
-        const double ih = 1.0 / hn;
+        const double ih = s_ih;
         const int first = blockIdx.x == 0 ? 32 : 0;
         double *Vn = g.V + (size_t)(i + 1) * g.N + r0;
         for (int t = tid - first; t < rows; t += GMS_THREADS - first) {
@@ -1087,9 +1084,16 @@ __global__ void gm_start_fin(GmresDev g) {
         r2 += g.part[b];
         b2 += g.part[g.nblk + b];
     }
-    const double beta = sqrt(block_sum(r2, sh));
-    double normb = sqrt(block_sum(b2, sh));
-    if (normb == 0.0) normb = 1.0;
+    r2 = block_sum(r2, sh);
+    b2 = block_sum(b2, sh);
+    __shared__ double s_v[3];
+    if (threadIdx.x == 0) {  // one root and quotient a CTA: the FP64 pipe is slow at them
+        s_v[0] = sqrt(r2);
+        s_v[1] = 1.0 / s_v[0];
+        s_v[2] = b2 == 0.0 ? 1.0 : sqrt(b2);
+    }
+    __syncthreads();
+    const double beta = s_v[0], ib = s_v[1], normb = s_v[2];
     if (blockIdx.x == 0) {
         for (int k = threadIdx.x; k <= g.m; k += blockDim.x) {
             g.s[k] = k == 0 ? beta : 0.0;
@@ -1105,7 +1109,6 @@ __global__ void gm_start_fin(GmresDev g) {
             g.iter[1] = 0;  // Arnoldi steps taken
         }
     }
-    const double ib = 1.0 / beta;
     int64_t r0, r1;
     gm_rows(g.N, g.nblk, r0, r1);
     for (int64_t t = r0 + threadIdx.x; t < r1; t += blockDim.x) {
@@ -1132,7 +1135,7 @@ __global__ void gm_backsub(GmresDev g, double *__restrict__ y) {
     for (int i = k; i >= 0; --i) {
         const double *Hc = g.H + (size_t)i * (g.m + 1);
         __syncthreads();
-        const double yi = ysh[i] / Hc[i];
+        const double yi = ysh[i] / Hc[i];  // (every thread: they wait for it anyway)
         __syncthreads();
         for (int j = threadIdx.x; j < i; j += blockDim.x) ysh[j] = __dsub_rn(ysh[j], __dmul_rn(Hc[j], yi));
         if (threadIdx.x == 0) ysh[i] = yi;

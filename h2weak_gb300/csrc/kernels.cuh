@@ -88,7 +88,8 @@ struct alignas(16) SvHdr {
 // the workspace are those that the launch of an earlier range left, and ctr are three
 // counters of this launch's own. na: list 0's part of the work of lists 0 and 1, in
 // thousandths. perm also gives the output position of a leaf row. Batches: active[p] != -1 a problem to
-// skip, vshift[p] its workspace offset minus its vector offset (may be NULL).
+// skip, vshift[p] its workspace offset minus its vector offset, Ap[p] its operator (in
+// place of A); each may be NULL.
 template <class T> struct SvArgs {
     const SvHdr *hdr;
     const uint32_t *idx, *cons;
@@ -97,6 +98,7 @@ template <class T> struct SvArgs {
     const int64_t *vshift;
     int32_t l0[3], l1[3], na, ngrp;
     const T *A;
+    const T *const *Ap;
     T *ws;
     int64_t nzero, xoff, nx;
     const double *xin;
@@ -289,10 +291,6 @@ struct BatchProb {
 cudaError_t launch_brgb_f64(const int64_t *roff, const int64_t *blob, const int64_t *pstart, int nphase,
                             const BatchProb *probs, const int32_t *active, const double *xin, double *yout,
                             unsigned *bar, int32_t *err, cudaStream_t st);
-cudaError_t launch_brgb_f32(const int64_t *roff, const int64_t *blob, const int64_t *pstart, int nphase,
-                            const BatchProb *probs, const int32_t *active, const double *xin, double *yout,
-                            unsigned *bar, int32_t *err, cudaStream_t st);
-
 // Segmented GMRES: P independent systems in lockstep over one concatenated
 // vector (problem p owns a contiguous row range); block b works on rows
 // [brow[b], brow[b+1]) of problem bprob[b], problem p owns blocks
@@ -311,14 +309,15 @@ struct GmresSeg {
     const int32_t *bprob;    // nblk
     const int64_t *brow;     // nblk + 1
     const int32_t *pblk;     // P + 1
+    const double *tolp;      // stopping tolerance (device, so that captured steps do not hold it)
     int64_t Ntot;
     int m, P, nblk;
 };
 bool gms_attr(const GmresSeg &g);
 cudaError_t gms_norms(const GmresSeg &g, const double *v, double *out, int zero_to_one, cudaStream_t st);
 cudaError_t gms_start(const GmresSeg &g, const double *b, const double *Ax, double tol, cudaStream_t st);
-cudaError_t gms_arnoldi(const GmresSeg &g, double tol, cudaStream_t st);
-cudaError_t gms_loop(const GmresSeg &g, cudaGraphConditionalHandle hnd, cudaStream_t st);
+// one step on w = A vcur; hnd (may be NULL): the while condition of a captured step
+cudaError_t gms_arnoldi(const GmresSeg &g, const cudaGraphConditionalHandle *hnd, cudaStream_t st);
 cudaError_t gms_finish(const GmresSeg &g, double *x, int last, int kmax, cudaStream_t st);
 // y[idx[t]] = x[t] (scatter) / y[t] = x[idx[t]] (gather) over n elements with
 // 64-bit indices (concatenated permutations of a batch)

@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
                 sr.next(nslots);
                 if (sr.i == 0) slot_used = true;
                 if (t >= 0 && !skip) {
-                    const T *A = a.A + h.a;
+                    const T *A = (a.Ap ? a.Ap[h.pid] : a.A) + h.a;
 #pragma unroll 1
                     for (int c = 0; c < h.W; c += cpc) {
                         if (stage_used && !sv_wait(empty + fr.i, fr.par ^ 1u, fail, a.err)) {
