@@ -76,6 +76,20 @@ template <class T> struct DBuf {
     }
 };
 
+// The target stream and operator image of the tensor-core FP64 product (mo.cu)
+struct MoStream {
+    DBuf<MoHdr> hdr;
+    DBuf<uint32_t> idx, cons, blist, zrow;
+    DBuf<uint2> grp;
+    DBuf<int32_t> cnt, rem, ctr, xb, sa, mx;
+    DBuf<int64_t> s0, slices;
+    DBuf<char> img;  // made on the first product
+    int64_t bytes = 0;
+    int32_t list[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+    int32_t share = 0, ngrp = 0, nwb = 0, nxb = 0, nzrow = 0;
+    bool fused = true, ready = false, refused = false;
+};
+
 // Device state of the lockstep GMRES for one Krylov-vector type T
 template <class T> struct GmbStore {
     DBuf<T> V, w, vcur;
@@ -155,6 +169,7 @@ struct h2w_handle {
     bool op32s_ready = false;
     SvStream sv;
     int32_t sv_split = 0;   // list 0: end of the upward passes
+    MoStream mo;
     bool fused_sv = true;
     bool op32m_ready = false;
     DBuf<int32_t> d_mctr;                           // its per-phase target counters
@@ -1754,6 +1769,13 @@ struct SvHost {
     std::vector<uint2> grp;
     std::vector<int32_t> cnt;
     std::vector<int64_t> slices;  // operator pieces to copy (slice_records)
+    std::vector<int64_t> s0;      // the slices of each target
+    // the tensor-core form (mo.cu): source block lists and blocks of the written rows per
+    // target, block starts (the workspace's, then the input's), rows nobody writes
+    std::vector<uint32_t> blist, bl0, ob0, zrow;
+    std::vector<uint16_t> nbl, nob;
+    std::vector<int64_t> blocks;
+    int32_t nwb = 0;
     int64_t opn = 0;
     int max_w = 1;
     bool fused = true;  // the leaf pass writes the result itself
@@ -1826,7 +1848,10 @@ void group_deps(const std::vector<const PlanBuilder::LTarget *> &groups, const s
 // adding to the rows of the one before: the sums come in the same order on every run.
 constexpr int SV_CUT_CTAS = 608;
 constexpr int64_t SV_CUT_MIN = 2048;
-void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t ws0, int64_t x0, int64_t xoff, SvHost &out) {
+// tiles: the tensor-core form's cut, tiles of 64 rows and at most MO_XW columns.
+constexpr int64_t MO_XW = 2048;
+void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t ws0, int64_t x0, int64_t xoff, SvHost &out,
+              bool tiles = false) {
     auto bad = [](const char *what) { throw ApiError(H2W_ERR_STATE, std::string("internal: single-vector stream: ") + what); };
     PlanBuilder &pb = *h->plan;
     const int last = h->nph_total - 1;
@@ -1843,8 +1868,8 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
     pb.S.clear();
     pb.win.clear();
     pb.fused = true;
-    pb.xw_cap = XW_CAP;
-    pb.max_rows = SV_MAX_ROWS;
+    pb.xw_cap = tiles ? MO_XW : (int64_t)XW_CAP;
+    pb.max_rows = tiles ? MR_ROWS : (int64_t)SV_MAX_ROWS;
     std::vector<const PlanBuilder::LTarget *> groups;
     std::deque<PlanBuilder::LTarget> cut;  // the column parts and what changes its flags
     struct Key { int list, hi, part; double work; };
@@ -1862,7 +1887,7 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
             for (const auto &p : l.panels)
                 for (const Seg &sg : p.segs)
                     if (!(sg.flags & S_GATHER)) bad("a free target reads the workspace");
-        if (xw <= XW_CAP) {
+        if (xw <= pb.xw_cap) {
             groups.push_back(&l);
             key.push_back({ls, l.hi, 0, w});
             continue;
@@ -1907,8 +1932,8 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
         }
         const auto &l = *groups[g];
         const int64_t share = (int64_t)(pass[key[g].list][std::min(l.hi, 127)] / ctas);
-        pb.row_split = std::min(row_split, std::max(SV_CUT_MIN, share));
-        pb.min_rows = rows_min;
+        pb.row_split = tiles ? 0 : std::min(row_split, std::max(SV_CUT_MIN, share));
+        pb.min_rows = tiles ? MR_ROWS : rows_min;
         const size_t t0 = pb.T.size();
         pb.split(l.dst, l.nrows, l.flags, l.panels);
         parts[g] = (int32_t)(pb.T.size() - t0);
@@ -1928,10 +1953,36 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
     first_writers_overwrite(roff, blob, h->ws_n, h->fly_active ? &h->fly_rows : nullptr);
     group_deps(groups, parts, h->ws_n, out);
     out.opn = slice_records(roff, blob, out.slices, 0);
+    std::vector<uint32_t> block;  // block of each row (tiles)
+    if (tiles) {
+        const int64_t nr = xoff + h->nv();
+        std::vector<uint8_t> mark((size_t)nr + 1, 0), written((size_t)xoff, 0), read((size_t)xoff, 0);
+        mark[0] = mark[(size_t)xoff] = 1;
+        for (const auto *l : groups) {
+            mark[(size_t)l->dst] = mark[(size_t)(l->dst + l->nrows)] = 1;
+            if (!(l->flags & T_SCATTER)) std::memset(written.data() + l->dst, 1, (size_t)l->nrows);
+            for (const auto &p : l->panels)
+                for (const Seg &sg : p.segs) {
+                    const int64_t r = sg.flags & S_GATHER ? xoff + sg.src : sg.src;
+                    mark[(size_t)r] = mark[(size_t)(r + sg.len)] = 1;
+                    if (!(sg.flags & S_GATHER)) std::memset(read.data() + sg.src, 1, (size_t)sg.len);
+                }
+        }
+        block.resize((size_t)nr);
+        for (int64_t r = 0; r < nr; ++r) {
+            if (mark[(size_t)r]) out.blocks.push_back(r);
+            block[(size_t)r] = (uint32_t)out.blocks.size() - 1;
+            if (r < xoff && read[(size_t)r] && !written[(size_t)r]) out.zrow.push_back((uint32_t)r);
+        }
+        out.nwb = (int32_t)block[(size_t)xoff];
+        out.blocks.push_back(nr);
+    }
+    out.s0.assign(1, 0);
     // headers; targets of a group that read the same sources share the list of rows.
     // Every value the kernel indexes with is checked against its field.
     std::vector<uint32_t> rows, prev;
-    uint32_t prev0 = 0;
+    uint32_t prev0 = 0, blist0 = 0;
+    uint16_t nblist = 0;
     for (size_t t = 0; t + 1 < roff.size(); ++t) {
         const size_t o = (size_t)roff[t];
         const int64_t nrows = blob[o + 1] & 0xffffffff, fl = blob[o + 1] >> 32;
@@ -1963,7 +2014,17 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
             W += w;
         }
         if (W < 1 || W > BRG_XS_ELEMS || ws0 + blob[o] + nrows > (int64_t)UINT32_MAX) bad("target out of range");
+        out.s0.push_back(out.s0.back() + np);
         if (rows != prev) {
+            if (tiles) {
+                const size_t b0 = out.blist.size();
+                for (uint32_t r : rows)
+                    if (out.blist.size() == b0 || out.blist.back() != block[r]) out.blist.push_back(block[r]);
+                std::sort(out.blist.begin() + (long)b0, out.blist.end());
+                out.blist.erase(std::unique(out.blist.begin() + (long)b0, out.blist.end()), out.blist.end());
+                blist0 = (uint32_t)b0;
+                nblist = (uint16_t)(out.blist.size() - b0);
+            }
             prev0 = (uint32_t)out.idx.size();
             if (out.idx.size() + rows.size() > (size_t)UINT32_MAX) bad("too many sources");
             out.idx.insert(out.idx.end(), rows.begin(), rows.end());
@@ -1971,6 +2032,12 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
         }
         d.idx0 = prev0;
         d.W = (uint16_t)W;
+        if (tiles) {
+            out.bl0.push_back(blist0);
+            out.nbl.push_back(nblist);
+            out.ob0.push_back(block[d.dst]);
+            out.nob.push_back((uint16_t)(block[d.dst + (uint32_t)nrows - 1] - block[d.dst] + 1));
+        }
         out.max_w = std::max(out.max_w, (int)W);
     }
     pb.T = std::vector<Target>();
@@ -2035,6 +2102,60 @@ void sv_upload(std::vector<SvHost> &v, const std::vector<int> &shift, SvStream &
     if (!d.ctr.p) d.ctr.alloc(SV_CTRS);
     CK(sv_configure(all.max_w, d.f64, d.f32));
     CK(cudaStreamSynchronize(st));  // the host arrays end here
+}
+
+// The tensor-core form's stream of one operator: targets are already in the order of
+// their lists.
+void mo_upload(const SvHost &v, MoStream &d, cudaStream_t st) {
+    std::vector<MoHdr> hdr(v.hdr.size());
+    for (int l = 0; l < 3; ++l) d.list[l][0] = d.list[l][1] = 0;
+    double work[3] = {0, 0, 0};
+    d.bytes = 0;
+    for (size_t t = 0; t < hdr.size(); ++t) {
+        const SvHdr &s = v.hdr[t];
+        MoHdr &h = hdr[t];
+        h.img = d.bytes;
+        d.bytes += mo_image_bytes(s.nrows, s.W);
+        h.dst = s.dst;
+        h.idx0 = s.idx0;
+        h.grp = s.grp;
+        h.bl0 = v.bl0[t];
+        h.ob0 = v.ob0[t];
+        h.nrows = s.nrows;
+        h.W = s.W;
+        h.flags = s.flags;
+        h.nbl = v.nbl[t];
+        h.nob = v.nob[t];
+        ++d.list[v.list[t]][1];
+        work[v.list[t]] += (double)s.nrows * s.W;
+    }
+    for (int l = 1; l < 3; ++l) {
+        d.list[l][0] = d.list[l - 1][1];
+        d.list[l][1] += d.list[l][0];
+    }
+    d.share = (int32_t)(1000.0 * work[0] / std::max(1.0, work[0] + work[1]));
+    d.ngrp = (int32_t)v.grp.size();
+    d.nwb = v.nwb;
+    d.nxb = (int32_t)v.blocks.size() - 1 - v.nwb;
+    d.nzrow = (int32_t)v.zrow.size();
+    d.fused = v.fused;
+    std::vector<int32_t> xb;
+    for (size_t b = (size_t)v.nwb; b < v.blocks.size(); ++b) xb.push_back((int32_t)(v.blocks[b] - v.blocks[(size_t)v.nwb]));
+    d.hdr.upload(hdr, st);
+    d.idx.upload(v.idx, st);
+    d.cons.upload(v.cons, st);
+    d.blist.upload(v.blist, st);
+    d.zrow.upload(v.zrow, st);
+    d.grp.upload(v.grp, st);
+    d.cnt.upload(v.cnt, st);
+    d.xb.upload(xb, st);
+    d.s0.upload(v.s0, st);
+    d.slices.upload(v.slices, st);
+    d.rem.alloc(v.cnt.size());
+    if (!d.ctr.p) d.ctr.alloc(SV_CTRS);
+    d.img.reset();
+    d.ready = d.refused = false;
+    CK(cudaStreamSynchronize(st));
 }
 
 // for the profiling statistics.
@@ -2737,6 +2858,11 @@ void build_plan(h2w_handle *h) {
         h->plan = pbp;
         realize_single(h, h->row_split);
         realize_multi(h, h->mr_xw);
+        if (!h->fly_active) {
+            SvHost mo;
+            sv_build(h, h->row_split, SV_CUT_CTAS, 0, 0, 0, h->xoff(), mo, true);
+            mo_upload(mo, h->mo, st);
+        }
     }
     h->d_ws.alloc((size_t)(h->xoff() + h->nv()));
     h->d_ctr.alloc(h->phases.size() + 1);
@@ -3153,6 +3279,70 @@ void mr_prof(h2w_handle *h, int prec, int rp, cudaStream_t st, F &&launch) {
     h->prof_recs.push_back(r);
 }
 
+// The tensor-core form's operator image; false without the room for it (as much again
+// is left free) or with an entry that is not finite: the products then stay on the FP64 and
+// FP32 pipes.
+bool ensure_mo(h2w_handle *h) {
+    MoStream &d = h->mo;
+    if (d.ready || d.refused) return d.ready;
+    size_t fr = 0, tot = 0;
+    CK(cudaMemGetInfo(&fr, &tot));
+    d.refused = d.bytes <= 0 || fr / 2 < (size_t)d.bytes || h->xoff() + h->nv() >= (int64_t)INT32_MAX;
+    if (d.refused) return false;
+    cudaStream_t st = h->stream;
+    d.img.alloc((size_t)d.bytes);
+    d.sa.alloc(d.hdr.n * 64);
+    d.mx.alloc((size_t)(d.nwb + d.nxb) * MR_MAX);
+    CK(cudaMemsetAsync(d.mx.p, 0, 4, st));  // the first word reports a bad entry
+    CK(launch_mo_image(d.hdr.p, d.list[2][1], d.s0.p, d.slices.p, h->d_op.p, d.img.p, d.sa.p, d.mx.p, st));
+    int32_t bad = 0;
+    CK(cudaMemcpyAsync(&bad, d.mx.p, 4, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    if (bad) {
+        d.refused = true;
+        d.img.reset();
+        return false;
+    }
+    d.ready = true;
+    return true;
+}
+
+MoArgs mo_args(h2w_handle *h, int rp, const double *xi, double *yi) {
+    MoStream &d = h->mo;
+    MoArgs a{};
+    a.hdr = d.hdr.p;
+    a.idx = d.idx.p;
+    a.cons = d.cons.p;
+    a.blist = d.blist.p;
+    a.zrow = d.zrow.p;
+    a.grp = d.grp.p;
+    a.sa = d.sa.p;
+    a.xb = d.xb.p;
+    a.img = d.img.p;
+    for (int l = 0; l < 3; ++l) {
+        a.l0[l] = d.list[l][0];
+        a.l1[l] = d.list[l][1];
+    }
+    a.na = d.share;
+    a.ngrp = d.ngrp;
+    a.nwb = d.nwb;
+    a.nxb = d.nxb;
+    a.nzrow = d.nzrow;
+    a.xoff = (uint32_t)h->xoff();
+    a.ld = rp;
+    a.rows = h->xoff() + h->nv();
+    a.mx = d.mx.p;
+    a.ws = h->m_wsd.p;
+    a.xin = xi;
+    a.yout = yi;
+    a.cnt = d.cnt.p;
+    a.rem = d.rem.p;
+    a.ctr = d.ctr.p;
+    a.bar = h->d_bar.p;
+    a.err = h->d_err.p;
+    return a;
+}
+
 // Y = A X for an interleaved leaf-order block of rp vectors (xi, yi: N x rp).
 void run_matvec_multi(h2w_handle *h, int prec, int rp, const double *xi, double *yi, cudaStream_t st) {
     if (h->fly_active)
@@ -3191,6 +3381,14 @@ void run_matvec_multi(h2w_handle *h, int prec, int rp, const double *xi, double 
         });
         if (!h->fused_scatter_m) CK(launch_mr_widen_f32(h->m_wsf.p + (size_t)h->yperm_off * rp, yi, h->tree.N * rp, st));
     } else {
+        if (h->dataflow && h->coop && ensure_mo(h)) {
+            const size_t need = (size_t)(h->xoff() + h->nv()) * (size_t)rp;
+            if (h->m_wsd.n < need) h->m_wsd.alloc(need);
+            const MoArgs a = mo_args(h, rp, xi, yi);
+            mr_prof(h, prec, rp, st, [&] { return launch_mo(a, st); });
+            if (!h->mo.fused) CK(launch_mo_unplane(a, h->tree.N, yi, st));
+            return;
+        }
         if (h->m_wsd.n < wsz) h->m_wsd.alloc(wsz);
         CK(cudaMemsetAsync(h->m_wsd.p, 0, wsz * 8, st));
         if (prec == H2W_PREC_DF64) {  // operator split once; the input block split per product
