@@ -423,8 +423,12 @@ void run_nca_small(h2w_handle *h, const std::vector<std::vector<int32_t>> &R, co
                    std::vector<std::vector<int32_t>> &prow, std::vector<std::vector<int32_t>> &pcol,
                    std::vector<size_t> &over);
 
-constexpr int64_t NCA_BIG = 8192;  // rows + columns from which a block gets a group of CTAs
-constexpr int64_t NCA_MED = 2048;  // ... and from which it does when one CTA per block would leave SMs idle
+// Rows + columns from which a block gets a group of CTAs of a cooperative launch. A cluster's
+// sixteen CTAs take 3 ms for four blocks of 10000 (groups 11) and 50 for 64 of 12000
+// (70), the same from 16000 on, 219 and 217 for 64 of 39000, 223 and 43 for two of 10^6.
+constexpr int64_t NCA_BIG = 16384;
+constexpr int64_t NCA_BIG_DF = 8192;  // the same for kernels built on log (double-FP32 groups)
+constexpr int64_t NCA_MED = 2048;  // ... and from which it does where the groups search in double-FP32 arithmetic
 constexpr int NCA_SMALL_CAP = 512;   // pivots one CTA per block holds; larger blocks move to the groups
 
 // Scratch bytes a batch of NCA blocks may take: most of the free device
@@ -569,13 +573,11 @@ void run_nca_big(h2w_handle *h, const std::vector<std::vector<int32_t>> &R, cons
     }
 }
 
-// The NCA pivot search: one CTA per block (nca_kernel) in batches that fit
+// The NCA pivot search: a cluster of CTAs per block (nca.cu) in batches that fit
 // the scratch budget; blocks of NCA_BIG or more rows + columns, and blocks
-// whose rank outgrows one CTA's scratch, get groups of CTAs (run_nca_big).
-// Blocks of NCA_MED or more rows + columns get groups too when there are no
-// more of them than SMs (one CTA each would leave SMs idle), and always for
-// the kernels whose group search runs in double-FP32 arithmetic.
-// H2W_NCA_BIG=0 keeps every block that fits on one CTA.
+// whose rank outgrows that scratch, get groups of CTAs (run_nca_big), blocks of
+// NCA_MED or more too for the kernels whose group search runs in double-FP32 arithmetic.
+// H2W_NCA_BIG=0 keeps every block that fits on a cluster.
 void run_nca_plain(h2w_handle *h, const std::vector<std::vector<int32_t>> &R, const std::vector<std::vector<int32_t>> &C,
                    std::vector<std::vector<int32_t>> &prow, std::vector<std::vector<int32_t>> &pcol) {
     prow.assign(R.size(), {});
@@ -583,19 +585,12 @@ void run_nca_plain(h2w_handle *h, const std::vector<std::vector<int32_t>> &R, co
     std::vector<size_t> big, med, small;
     const char *eb = getenv("H2W_NCA_BIG");
     const bool use_big = !(eb && std::string(eb) == "0");
+    // kernels built on log search in double-FP32 arithmetic on the groups
+    const bool df = h->nca_df && ((h->cfg.dim < 3 && h->cfg.choice == 0) || (h->cfg.dim == 3 && h->cfg.choice == 1));
     for (size_t p = 0; p < R.size(); ++p) {
         const int64_t w = (int64_t)(R[p].size() + C[p].size());
-        (use_big && w >= NCA_BIG ? big : use_big && w >= NCA_MED ? med : small).push_back(p);
+        (use_big && w >= (df ? NCA_BIG_DF : NCA_BIG) ? big : use_big && df && w >= NCA_MED ? med : small).push_back(p);
     }
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, std::max(0, h->cfg.device)) != cudaSuccess) {
-        cudaGetLastError();
-        sms = 0;
-    }
-    // kernels built on log search in double-FP32 arithmetic on the groups,
-    // faster than one CTA's FP64 whatever the count
-    const bool df = h->nca_df && ((h->cfg.dim < 3 && h->cfg.choice == 0) || (h->cfg.dim == 3 && h->cfg.choice == 1));
-    if (!df && (int64_t)med.size() > (int64_t)sms) small.insert(small.end(), med.begin(), med.end()), med.clear();
     std::sort(small.begin(), small.end());
     // H2W_TIMING=1: the time of each part of the search on stderr (diagnostic)
     static const bool timing = getenv("H2W_TIMING") && std::string(getenv("H2W_TIMING")) == "1";
@@ -634,7 +629,7 @@ void run_nca_plain(h2w_handle *h, const std::vector<std::vector<int32_t>> &R, co
             int64_t rm = 0;
             for (size_t p : med) rm += (int64_t)prow[p].size();
             fprintf(stderr, "h2w nca: %zu group blocks %.3f s (pivots %lld); %zu medium blocks on groups %.3f s (pivots "
-                            "%lld); %zu one-CTA blocks %.3f s (pivots %lld); %zu outgrew one CTA %.3f s\n", big.size(),
+                            "%lld); %zu cluster blocks %.3f s (pivots %lld); %zu outgrew them %.3f s\n", big.size(),
                     std::chrono::duration<double>(tm - t0).count(), (long long)rb, med.size(),
                     std::chrono::duration<double>(t1 - tm).count(), (long long)rm, small.size(),
                     std::chrono::duration<double>(t2 - t1).count(), (long long)rs, over.size(),
@@ -661,7 +656,7 @@ void run_nca_plain(h2w_handle *h, const std::vector<std::vector<int32_t>> &R, co
     }
 }
 
-// One CTA per block. over: blocks whose rank outgrew the CTA's scratch
+// A cluster per block. over: blocks whose rank outgrew the scratch
 // (NCA_SMALL_CAP pivots, or rank_cap when smaller); their pivots are left
 // empty for the caller to search with groups of CTAs.
 void run_nca_small(h2w_handle *h, const std::vector<std::vector<int32_t>> &R, const std::vector<std::vector<int32_t>> &C,

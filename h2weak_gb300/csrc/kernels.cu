@@ -2,8 +2,6 @@
 //
 //  * kentry            kernel-matrix entries, operation order and rounding of
 //                      the reference's getMatrixEntry (no FMA contraction)
-//  * nca_kernel        batched NCA/ACA pivot search, one CTA per block
-//                      (1D/codes/aca.hpp:296-446 pivoting and stopping rule)
 //  * factor_kernel     LU of K(I,J) in pivot order = the ACA's L and R
 //  * xfer_kernel       rows K(p,J) R^-1 L^-1 (transfer matrices), columns
 //                      R^-1 L^-1 K(I,p), and the 1D U / V^T factors
@@ -13,7 +11,6 @@
 //  * GMRES kernels     CGS2 Arnoldi step, normalisation, Givens rotations
 #include <atomic>
 #include <cfloat>
-#include <climits>
 
 #include "kernels.cuh"
 #include "sync.cuh"
@@ -31,17 +28,6 @@ __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
-__device__ __forceinline__ bool amax_better(double va, int ia, double vb, int ib) {
-    return va > vb || (va == vb && ia < ib);
-}
-__device__ __forceinline__ void warp_amax(double &v, int &i) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        double ov = __shfl_xor_sync(0xffffffffu, v, o);
-        int oi = __shfl_xor_sync(0xffffffffu, i, o);
-        if (amax_better(ov, oi, v, i)) { v = ov; i = oi; }
-    }
-}
 // Block-wide sum; every thread gets the total. sh: >= 32 doubles.
 __device__ double block_sum(double v, double *sh) {
     v = warp_sum(v);
@@ -53,238 +39,7 @@ __device__ double block_sum(double v, double *sh) {
     for (int q = 0; q < nw; ++q) t += sh[q];
     return t;
 }
-// Block-wide argmax of (value, lowest index); every thread gets the result.
-__device__ void block_amax(double &v, int &i, double *shv, int *shi) {
-    warp_amax(v, i);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-    __syncthreads();
-    if (l == 0) { shv[w] = v; shi[w] = i; }
-    __syncthreads();
-    v = shv[0];
-    i = shi[0];
-    for (int q = 1; q < nw; ++q)
-        if (amax_better(shv[q], shi[q], v, i)) { v = shv[q]; i = shi[q]; }
-}
-
-__device__ __forceinline__ bool bit_get(const uint32_t *m, int i) { return (m[i >> 5] >> (i & 31)) & 1u; }
-
-// ----------------------------------------------------------------- NCA ---
-// One CTA per block (I, J). Pivoting and stopping follow ACA_only_nodes:
-// first row with a non-negligible entry, column pivot = first largest |.|
-// among unused columns of the residual row, row pivot = first largest |.|
-// among unused rows of the residual column, stop when ||u|| ||v|| <= tol
-// normS or the rank reaches min(n1, n2) (a block whose rank reaches its
-// scratch capacity rcap first reports -rcap). Residual rows and columns are
-// formed entry by entry in pivot order with separate multiply and subtract,
-// so for identical entries they are bitwise those of the reference; norms
-// and dot products are tree reductions (they only enter the stopping test).
-constexpr int NCA_THREADS = 256;
 constexpr int GM_THREADS = 256;
-
-__global__ void __launch_bounds__(NCA_THREADS) nca_kernel(const NcaProb *__restrict__ probs,
-                                                          const int32_t *__restrict__ idx, KParams kp, double tol,
-                                                          double *__restrict__ scr, int32_t *__restrict__ rank_out,
-                                                          int32_t *__restrict__ prow, int32_t *__restrict__ pcol,
-                                                          int32_t *status, int mask1_words, int mask2_words,
-                                                          int coef_len) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    uint32_t *rmask = reinterpret_cast<uint32_t *>(smem);
-    uint32_t *cmask = rmask + mask1_words;
-    double *coef = reinterpret_cast<double *>(cmask + mask2_words + ((mask1_words + mask2_words) & 1));
-    double *red = coef + coef_len;                       // coef_len * 8 (per-warp partial dots)
-    __shared__ double shv[32];
-    __shared__ int shi[32];
-    __shared__ double shs[32];
-
-    const NcaProb pb = probs[blockIdx.x];
-    const int n1 = pb.n1, n2 = pb.n2, rcap = pb.rcap;
-    const int32_t *I = idx + pb.ri;
-    const int32_t *J = idx + pb.ci;
-    double *U = scr + pb.u;
-    double *V = scr + pb.v;
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-
-    for (int q = tid; q < mask1_words; q += nt) rmask[q] = 0u;
-    for (int q = tid; q < mask2_words; q += nt) cmask[q] = 0u;
-    __syncthreads();
-    if (tid == 0) rank_out[blockIdx.x] = 0;
-    const int mn = n1 < n2 ? n1 : n2;
-    if (mn == 0 || rcap == 0) return;
-
-    // first pivot row: first row whose largest |entry| exceeds 1e-36
-    const double tiny = 1e-36;
-    int ri = -1, ci = -1;
-    for (int l = 0; l < n1; ++l) {
-        double bv = -1.0;
-        int bi = INT_MAX;
-        const int gi = I[l];
-        for (int s = tid; s < n2; s += nt) {
-            double v = kentry(kp, gi, J[s]);
-            V[s] = v;
-            double a = fabs(v);
-            if (amax_better(a, s, bv, bi)) { bv = a; bi = s; }
-        }
-        block_amax(bv, bi, shv, shi);
-        if (bv > tiny) { ri = l; ci = bi; break; }
-    }
-    if (ri < 0) return;
-    __syncthreads();
-    double piv = V[ci];
-    double usq = 0.0, vsq = 0.0;
-    int nri = INT_MAX;
-    {
-        double bv = -1.0;
-        int bi = INT_MAX;
-        const int gj = J[ci];
-        for (int t = tid; t < n1; t += nt) {
-            double c = kentry(kp, I[t], gj);
-            double u = __ddiv_rn(c, piv);
-            U[t] = u;
-            usq += u * u;
-            if (t != ri) {
-                double a = fabs(c);
-                if (amax_better(a, t, bv, bi)) { bv = a; bi = t; }
-            }
-        }
-        for (int s = tid; s < n2; s += nt) vsq += V[s] * V[s];
-        block_amax(bv, bi, shv, shi);
-        nri = bi;
-    }
-    double nu = sqrt(block_sum(usq, shs));
-    double nv = sqrt(block_sum(vsq, shs));
-    if (tid == 0) {
-        prow[pb.piv] = ri;
-        pcol[pb.piv] = ci;
-        rmask[ri >> 5] |= 1u << (ri & 31);
-        cmask[ci >> 5] |= 1u << (ci & 31);
-    }
-    int rank = 1;
-    double normS = 0.0;
-    ri = nri;
-    __syncthreads();
-
-    bool over = false;  // the block needs more pivots than its scratch holds
-    while (nu * nv > tol * normS && rank < mn) {
-        if (rank >= rcap) {
-            over = true;
-            break;
-        }
-        if (ri < 0 || ri >= n1) {  // no finite candidate row
-            if (tid == 0) atomicOr(status, 2);
-            break;
-        }
-        // residual row ri
-        for (int l = tid; l < rank; l += nt) coef[l] = U[(size_t)l * n1 + ri];
-        __syncthreads();
-        double *Vr = V + (size_t)rank * n2;
-        double bv = -1.0;
-        int bi = INT_MAX;
-        vsq = 0.0;
-        {
-            const int gi = I[ri];
-            for (int s = tid; s < n2; s += nt) {
-                double v = kentry(kp, gi, J[s]);
-                for (int l = 0; l < rank; ++l) v = __dsub_rn(v, __dmul_rn(coef[l], V[(size_t)l * n2 + s]));
-                Vr[s] = v;
-                vsq += v * v;
-                if (!bit_get(cmask, s)) {
-                    double a = fabs(v);
-                    if (amax_better(a, s, bv, bi)) { bv = a; bi = s; }
-                }
-            }
-        }
-        block_amax(bv, bi, shv, shi);
-        if (bi < 0 || bi >= n2) {  // no finite candidate column (non-finite entries)
-            if (tid == 0) atomicOr(status, 2);
-            break;
-        }
-        ci = bi;
-        nv = sqrt(block_sum(vsq, shs));
-        // residual column ci
-        piv = Vr[ci];
-        for (int l = tid; l < rank; l += nt) coef[l] = V[(size_t)l * n2 + ci];
-        __syncthreads();
-        double *Ur = U + (size_t)rank * n1;
-        usq = 0.0;
-        bv = -1.0;
-        bi = INT_MAX;
-        {
-            const int gj = J[ci];
-            for (int t = tid; t < n1; t += nt) {
-                double c = kentry(kp, I[t], gj);
-                for (int l = 0; l < rank; ++l) c = __dsub_rn(c, __dmul_rn(coef[l], U[(size_t)l * n1 + t]));
-                double u = __ddiv_rn(c, piv);
-                Ur[t] = u;
-                usq += u * u;
-                if (t != ri && !bit_get(rmask, t)) {
-                    double a = fabs(c);
-                    if (amax_better(a, t, bv, bi)) { bv = a; bi = t; }
-                }
-            }
-        }
-        block_amax(bv, bi, shv, shi);
-        nri = bi;
-        nu = sqrt(block_sum(usq, shs));
-        if (nu < 1e-36 || nv < 1e-36) break;
-        if (tid == 0) {
-            prow[pb.piv + rank] = ri;
-            pcol[pb.piv + rank] = ci;
-            rmask[ri >> 5] |= 1u << (ri & 31);
-            cmask[ci >> 5] |= 1u << (ci & 31);
-        }
-        ++rank;
-        // normS update: dots of every stored u and v with the new ones
-        for (int l = 0; l < rank; ++l) {
-            const double *Ul = U + (size_t)l * n1, *Vl = V + (size_t)l * n2;
-            double du = 0.0, dv = 0.0;
-            for (int t = tid; t < n1; t += nt) du += Ul[t] * Ur[t];
-            for (int s = tid; s < n2; s += nt) dv += Vl[s] * Vr[s];
-            du = warp_sum(du);
-            dv = warp_sum(dv);
-            if (lane == 0) {
-                red[(size_t)(2 * l) * nw + warp] = du;
-                red[(size_t)(2 * l + 1) * nw + warp] = dv;
-            }
-        }
-        __syncthreads();
-        for (int l = tid; l < rank; l += nt) {
-            double du = 0.0, dv = 0.0;
-            for (int q = 0; q < nw; ++q) {
-                du += red[(size_t)(2 * l) * nw + q];
-                dv += red[(size_t)(2 * l + 1) * nw + q];
-            }
-            coef[l] = 2.0 * fabs(du * dv);
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double uv = nu * nv;
-            double ns = normS * normS + uv * uv;
-            for (int l = 0; l < rank; ++l) ns += coef[l];
-            shs[0] = sqrt(ns);
-        }
-        __syncthreads();
-        normS = shs[0];
-        ri = nri;
-        __syncthreads();
-    }
-    // an overflowing block reports -rank: the host runs it again with more scratch
-    if (tid == 0) rank_out[blockIdx.x] = over ? -rank : rank;
-}
-
-cudaError_t launch_nca(const NcaProb *probs, int nprob, const int32_t *idx, const KParams &kp, double tol,
-                       double *scratch, int32_t *rank, int32_t *prow, int32_t *pcol, int32_t *status, int max_n1,
-                       int max_n2, int max_rcap, cudaStream_t st) {
-    if (nprob == 0) return cudaSuccess;
-    int m1 = (max_n1 + 31) / 32, m2 = (max_n2 + 31) / 32;
-    int coef_len = max_rcap + 1;
-    size_t smem = (size_t)(m1 + m2 + 1) * 4 + (size_t)coef_len * 8 + (size_t)coef_len * 2 * (NCA_THREADS / 32) * 8;
-    cudaError_t e = cudaFuncSetAttribute(nca_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    nca_kernel<<<nprob, NCA_THREADS, smem, st>>>(probs, idx, kp, tol, scratch, rank, prow, pcol, status, m1, m2,
-                                                 coef_len);
-    count_launch(); return cudaGetLastError();
-}
 
 // ------------------------------------------------------------- factors ---
 // F (r x r, row-major) <- K(I,J) factorised in pivot order: R on and above

@@ -1,8 +1,8 @@
 // The NCA pivot search for large blocks on many SMs at once (sm_103a).
 //
 // The reference's ACA (1D/codes/aca.hpp:296-446) is sequential in its
-// pivots, and one CTA per block (nca_kernel) leaves a block of tens of
-// thousands of rows and columns on a single SM. Here the CTAs of one
+// pivots, and a cluster per block (nca.cu) leaves a block of tens of
+// thousands of rows and columns on sixteen SMs at most. Here the CTAs of one
 // cooperative launch form G groups; a group works on one large block at a
 // time, its CTAs striding over the block's columns (residual rows) and rows
 // (residual columns), with a bounded group barrier after each pass. Every
