@@ -143,7 +143,7 @@ struct h2w_handle {
     bool cplx = false;
     bool cgm_hermitian = false;  // H2W_OPT_COMPLEX_ARNOLDI
     double diag_im = 0;
-    DBuf<double2> c_V, c_w, c_r, c_ax, c_part, c_h, c_y;  // complex GMRES state
+    DBuf<double2> c_V, c_w, c_v, c_ax, c_part, c_h, c_y;  // complex GMRES state
     int64_t nv() const { return cplx ? 2 * tree.N : tree.N; }  // doubles per vector
     int64_t xoff() const { return pad4(ws_n); }  // the input in leaf order behind the workspace rows
     // device state
@@ -4268,131 +4268,85 @@ void require_real(const h2w_handle *h, const char *what) {
 // with Eigen's conjugate-first dot (sum conj(w) v_k), modified Gram-Schmidt
 // in the reference's order, the reference's complex Givens formulas
 // (GeneratePlaneRotation, gmres.hpp:52-68; ApplyPlaneRotation, :70-75) and
-// back substitution on the host in std::complex arithmetic, stop when
-// |s(i+1)| / ||b|| < tol. With H2W_OPT_COMPLEX_ARNOLDI the projections are
-// Hermitian (sum conj(v_k) w) and the rotations unitary (dy' = -conj(sn) dx
-// + cs dy). Krylov vectors, products and Gram-Schmidt on the GPU; the
-// Hessenberg column comes to the host once per step. b, x: leaf order,
+// back substitution, stop when |s(i+1)| / ||b|| < tol. With
+// H2W_OPT_COMPLEX_ARNOLDI the projections are Hermitian (sum conj(v_k) w) and
+// the rotations unitary (dy' = -conj(sn) dx + cs dy). All on the device, the
+// steps as a graph's loop; the host reads the result. b, x: leaf order,
 // interleaved (re, im), device.
 int cgmres_run(h2w_handle *h, const double *db, double *dx, int max_iter, double tol, int *iters, double *resid) {
-    typedef std::complex<double> cd;
     cudaStream_t st = h->stream;
     const int64_t n = h->tree.N;
-    const int m = max_iter;
-    if (h->c_V.n < (size_t)n * (size_t)(m + 1)) h->c_V.alloc((size_t)n * (size_t)(m + 1));
-    if (h->c_w.n < (size_t)n) h->c_w.alloc((size_t)n);
-    if (h->c_r.n < (size_t)n) h->c_r.alloc((size_t)n);
-    if (h->c_ax.n < (size_t)n) h->c_ax.alloc((size_t)n);
-    if (h->c_part.n < (size_t)cgm_blocks()) h->c_part.alloc((size_t)cgm_blocks());
-    if (h->c_h.n < (size_t)(m + 2)) h->c_h.alloc((size_t)(m + 2));
-    if (h->c_y.n < (size_t)(m + 1)) h->c_y.alloc((size_t)(m + 1));
+    const size_t m = (size_t)max_iter;
+    CgmDev g{};
+    g.N = n;
+    g.m = max_iter;
+    g.nblk = cgm_blocks(n);
+    g.herm = h->cgm_hermitian ? 1 : 0;
+    auto room = [](DBuf<double2> &v, size_t k) {
+        if (v.n < k) v.alloc(k);
+        return v.p;
+    };
+    g.V = room(h->c_V, (size_t)n * (m + 1));
+    g.w = room(h->c_w, (size_t)n);
+    g.vcur = room(h->c_v, (size_t)n);
+    g.part = room(h->c_part, (size_t)g.nblk * (m + 2));
+    g.H = room(h->c_h, (m + 1) * m);
+    double2 *sm = room(h->c_y, 4 * (m + 1));
+    g.s = sm;
+    g.cs = sm + (m + 1);
+    g.sn = sm + 2 * (m + 1);
+    g.y = sm + 3 * (m + 1);
+    double2 *ax = room(h->c_ax, (size_t)n);
+    if (!h->g_scal.p) h->g_scal.alloc(8);
+    if (!h->g_iter.p) h->g_iter.alloc(2);
+    g.scal = h->g_scal.p;
+    g.iter = h->g_iter.p;
+    g.bar = h->d_bar.p;
+    g.err = h->d_err.p;
     const double2 *b = reinterpret_cast<const double2 *>(db);
     double2 *x = reinterpret_cast<double2 *>(dx);
-    auto A = [&](const double2 *in, double2 *out) {
-        run_matvec_f64(h, reinterpret_cast<const double *>(in), reinterpret_cast<double *>(out), st, true);
+    auto A = [&](const double2 *in, double2 *out, cudaStream_t s) {
+        run_matvec_f64(h, reinterpret_cast<const double *>(in), reinterpret_cast<double *>(out), s, true);
     };
-    auto dot = [&](const double2 *a, const double2 *bb, double2 *out) { CK(cgm_dot(a, bb, n, h->c_part.p, out, st)); };
-    auto fetch = [&](const double2 *src, int cnt, std::vector<cd> &o) {
-        std::vector<double2> t((size_t)cnt);
-        CK(cudaMemcpyAsync(t.data(), src, (size_t)cnt * 16, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        o.resize((size_t)cnt);
-        for (int i = 0; i < cnt; ++i) o[(size_t)i] = cd(t[(size_t)i].x, t[(size_t)i].y);
-    };
-    auto norm = [&](const double2 *a) {
-        dot(a, a, h->c_h.p + m + 1);
-        std::vector<cd> o;
-        fetch(h->c_h.p + m + 1, 1, o);
-        return std::sqrt(o[0].real());
-    };
-    auto gen_rot = [](cd &dxv, cd &dyv, cd &cs, cd &sn) {
-        if (dxv == cd(0)) {
-            cs = cd(0);
-            sn = cd(1);
-        } else {
-            double scale = std::abs(dxv) + std::abs(dyv);
-            double nrm = scale * std::sqrt(std::abs(dxv / scale) * std::abs(dxv / scale) +
-                                           std::abs(dyv / scale) * std::abs(dyv / scale));
-            cd alpha = dxv / std::abs(dxv);
-            cs = std::abs(dxv) / nrm;
-            sn = alpha * std::conj(dyv) / nrm;
-        }
-    };
-    const bool herm = h->cgm_hermitian;
-    auto app_rot = [herm](cd &dxv, cd &dyv, cd &cs, cd &sn) {
-        cd temp = cs * dxv + sn * dyv;
-        dyv = (herm ? -std::conj(sn) : -sn) * dxv + cs * dyv;
-        dxv = temp;
-    };
-    std::vector<cd> H((size_t)(m + 1) * m, cd(0)), s((size_t)m + 1), cs((size_t)m + 1), sn((size_t)m + 1);
-    auto Hc = [&](int r, int c) -> cd & { return H[(size_t)c * (m + 1) + r]; };
-    auto update = [&](int k) {  // Update(x, k, H, s, v): back substitution, then x += sum_j v_j y_j
-        std::vector<cd> y(s);
-        for (int i = k; i >= 0; i--) {
-            y[(size_t)i] /= Hc(i, i);
-            for (int j = i - 1; j >= 0; j--) y[(size_t)j] -= Hc(j, i) * y[(size_t)i];
-        }
-        std::vector<double2> yd((size_t)k + 1);
-        for (int j = 0; j <= k; ++j) yd[(size_t)j] = make_double2(y[(size_t)j].real(), y[(size_t)j].imag());
-        CK(cudaMemcpyAsync(h->c_y.p, yd.data(), yd.size() * 16, cudaMemcpyHostToDevice, st));
-        CK(cgm_update_launch(x, h->c_V.p, h->c_y.p, k + 1, n, st));
+    double sc[3];
+    int32_t it2[2];
+    auto read = [&] {
+        CK(cudaMemcpyAsync(sc, g.scal, 24, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(it2, g.iter, 8, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
     };
-    double normb = norm(b);
-    A(x, h->c_ax.p);
-    CK(cgm_resid_launch(h->c_r.p, b, h->c_ax.p, n, st));
-    double beta = norm(h->c_r.p);
-    if (normb == 0.0) normb = 1;
-    double res = beta / normb;
-    *resid = res;
-    *iters = 0;
-    if (res <= tol) return H2W_OK;
-    int j = 1;
-    while (j <= max_iter) {
-        CK(cgm_scale_launch(h->c_V.p, h->c_r.p, 1.0 / beta, n, st));
-        std::fill(s.begin(), s.end(), cd(0));
-        s[0] = beta;
-        int i;
-        for (i = 0; i < m && j <= max_iter; i++, j++) {
-            double2 *vi = h->c_V.p + (size_t)i * n;
-            A(vi, h->c_w.p);
-            for (int k = 0; k <= i; k++) {
-                double2 *hk = h->c_h.p + k;
-                if (herm) dot(h->c_V.p + (size_t)k * n, h->c_w.p, hk);
-                else dot(h->c_w.p, h->c_V.p + (size_t)k * n, hk);
-                CK(cgm_axpy_launch(h->c_w.p, h->c_V.p + (size_t)k * n, hk, n, st));
-            }
-            const double hn = norm(h->c_w.p);
-            std::vector<cd> col;
-            fetch(h->c_h.p, i + 1, col);
-            for (int k = 0; k <= i; ++k) Hc(k, i) = col[(size_t)k];
-            Hc(i + 1, i) = hn;
-            CK(cgm_scale_launch(h->c_V.p + (size_t)(i + 1) * n, h->c_w.p, 1.0 / hn, n, st));
-            for (int k = 0; k < i; k++) app_rot(Hc(k, i), Hc(k + 1, i), cs[(size_t)k], sn[(size_t)k]);
-            gen_rot(Hc(i, i), Hc(i + 1, i), cs[(size_t)i], sn[(size_t)i]);
-            app_rot(Hc(i, i), Hc(i + 1, i), cs[(size_t)i], sn[(size_t)i]);
-            app_rot(s[(size_t)i], s[(size_t)i + 1], cs[(size_t)i], sn[(size_t)i]);
-            res = std::abs(s[(size_t)i + 1]) / normb;
-            if (res < tol) {
-                update(i);
-                *resid = res;
-                *iters = j;
-                return H2W_OK;
-            }
-        }
-        update(m - 1);
-        A(x, h->c_ax.p);
-        CK(cgm_resid_launch(h->c_r.p, b, h->c_ax.p, n, st));
-        beta = norm(h->c_r.p);
-        res = beta / normb;
-        if (res < tol) {
-            *resid = res;
-            *iters = j;
-            return H2W_OK;
+    cgm_prepare();
+    CK(cudaMemcpyAsync(g.scal + 6, &tol, 8, cudaMemcpyHostToDevice, st));
+    A(x, ax, st);  // also makes the product's buffers and launch attributes before a capture
+    CK(cgm_start(g, b, ax, st));
+    int64_t kps = 0;
+    cudaGraphExec_t ex = loop_graph(h, 8 + g.herm, H2W_PREC_FP64, max_iter, 1, 1, kps,
+                                    [&](cudaStream_t s, cudaGraphConditionalHandle c) {
+                                        A(g.vcur, g.w, s);
+                                        CK(cgm_step(g, &c, s));
+                                    });
+    if (ex) {
+        CK(cudaGraphLaunch(ex, st));
+    } else {
+        read();
+        for (int i = 0; i < max_iter && sc[2] == 0.0; ++i) {
+            A(g.vcur, g.w, st);
+            CK(cgm_step(g, nullptr, st));
+            read();
         }
     }
-    *resid = res;
-    *iters = max_iter;
+    CK(cgm_update(g, x, st));
+    read();
+    if (ex) count_launch(kps * std::max(it2[1], 1));
+    *resid = sc[1];
+    *iters = it2[1];
+    if (sc[2] != 0.0) return H2W_OK;
+    // all max_iter steps taken without meeting the tolerance: the true relative residual
+    A(x, ax, st);
+    CK(cgm_start(g, b, ax, st));
+    read();
+    *resid = sc[1];
+    *iters = sc[1] < tol ? max_iter + 1 : max_iter;
     return H2W_OK;
 }
 

@@ -27,6 +27,7 @@
 
 #include "bessel.cuh"
 #include "kernels.cuh"
+#include "sync.cuh"
 
 namespace h2w {
 
@@ -525,93 +526,223 @@ cudaError_t launch_dense_c(const KParams &kp, int64_t N, const double2 *x, doubl
 }
 
 // ----------------------------------------------------------------- GMRES ---
-// Vector operations of the reference GMRES (3D/codes/gmres.hpp:92-200) on
-// complex vectors of n entries. Reductions: per-block partials, then one
-// block sums them in order.
-constexpr int CGM_THREADS = 256;
-constexpr int CGM_BLOCKS = 304;
+// The reference GMRES (3D/codes/gmres.hpp:92-200) on complex vectors. A step is one
+// cooperative launch: the column's modified Gram-Schmidt, whose coefficients follow one
+// another, takes a grid barrier each, then the norm, the next basis vector and (one lane of
+// CTA 0) the rotations and the stopping test. A CTA keeps its rows of w in shared memory
+// (ws_rows > 0; else in g.w). What bounds it: the chain of barriers, read partials and
+// dot products, up to 1e5 rows; then memory, each basis vector read twice. A solve of 4001
+// points, 6 steps, beside its products: 860 us with three launches a coefficient, a copy
+// and a wait a norm and the rotations on the host; 420 here.
+constexpr int CGM_T = 256, CGM_W = CGM_T / 32;
 
-// part[b] = sum over the block's entries of conj(a_i) b_i  (Eigen's a.dot(b))
-__global__ void cgm_dot_part(const double2 *__restrict__ a, const double2 *__restrict__ b, int64_t n,
-                             double2 *__restrict__ part) {
-    __shared__ double sh[32];
-    double2 acc = make_double2(0.0, 0.0);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double2 p = c_cmul(a[i], b[i]);
-        acc.x += p.x;
-        acc.y += p.y;
+__device__ __forceinline__ void cgm_rows(int64_t N, int nblk, int64_t &r0, int64_t &r1) {
+    const int64_t chunk = (N + nblk - 1) / nblk;
+    r0 = (int64_t)blockIdx.x * chunk < N ? (int64_t)blockIdx.x * chunk : N;
+    r1 = r0 + chunk < N ? r0 + chunk : N;
+}
+// Sums of both components over the grid, the same in every thread. part: this sum's nblk
+// partials; sh: 2 CGM_W + 2 doubles. Half a warp adds up each component.
+__device__ double2 cgm_sum(const CgmDev &g, double2 v, double2 *part, double *sh) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double a = (lane & 16 ? v.y : v.x) + __shfl_xor_sync(0xffffffffu, lane & 16 ? v.x : v.y, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if ((lane & 15) == 0) sh[2 * warp + (lane >> 4)] = a;
+    __syncthreads();
+    if (warp == 0) {
+        a = lane < 2 * CGM_W ? sh[lane] : 0.0;
+#pragma unroll
+        for (int o = CGM_W; o > 1; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane < 2) reinterpret_cast<double *>(part + blockIdx.x)[lane] = a;
     }
-    acc.x = c_block_sum(acc.x, sh);
-    acc.y = c_block_sum(acc.y, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = acc;
-}
-// out = sum of part[0..nb)
-__global__ void cgm_dot_fin(const double2 *__restrict__ part, int nb, double2 *__restrict__ out) {
-    __shared__ double sh[32];
-    double2 acc = make_double2(0.0, 0.0);
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        acc.x += part[i].x;
-        acc.y += part[i].y;
+    grid_barrier(g.bar, gridDim.x, g.err);
+    if (warp == 0) {
+        a = 0.0;
+        for (int b = lane >> 1; b < g.nblk; b += 16) a += __ldcg(reinterpret_cast<const double *>(part + b) + (lane & 1));
+#pragma unroll
+        for (int o = 16; o > 1; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane < 2) sh[2 * CGM_W + lane] = a;
     }
-    acc.x = c_block_sum(acc.x, sh);
-    acc.y = c_block_sum(acc.y, sh);
-    if (threadIdx.x == 0) *out = acc;
+    __syncthreads();
+    return make_double2(sh[2 * CGM_W], sh[2 * CGM_W + 1]);
 }
-// w -= (*h) v
-__global__ void cgm_axpy(double2 *__restrict__ w, const double2 *__restrict__ v, const double2 *__restrict__ h,
-                         int64_t n) {
-    const double2 c = *h;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        w[i] = c_sub(w[i], c_mul(c, v[i]));
+
+// r = b - ax, the norms of b and r, v_0 = r / ||r||; the start's test
+__global__ void __launch_bounds__(CGM_T) cgm_start_kernel(CgmDev g, const double2 *__restrict__ b, const double2 *__restrict__ ax) {
+    __shared__ double sh[2 * CGM_W + 2];
+    int64_t r0, r1;
+    cgm_rows(g.N, g.nblk, r0, r1);
+    double2 acc = make_double2(0.0, 0.0);
+    for (int64_t t = r0 + threadIdx.x; t < r1; t += CGM_T) {
+        const double2 bt = b[t], r = c_sub(bt, ax[t]);
+        g.w[t] = r;
+        acc.x += c_abs2(bt);
+        acc.y += c_abs2(r);
+    }
+    acc = cgm_sum(g, acc, g.part, sh);
+    const double nb = sqrt(acc.x), beta = sqrt(acc.y), normb = nb == 0.0 ? 1.0 : nb, ib = 1.0 / beta;
+    for (int64_t t = r0 + threadIdx.x; t < r1; t += CGM_T) {
+        const double2 r = g.w[t], v = make_double2(__dmul_rn(r.x, ib), __dmul_rn(r.y, ib));
+        g.V[t] = v;
+        g.vcur[t] = v;
+    }
+    if (blockIdx.x != 0) return;
+    for (int k = threadIdx.x; k <= g.m; k += CGM_T) g.s[k] = make_double2(k == 0 ? beta : 0.0, 0.0);
+    if (threadIdx.x == 0) {
+        const double res = beta / normb;
+        g.scal[0] = normb;
+        g.scal[1] = res;
+        g.scal[2] = res <= g.scal[6] ? 2.0 : 0.0;
+        g.iter[0] = g.iter[1] = 0;
+    }
 }
-// dst = src * s (s real)
-__global__ void cgm_scale(double2 *__restrict__ dst, const double2 *__restrict__ src, double s, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        dst[i] = make_double2(__dmul_rn(src[i].x, s), __dmul_rn(src[i].y, s));
+
+// ApplyPlaneRotation (gmres.hpp:70-75); herm: the unitary one
+__device__ __forceinline__ void cgm_apply(double2 &dx, double2 &dy, double2 cs, double2 sn, int herm) {
+    const double2 t = c_add(c_mul(cs, dx), c_mul(sn, dy));
+    const double2 n = make_double2(-sn.x, herm ? sn.y : -sn.y);
+    dy = c_add(c_mul(n, dx), c_mul(cs, dy));
+    dx = t;
 }
-// x += sum_j v_j y_j (y: k complex coefficients, v: column-major n x k)
-__global__ void cgm_update(double2 *__restrict__ x, const double2 *__restrict__ V, const double2 *__restrict__ y,
-                           int k, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+
+__global__ void __launch_bounds__(CGM_T) cgm_step_kernel(CgmDev g, int ws_rows, cudaGraphConditionalHandle hnd, int cond) {
+    extern __shared__ __align__(16) unsigned char cgm_smem[];
+    __shared__ double sh[2 * CGM_W + 2];
+    double2 *wsh = reinterpret_cast<double2 *>(cgm_smem);
+    const int tid = threadIdx.x, i = *g.iter;
+    if (g.scal[2] != 0.0) {  // done; CTA 0 changes these two only after the last barrier
+        if (cond && blockIdx.x == 0 && tid == 0) cudaGraphSetConditional(hnd, 0u);
+        return;
+    }
+    int64_t r0, r1;
+    cgm_rows(g.N, g.nblk, r0, r1);
+    const int rows = (int)(r1 - r0);
+    double2 *w = ws_rows > 0 ? wsh : g.w + r0;  // a thread's own rows: no other reads them
+    if (ws_rows > 0)
+        for (int t = tid; t < rows; t += CGM_T) w[t] = g.w[r0 + t];
+    double2 *Hc = g.H + (size_t)i * (g.m + 1);
+#pragma unroll 1
+    for (int k = 0; k <= i; ++k) {
+        const double2 *v = g.V + (size_t)k * g.N + r0;
+        double2 acc = make_double2(0.0, 0.0);
+        for (int t = tid; t < rows; t += CGM_T) {
+            const double2 p = g.herm ? c_cmul(v[t], w[t]) : c_cmul(w[t], v[t]);
+            acc.x += p.x;
+            acc.y += p.y;
+        }
+        const double2 c = cgm_sum(g, acc, g.part + (size_t)k * g.nblk, sh);
+        for (int t = tid; t < rows; t += CGM_T) w[t] = c_sub(w[t], c_mul(c, v[t]));
+        if (blockIdx.x == 0 && tid == 0) Hc[k] = c;
+    }
+    double2 acc = make_double2(0.0, 0.0);
+    for (int t = tid; t < rows; t += CGM_T) acc.x += c_abs2(w[t]);
+    const double hn = sqrt(cgm_sum(g, acc, g.part + (size_t)(i + 1) * g.nblk, sh).x), ih = 1.0 / hn;
+    double2 *Vn = g.V + (size_t)(i + 1) * g.N + r0;
+    for (int t = tid; t < rows; t += CGM_T) {
+        const double2 v = make_double2(__dmul_rn(w[t].x, ih), __dmul_rn(w[t].y, ih));
+        Vn[t] = v;
+        g.vcur[r0 + t] = v;
+    }
+    if (blockIdx.x != 0 || tid != 0) return;
+    // the column's rotations (GeneratePlaneRotation: gmres.hpp:52-68); this lane wrote it
+    double2 h = Hc[0], next = make_double2(hn, 0.0);
+    for (int k = 0; k < i; ++k) {
+        double2 below = Hc[k + 1];
+        cgm_apply(h, below, g.cs[k], g.sn[k], g.herm);
+        Hc[k] = h;
+        h = below;
+    }
+    double2 cs = make_double2(0.0, 0.0), sn = make_double2(1.0, 0.0);
+    if (h.x != 0.0 || h.y != 0.0) {
+        const double ax = c_abs(h), ay = c_abs(next), scale = ax + ay;
+        const double qx = c_abs(make_double2(h.x / scale, h.y / scale)), qy = c_abs(make_double2(next.x / scale, next.y / scale));
+        const double nrm = scale * sqrt(qx * qx + qy * qy);
+        const double2 al = make_double2(h.x / ax, h.y / ax), p = c_mul(al, make_double2(next.x, -next.y));
+        cs = make_double2(ax / nrm, 0.0);
+        sn = make_double2(p.x / nrm, p.y / nrm);
+    }
+    g.cs[i] = cs;
+    g.sn[i] = sn;
+    cgm_apply(h, next, cs, sn, g.herm);
+    Hc[i] = h;
+    Hc[i + 1] = next;
+    double2 s0 = g.s[i], s1 = g.s[i + 1];
+    cgm_apply(s0, s1, cs, sn, g.herm);
+    g.s[i] = s0;
+    g.s[i + 1] = s1;
+    const double res = c_abs(s1) / g.scal[0];
+    g.scal[1] = res;
+    const bool stop = res < g.scal[6];
+    if (stop) g.scal[2] = 1.0;
+    else if (i + 1 < g.m) *g.iter = i + 1;
+    const int n = ++g.iter[1];
+    if (cond) cudaGraphSetConditional(hnd, !stop && n < g.m ? 1u : 0u);
+}
+
+// y: the steps taken's triangular system (one CTA; in shared memory where it fits)
+__global__ void __launch_bounds__(CGM_T) cgm_backsub_kernel(CgmDev g, int shared) {
+    extern __shared__ __align__(16) unsigned char cgm_smem[];
+    double2 *y = shared ? reinterpret_cast<double2 *>(cgm_smem) : g.y;
+    const int k = g.iter[1];
+    for (int j = threadIdx.x; j < k; j += CGM_T) y[j] = g.s[j];
+    __syncthreads();
+    for (int i = k - 1; i >= 0; --i) {
+        const double2 *H = g.H + (size_t)i * (g.m + 1);
+        const double2 yi = c_div(y[i], H[i]);
+        __syncthreads();
+        for (int j = threadIdx.x; j < i; j += CGM_T) y[j] = c_sub(y[j], c_mul(H[j], yi));
+        if (threadIdx.x == 0) y[i] = yi;
+        __syncthreads();
+    }
+    if (shared)
+        for (int j = threadIdx.x; j < k; j += CGM_T) g.y[j] = y[j];
+}
+// x += sum_j v_j y_j
+__global__ void cgm_update_kernel(CgmDev g, double2 *__restrict__ x) {
+    const int k = g.iter[1];
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x) {
         double2 a = x[i];
-        for (int j = 0; j < k; ++j) a = c_add(a, c_mul(V[(size_t)j * n + i], y[j]));
+        for (int j = 0; j < k; ++j) a = c_add(a, c_mul(g.V[(size_t)j * g.N + i], g.y[j]));
         x[i] = a;
     }
 }
-// r = b - Ax
-__global__ void cgm_resid(double2 *__restrict__ r, const double2 *__restrict__ b, const double2 *__restrict__ ax,
-                          int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        r[i] = c_sub(b[i], ax[i]);
-}
 
-cudaError_t cgm_dot(const double2 *a, const double2 *b, int64_t n, double2 *part, double2 *out, cudaStream_t st) {
-    cgm_dot_part<<<CGM_BLOCKS, CGM_THREADS, 0, st>>>(a, b, n, part);
-    cgm_dot_fin<<<1, CGM_THREADS, 0, st>>>(part, CGM_BLOCKS, out);
+int cgm_blocks(int64_t N) {  // one CTA an SM at most, and at least a row a thread
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int64_t want = (N + CGM_T - 1) / CGM_T;
+    return (int)(want < 1 ? 1 : want < sms ? want : sms > 0 ? sms : 1);
+}
+void cgm_prepare() {
+    cudaFuncSetAttribute(cgm_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(cgm_backsub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+}
+cudaError_t cgm_start(const CgmDev &g, const double2 *b, const double2 *ax, cudaStream_t st) {
+    CgmDev ga = g;
+    void *args[] = {(void *)&ga, (void *)&b, (void *)&ax};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)cgm_start_kernel, dim3(g.nblk), dim3(CGM_T), args, 0, st);
+    count_launch();
+    return e;
+}
+cudaError_t cgm_step(const CgmDev &g, const cudaGraphConditionalHandle *hnd, cudaStream_t st) {
+    const int64_t chunk = (g.N + g.nblk - 1) / g.nblk;
+    int ws_rows = chunk * 16 <= 200 * 1024 ? (int)chunk : 0, cond = hnd ? 1 : 0;
+    cudaGraphConditionalHandle c = hnd ? *hnd : cudaGraphConditionalHandle{};
+    CgmDev ga = g;
+    void *args[] = {(void *)&ga, (void *)&ws_rows, (void *)&c, (void *)&cond};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)cgm_step_kernel, dim3(g.nblk), dim3(CGM_T), args,
+                                                      (size_t)ws_rows * 16, st);
+    count_launch();
+    return e;
+}
+cudaError_t cgm_update(const CgmDev &g, double2 *x, cudaStream_t st) {
+    const size_t smem = (size_t)g.m * 16 <= 200 * 1024 ? (size_t)g.m * 16 : 0;
+    cgm_backsub_kernel<<<1, CGM_T, smem, st>>>(g, smem > 0);
+    cgm_update_kernel<<<304, CGM_T, 0, st>>>(g, x);
     count_launch(2);
     return cudaGetLastError();
 }
-cudaError_t cgm_axpy_launch(double2 *w, const double2 *v, const double2 *h, int64_t n, cudaStream_t st) {
-    cgm_axpy<<<CGM_BLOCKS, CGM_THREADS, 0, st>>>(w, v, h, n);
-    count_launch();
-    return cudaGetLastError();
-}
-cudaError_t cgm_scale_launch(double2 *dst, const double2 *src, double s, int64_t n, cudaStream_t st) {
-    cgm_scale<<<CGM_BLOCKS, CGM_THREADS, 0, st>>>(dst, src, s, n);
-    count_launch();
-    return cudaGetLastError();
-}
-cudaError_t cgm_update_launch(double2 *x, const double2 *V, const double2 *y, int k, int64_t n, cudaStream_t st) {
-    if (k <= 0) return cudaSuccess;
-    cgm_update<<<CGM_BLOCKS, CGM_THREADS, 0, st>>>(x, V, y, k, n);
-    count_launch();
-    return cudaGetLastError();
-}
-cudaError_t cgm_resid_launch(double2 *r, const double2 *b, const double2 *ax, int64_t n, cudaStream_t st) {
-    cgm_resid<<<CGM_BLOCKS, CGM_THREADS, 0, st>>>(r, b, ax, n);
-    count_launch();
-    return cudaGetLastError();
-}
-int cgm_blocks() { return CGM_BLOCKS; }
 
 }  // namespace h2w

@@ -185,15 +185,24 @@ cudaError_t launch_assemble_c(const FactorJob *fac, int nfac, const XferJob *xf,
 cudaError_t launch_realify(const int64_t *blk, int64_t nblk, const double2 *opc, double *op, cudaStream_t st);
 cudaError_t launch_dense_c(const KParams &kp, int64_t N, const double2 *x, double2 *y, int64_t row0, int64_t nrows,
                            cudaStream_t st);
-// The reference GMRES's complex vector operations (n complex entries):
-// out = sum conj(a_i) b_i (part: cgm_blocks() scratch entries), w -= (*h) v,
-// dst = s src (s real), x += sum_j V[:, j] y_j, r = b - ax.
-int cgm_blocks();
-cudaError_t cgm_dot(const double2 *a, const double2 *b, int64_t n, double2 *part, double2 *out, cudaStream_t st);
-cudaError_t cgm_axpy_launch(double2 *w, const double2 *v, const double2 *h, int64_t n, cudaStream_t st);
-cudaError_t cgm_scale_launch(double2 *dst, const double2 *src, double s, int64_t n, cudaStream_t st);
-cudaError_t cgm_update_launch(double2 *x, const double2 *V, const double2 *y, int k, int64_t n, cudaStream_t st);
-cudaError_t cgm_resid_launch(double2 *r, const double2 *b, const double2 *ax, int64_t n, cudaStream_t st);
+// The reference GMRES on complex vectors of N entries (helm.cu)
+struct CgmDev {
+    double2 *V, *w, *vcur, *H, *cs, *sn, *s, *y;  // V: N x (m+1); H: (m+1) x m column-major
+    double2 *part;                                // nblk (m+2) partial sums
+    double *scal;                                 // [0] ||b||, [1] resid, [2] 0 running, 1 converged, 2 at the start,
+                                                  // [6] stopping tolerance
+    int32_t *iter;                                // [0] current Arnoldi column i, [1] steps taken
+    unsigned *bar;
+    int32_t *err;
+    int64_t N;
+    int m, nblk, herm;  // herm: Hermitian projections, unitary rotations
+};
+int cgm_blocks(int64_t N);  // nblk
+void cgm_prepare();         // kernel attributes, before a capture
+cudaError_t cgm_start(const CgmDev &g, const double2 *b, const double2 *ax, cudaStream_t st);
+// one Arnoldi step on w = A vcur; hnd (may be NULL): the while condition of a captured step
+cudaError_t cgm_step(const CgmDev &g, const cudaGraphConditionalHandle *hnd, cudaStream_t st);
+cudaError_t cgm_update(const CgmDev &g, double2 *x, cudaStream_t st);  // x += V y
 
 // Dense FP64 oracle rows y[r] = sum_j K(r, j) x[j], r in [row0, row0+nrows).
 cudaError_t launch_dense_matvec(const KParams &kp, int64_t N, const double *x, double *y, int64_t row0,
