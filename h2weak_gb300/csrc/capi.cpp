@@ -3381,7 +3381,7 @@ void run_matvec_multi(h2w_handle *h, int prec, int rp, const double *xi, double 
             if (h->m_wsd.n < need) h->m_wsd.alloc(need);
             const MoArgs a = mo_args(h, rp, xi, yi);
             mr_prof(h, prec, rp, st, [&] { return launch_mo(a, st); });
-            if (!h->mo.fused) CK(launch_mo_unplane(a, h->tree.N, yi, st));
+            if (!h->mo.fused) CK(launch_mo_unplane(a, h->yperm_off, h->tree.N, yi, st));
             return;
         }
         if (h->m_wsd.n < wsz) h->m_wsd.alloc(wsz);

@@ -419,7 +419,7 @@ cudaError_t launch_mo_image(const MoHdr *hdr, int64_t nt, const int64_t *s0, con
                             char *img, int32_t *sa, int32_t *bad, cudaStream_t st);
 cudaError_t launch_mo(const MoArgs &a, cudaStream_t st);
 // the first n rows of the workspace planes as an interleaved block
-cudaError_t launch_mo_unplane(const MoArgs &a, int64_t n, double *y, cudaStream_t st);
+cudaError_t launch_mo_unplane(const MoArgs &a, int64_t r0, int64_t n, double *y, cudaStream_t st);
 // Double-FP32 arithmetic on the FP32 pipes (each product and sum carried as
 // an FP32 pair; about 2^-44 relative per term instead of FP64's 2^-53): A and
 // xin are (hi, lo) pairs (launch_mr_split of the FP64 operator and input),

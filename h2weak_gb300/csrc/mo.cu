@@ -745,12 +745,13 @@ __global__ void __launch_bounds__(MO_NT, 1) mo_kernel(const MoArgs a) {
     if (lane == 0) mo_arrive(quit);
 }
 
-// y (n x ld, interleaved) from the rows of the workspace planes
-__global__ void mo_unplane_kernel(const double *__restrict__ ws, int64_t rows, int gc, int ld, int64_t n, double *__restrict__ y) {
+// y (n x ld, interleaved) from the workspace planes' rows r0 ..
+__global__ void mo_unplane_kernel(const double *__restrict__ ws, int64_t rows, int64_t r0, int gc, int ld, int64_t n,
+                                  double *__restrict__ y) {
     for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * ld; e += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = e / ld;
         const int c = (int)(e - r * ld);
-        y[e] = ws[((int64_t)(c / gc) * rows + r) * gc + c % gc];
+        y[e] = ws[((int64_t)(c / gc) * rows + r0 + r) * gc + c % gc];
     }
 }
 
@@ -843,8 +844,8 @@ cudaError_t launch_mo_image(const MoHdr *hdr, int64_t nt, const int64_t *s0, con
 cudaError_t launch_mo(const MoArgs &a, cudaStream_t st) {
     return a.ld == 16 ? mo_launch_t<16>(a, st) : a.ld == 32 || a.ld == 64 ? mo_launch_t<32>(a, st) : cudaErrorInvalidValue;
 }
-cudaError_t launch_mo_unplane(const MoArgs &a, int64_t n, double *y, cudaStream_t st) {
-    mo_unplane_kernel<<<1216, 256, 0, st>>>(a.ws, a.rows, a.ld == 16 ? 16 : 32, a.ld, n, y);
+cudaError_t launch_mo_unplane(const MoArgs &a, int64_t r0, int64_t n, double *y, cudaStream_t st) {
+    mo_unplane_kernel<<<1216, 256, 0, st>>>(a.ws, a.rows, r0, a.ld == 16 ? 16 : 32, a.ld, n, y);
     count_launch();
     return cudaGetLastError();
 }

@@ -21,6 +21,8 @@ CASES = {
     "2d_plain": (2, 2, 1, 8, 3, -1501),
     "3d_wide": (3, 0, 0, 7, 2, -5003),
     "3d_semi_wide": (3, 1, 1, 7, 2, -4001),
+    "3d_one_level_down": (3, 0, 0, 7, 3, 13),
+    "2d_three_boxes": (2, 0, 1, 8, 3, -271),
 }
 
 
@@ -31,7 +33,10 @@ def make(hw, case):
     if n > 0:
         op.gen_grid(n)
     else:
-        op.set_points(synth.uniform_points(synth.config_seed(63, N), N, dim))
+        p = synth.uniform_points(synth.config_seed(63, N), N, dim)
+        if case == "2d_three_boxes":  # all points in a row of three leaf boxes: the middle one has no far field
+            p = np.ascontiguousarray((p + 1.0) * [0.375, 0.125] - 1.0)
+        op.set_points(p)
     op.build_tree()
     op.assemble()
     return op
