@@ -219,7 +219,7 @@ struct h2w_handle {
     DBuf<double> s_b, s_x, s_r, s_d;   // solver vectors in leaf order (kept between calls)
     // multiple right-hand sides: interleaved workspaces (ws_n x rp), staging, batched GMRES
     DBuf<double> m_wsd, m_xi, m_yi, m_ri, m_di, m_bi, m_stage_x, m_stage_y, m_onorm, m_ores;
-    DBuf<float> m_wsf, m_xf;
+    DBuf<float> m_wsf, m_xf, m_yf;
     DBuf<double> d_opdf, m_xdf;  // (hi, lo) FP32 pairs (8 bytes each) of the operator and of an input block
     std::vector<int64_t> ph_t0, ph_t1;   // phase target ranges (per-phase launches)
     GmbStore<double> gbd;  // FP64 Krylov vectors (FP64 solves)
@@ -4834,7 +4834,6 @@ int h2w_matvec(h2w_handle *h, const double *x, double *y, int nrhs, int precisio
         const bool df_single = nrhs == 1 && precision == H2W_PREC_DF64 && h->fly_active;
         if (nrhs > 1 || (precision == H2W_PREC_DF64 && !df_single)) {
             // blocks of up to 64 columns through the multi-vector kernel
-            ensure_multi_vectors(h);
             if (where == H2W_HOST) {
                 if (h->m_stage_x.n < (size_t)N * MR_MAX) h->m_stage_x.alloc((size_t)N * MR_MAX);
                 if (h->m_stage_y.n < (size_t)N * MR_MAX) h->m_stage_y.alloc((size_t)N * MR_MAX);
@@ -4847,10 +4846,19 @@ int h2w_matvec(h2w_handle *h, const double *x, double *y, int nrhs, int precisio
                     CK(cudaMemcpyAsync(h->m_stage_x.p, xc, (size_t)N * nc * 8, cudaMemcpyHostToDevice, st));
                     xc = h->m_stage_x.p;
                 }
-                CK(launch_mr_pack(xc, N, h->m_xi.p, h->d_perm.p, N, nc, rp, st));
-                run_matvec_multi(h, precision, rp, h->m_xi.p, h->m_yi.p, st);
-                CK(launch_mr_unpack(h->m_yi.p, where == H2W_HOST ? h->m_stage_y.p : yc, N, h->d_perm.p, N, nc, rp,
-                                    st));
+                double *out = where == H2W_HOST ? h->m_stage_y.p : yc;
+                if (precision == H2W_PREC_FP32) {
+                    for (DBuf<float> *v : {&h->m_xf, &h->m_yf})
+                        if (v->n < (size_t)N * rp) v->alloc((size_t)N * rp);
+                    CK(launch_mr_pack(xc, N, h->m_xf.p, h->d_perm.p, N, nc, rp, st));
+                    run_matvec_multi_f32io(h, rp, h->m_xf.p, h->m_yf.p, st);
+                    CK(launch_mr_unpack(h->m_yf.p, out, N, h->d_perm.p, N, nc, rp, st));
+                } else {
+                    ensure_multi_vectors(h);
+                    CK(launch_mr_pack(xc, N, h->m_xi.p, h->d_perm.p, N, nc, rp, st));
+                    run_matvec_multi(h, precision, rp, h->m_xi.p, h->m_yi.p, st);
+                    CK(launch_mr_unpack(h->m_yi.p, out, N, h->d_perm.p, N, nc, rp, st));
+                }
                 if (where == H2W_HOST)
                     CK(cudaMemcpyAsync(yc, h->m_stage_y.p, (size_t)N * nc * 8, cudaMemcpyDeviceToHost, st));
             }

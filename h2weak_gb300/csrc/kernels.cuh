@@ -440,10 +440,12 @@ cudaError_t launch_mr_df64(int rp, const int64_t *roff, const int64_t *blob, con
 cudaError_t launch_mr_split(const double *a, void *b, int64_t n, cudaStream_t st);
 // calibration vectors (even columns pseudo-random, odd columns smooth), n x rp interleaved
 cudaError_t launch_calib_fill(double *z, int64_t n, int rp, int c0, cudaStream_t st);
-cudaError_t launch_mr_pack(const double *x, int64_t ldx, double *xi, const int32_t *perm, int64_t n, int nrhs,
-                           int rp, cudaStream_t st);
-cudaError_t launch_mr_unpack(const double *yi, double *y, int64_t ldy, const int32_t *perm, int64_t n, int nrhs,
-                             int rp, cudaStream_t st);
+template <class T>  // double or float
+cudaError_t launch_mr_pack(const double *x, int64_t ldx, T *xi, const int32_t *perm, int64_t n, int nrhs, int rp,
+                           cudaStream_t st);
+template <class T>
+cudaError_t launch_mr_unpack(const T *yi, double *y, int64_t ldy, const int32_t *perm, int64_t n, int nrhs, int rp,
+                             cudaStream_t st);
 cudaError_t launch_mr_widen_f64(const double *a, double *b, int64_t n, cudaStream_t st);
 cudaError_t launch_mr_widen_f32(const float *a, double *b, int64_t n, cudaStream_t st);
 
