@@ -2767,9 +2767,17 @@ void build_plan(h2w_handle *h) {
         h->d_pts4.alloc((size_t)t.N * 4);
         CK(launch_pts4(h->d_pts.p, dim, t.N, h->d_pts4.p, st));
         h->d_ptsdf.alloc((size_t)t.N * 8);
+        // the log table covers R^2 from the square of the deepest boxes' width (far boxes are not
+        // adjacent) to that of the points' largest distance
+        double big = 0.0;
+        for (double v : h->pts) big = std::max(big, std::fabs(v));
+        const int eb = big > 0.0 ? std::ilogb(big) + 1 : 0;  // |x| < 2^eb
         CK(launch_ptsdf(h->d_pts.p, dim, t.N, h->d_ptsdf.p, st));
-        std::vector<float> lt(128 * 8);
-        fly_df_logtab(lt.data());
+        const int e0 = 2 - 2 * L - 1, ne = 2 * eb + 2 + 2 - e0;  // R^2 <= dim 2^(2 eb + 2)
+        h->k32.tab_e0 = e0;
+        h->k32.ntab = ne > 0 && ne <= 90 ? 128 * ne : 0;
+        std::vector<float> lt((size_t)std::max(4 * h->k32.ntab, 4));
+        if (h->k32.ntab > 0) fly_df_table(e0, ne, lt.data());
         h->d_logtab.upload(lt, st);
         CK(cudaStreamSynchronize(st));
         const double a = 0.0001;

@@ -151,6 +151,7 @@ struct FlyItem {
 struct FlyK32 {
     float c2d, inv4pi, inv_loga, inv_den, a, a2, inv_a;
     int32_t sep;  // every far pair is farther apart than a (deepest box wider than a)
+    int32_t tab_e0, ntab;  // first exponent and entries of the log table (fly_df_table; 0: none)
 };
 cudaError_t launch_fly_f64(const FlyItem *items, int64_t nitems, unsigned long long *ctr, const int32_t *rowpid,
                            const int32_t *cpid, const int32_t *cws, double *ws, const KParams &kp, cudaStream_t st);
@@ -162,12 +163,13 @@ cudaError_t launch_pts4(const double *pts, int dim, int64_t n, float *out, cudaS
 // The FP64-accurate form on the FP32 pipes (double-FP32 arithmetic) for the
 // kernels built on log(R^2) when every far pair is farther apart than a (else
 // the FP64 form): ptsdf = (hi, lo) FP32 quadruples of the points
-// (launch_ptsdf, 8 floats per point), logtab = fly_df_logtab's 128 x 8 floats.
+// (launch_ptsdf, 8 floats per point), logtab = fly_df_table's entries.
 bool fly_df_supported(const KParams &kp, const FlyK32 &k32);
 cudaError_t launch_fly_df64(const FlyItem *items, int64_t nitems, unsigned long long *ctr, const int32_t *rowpid,
                             const int32_t *cpid, const int32_t *cws, const float *ptsdf, const void *logtab,
                             double *ws, const KParams &kp, const FlyK32 &k32, cudaStream_t st);
-void fly_df_logtab(float *out);
+void fly_df_table(int e0, int ne, float *out);  // 128 ne x 4 floats
+void fly_df_logtab(float *out);                 // of the pivot search, 128 x 8 floats
 cudaError_t launch_ptsdf(const double *pts, int dim, int64_t n, float *out, cudaStream_t st);
 
 // Complex Helmholtz kernels (helm.cu). Positions of the assembly jobs are in

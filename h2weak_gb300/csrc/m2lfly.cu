@@ -19,6 +19,7 @@
 // first writer of them in the product. The FP64 form evaluates the entries
 // with a few ulps of the stored ones (fly_entry64); the FP32 form evaluates
 // them in FP32 from FP32 coordinates.
+#include <algorithm>
 #include <cmath>
 
 #include "dfmath.cuh"
@@ -256,25 +257,55 @@ __global__ void __launch_bounds__(FLY_THREADS)
 // ---- double-FP32 form (FP64-accurate far M2L on the FP32 pipes) ---------
 //
 // GB300 runs FP64 at 1/64 of its FP32 rate, and the FP64 entries spend it on
-// the logarithm. Here every value is an unevaluated pair of floats and every
-// operation an error-free transformation (dfmath.cuh); the points are split
-// once into (hi, lo) pairs, R^2 is formed from pair differences and log(R^2)
-// by the table-driven pair logarithm. Each row's sum is a pair; the kernel's
-// constant multiplies it once. For the kernels built on log(R^2) (3D RBF, 2D
-// integral equation) with every far pair farther apart than a; the others
-// keep the FP64 form.
+// the logarithm. Here values are unevaluated pairs of floats. Issue slots bound it, so
+// no operation keeps more of a pair than the next one needs:
+//  * differences of the points' pairs stay a rounded high part and its error with the lows: the
+//    square's cross term takes both, so nothing is renormalised before R^2 is whole;
+//  * log(R^2) by Tang's table method (ACM TOMS 16(4), 1990) with a table over exponent
+//    and bin, log c and 1 / c of the bin's centre c as pairs: no scaling to [1, 2), no
+//    pair of e log 2; log(1 + u) = u - u^2/2 + u^3 (1/3 - u/4 + u^2/5), |u| <= 2^-8 (the u^6
+//    term is below 2^-50);
+//  * sums whose larger term is known take three operations (Dekker's FastTwoSum).
+// Two columns a thread at a time hide the chains' latency. About 113 operations an entry (165 with general pair arithmetic). The logarithm's error, rms
+// over far pairs of boxes 1/2 to 1/16 wide: 5e-15 to 4e-14, before 5e-14 to 6e-13 (the pair of
+// log 2 carried 44 bits). A launch of the 3D RBF operator of 65536 points: 5.56 -> 3.96 ms.
+// Each row's sum is a pair; the kernel's constant multiplies it once. For the kernels built on
+// log(R^2) (3D RBF, 2D integral equation) with every far pair farther apart than a; the
+// others keep the FP64 form.
 
-// the FP64-accurate far M2L: rows' sums as pairs times `scale`, into an FP64 workspace
+// log of r.h + r.l > 0 within the table's range (a pair, not renormalised); tab: n entries from
+// the bin of bits `base`, (log c, 1 / c) pairs
+__device__ __forceinline__ Df fly_log(Df r, const float4 *tab, unsigned base, unsigned n) {
+    const unsigned bits = __float_as_uint(r.h);
+    const float4 t = tab[min((bits >> 16) - base, n - 1u)];
+    const float d = __fsub_rn(r.h, __uint_as_float((bits & 0xffff0000u) | 0x8000u));  // r.h - c, exact
+    const float u0 = __fmul_rn(d, t.z);
+    float e = __fmaf_rn(d, t.z, -u0);
+    e = __fmaf_rn(d, t.w, e);
+    e = __fmaf_rn(r.l, t.z, e);
+    const Df u = df_fast(u0, e);  // d is zero or at least 2 |r.l|
+    const float p = __fmul_rn(u.h, u.h);
+    const float q = __fmaf_rn(__fadd_rn(u.h, u.h), u.l, __fmaf_rn(u.h, u.h, -p));
+    const float s = __fmaf_rn(-0.5f, p, u.h);
+    const float es = __fmaf_rn(-0.5f, p, __fsub_rn(u.h, s));
+    const float poly = __fmaf_rn(u.h, __fmaf_rn(u.h, 0.2f, -0.25f), 0.33333334f);
+    const float low = __fadd_rn(__fmaf_rn(-0.5f, q, __fmul_rn(__fmul_rn(p, u.h), poly)), __fadd_rn(u.l, es));
+    const Df g = df_two_sum(t.x, s);
+    return {g.h, __fadd_rn(g.l, __fadd_rn(t.y, low))};
+}
+
+// the FP64-accurate far M2L: rows' sums as pairs times `scale`, into an FP64 workspace. An
+// item of at most 16, 8 or 4 rows gives 8, 16 or 32 threads to a row in place of four.
 template <int DIM>
 __global__ void __launch_bounds__(FLY_THREADS)
     m2l_flydf_kernel(const FlyItem *__restrict__ items, int64_t nitems, unsigned long long *ctr,
                      const int32_t *__restrict__ rowpid, const int32_t *__restrict__ cpid,
                      const int32_t *__restrict__ cws, const float *__restrict__ ptsdf, double *ws,
-                     const DfLogTab *__restrict__ gtab, double scale) {
+                     const float4 *__restrict__ gtab, unsigned base, unsigned ntab, double scale) {
+    extern __shared__ __align__(16) float4 fly_tab[];
     __shared__ __align__(16) float sc[FLY_TILE][8];  // x, y, z hi; x, y, z lo; value hi, lo
-    __shared__ __align__(16) DfLogTab tab[128];
     __shared__ long long s_it;
-    for (int i = threadIdx.x; i < 128; i += FLY_THREADS) tab[i] = gtab[i];
+    for (unsigned i = threadIdx.x; i < ntab; i += FLY_THREADS) fly_tab[i] = gtab[i];
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) s_it = (long long)atomicAdd(ctr, 1ull);
@@ -282,15 +313,16 @@ __global__ void __launch_bounds__(FLY_THREADS)
         const long long it = s_it;
         if (it >= nitems) return;
         const FlyItem m = items[it];
-        const int row = threadIdx.x / FLY_TPR, sub = threadIdx.x - row * FLY_TPR;
+        const int lt = m.nrows > 16 ? 2 : m.nrows > 8 ? 3 : m.nrows > 4 ? 4 : 5, tpr = 1 << lt;
+        const int row = threadIdx.x >> lt, sub = threadIdx.x & (tpr - 1);
         const bool has = row < m.nrows;
-        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f};
         if (has) {
             const float4 *q = reinterpret_cast<const float4 *>(ptsdf) + 2 * (int64_t)rowpid[m.rows + row];
             const float4 hi = q[0], lo = q[1];
-            a[0] = hi.x; a[1] = hi.y; a[2] = hi.z; a[4] = lo.x; a[5] = lo.y; a[6] = lo.z;
+            ah[0] = hi.x; ah[1] = hi.y; ah[2] = hi.z; al[0] = lo.x; al[1] = lo.y; al[2] = lo.z;
         }
-        Df acc{0.f, 0.f};
+        Df acc{0.f, 0.f}, acc2{0.f, 0.f};
         for (int c0 = 0; c0 < m.ncols; c0 += FLY_TILE) {
             const int nc = m.ncols - c0 < FLY_TILE ? m.ncols - c0 : FLY_TILE;
             __syncthreads();
@@ -306,28 +338,45 @@ __global__ void __launch_bounds__(FLY_THREADS)
             }
             __syncthreads();
             if (has) {
-                for (int c = sub; c < nc; c += FLY_TPR) {
+                auto entry = [&](int c, Df &sum) {
                     const float4 p0 = reinterpret_cast<const float4 *>(sc[c])[0];
                     const float4 p1 = reinterpret_cast<const float4 *>(sc[c])[1];
-                    const Df dx = df_sub(Df{a[0], a[4]}, Df{p0.x, p0.w});
-                    const Df dy = df_sub(Df{a[1], a[5]}, Df{p0.y, p1.x});
-                    const Df sx = df_sqr(dx), sy = df_sqr(dy);
-                    Df r2 = df_add(sx, sy);
-                    if (DIM == 3) r2 = df_add(r2, df_sqr(df_sub(Df{a[2], a[6]}, Df{p0.z, p1.y})));
-                    const Df lg = df_log(r2, tab);
-                    // acc += lg * v
+                    const float bh[3] = {p0.x, p0.y, p0.z}, bl[3] = {p0.w, p1.x, p1.y};
+                    // R^2: squares of h + l with their errors, summed
+                    Df r2{0.f, 0.f};
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) {
+                        const Df h = df_two_sum(ah[d], -bh[d]);
+                        const float l = __fadd_rn(h.l, __fsub_rn(al[d], bl[d])), p = __fmul_rn(h.h, h.h);
+                        const float e = __fmaf_rn(__fmaf_rn(2.f, h.h, l), l, __fmaf_rn(h.h, h.h, -p));
+                        if (d == 0) {
+                            r2 = Df{p, e};
+                        } else {
+                            const Df t = df_two_sum(r2.h, p);
+                            r2 = Df{t.h, __fadd_rn(__fadd_rn(r2.l, e), t.l)};
+                        }
+                    }
+                    const Df lg = fly_log(df_fast(r2.h, r2.l), fly_tab, base, ntab);
+                    // sum += lg * v
                     const float ph = __fmul_rn(lg.h, p1.z);
                     float pe = __fmaf_rn(lg.h, p1.z, -ph);
                     pe = __fmaf_rn(lg.h, p1.w, pe);
                     pe = __fmaf_rn(lg.l, p1.z, pe);
-                    const Df s2 = df_two_sum(acc.h, ph);
-                    acc = df_fast(s2.h, __fadd_rn(s2.l, __fadd_rn(acc.l, pe)));
+                    const Df s2 = df_two_sum(sum.h, ph);
+                    sum = df_fast(s2.h, __fadd_rn(s2.l, __fadd_rn(sum.l, pe)));
+                };
+                int c = sub;
+#pragma unroll 1
+                for (; c + tpr < nc; c += 2 * tpr) {
+                    entry(c, acc);
+                    entry(c + tpr, acc2);
                 }
+                if (c < nc) entry(c, acc);
             }
         }
-        // partial sums of a row's four threads (pairs)
-#pragma unroll
-        for (int o = 1; o < FLY_TPR; o <<= 1) {
+        // partial sums of a row's threads (pairs)
+        acc = df_add(acc, acc2);
+        for (int o = 1; o < tpr; o <<= 1) {
             const Df b{__shfl_xor_sync(0xffffffffu, acc.h, o), __shfl_xor_sync(0xffffffffu, acc.l, o)};
             acc = df_add(acc, b);
         }
@@ -424,23 +473,25 @@ cudaError_t launch_fly_f32(const FlyItem *items, int64_t nitems, unsigned long l
 template <int DIM>
 static cudaError_t flydf_launch(const FlyItem *items, int64_t nitems, unsigned long long *ctr, const int32_t *rowpid,
                                 const int32_t *cpid, const int32_t *cws, const float *ptsdf, double *ws,
-                                const DfLogTab *tab, double scale, cudaStream_t st) {
-    static int per_sm = 0;
-    if (per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m2l_flydf_kernel<DIM>, FLY_THREADS, 0);
-        if (per_sm <= 0) per_sm = 1;
-    }
-    const int64_t cap = (int64_t)fly_sms() * per_sm;
-    const int grid = (int)(nitems < cap ? nitems : cap);
-    cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st);
+                                const float4 *tab, const FlyK32 &k32, double scale, cudaStream_t st) {
+    const size_t smem = (size_t)k32.ntab * sizeof(float4);
+    int per_sm = 0;
+    cudaError_t e = cudaFuncSetAttribute(m2l_flydf_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m2l_flydf_kernel<DIM>, FLY_THREADS, smem);
     if (e != cudaSuccess) return e;
-    m2l_flydf_kernel<DIM><<<grid, FLY_THREADS, 0, st>>>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, scale);
+    const int64_t cap = (int64_t)fly_sms() * std::max(per_sm, 1);
+    const int grid = (int)(nitems < cap ? nitems : cap);
+    e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
+    m2l_flydf_kernel<DIM><<<grid, FLY_THREADS, smem, st>>>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab,
+                                                           (unsigned)(127 + k32.tab_e0) << 7, (unsigned)k32.ntab, scale);
     count_launch();
     return cudaGetLastError();
 }
 
 bool fly_df_supported(const KParams &kp, const FlyK32 &k32) {
-    return k32.sep && ((kp.dim == 3 && kp.choice == 1) || (kp.dim == 2 && kp.choice == 0));
+    return k32.sep && k32.ntab > 0 && ((kp.dim == 3 && kp.choice == 1) || (kp.dim == 2 && kp.choice == 0));
 }
 
 cudaError_t launch_fly_df64(const FlyItem *items, int64_t nitems, unsigned long long *ctr, const int32_t *rowpid,
@@ -449,12 +500,24 @@ cudaError_t launch_fly_df64(const FlyItem *items, int64_t nitems, unsigned long 
     if (nitems <= 0) return cudaSuccess;
     if (!fly_df_supported(kp, k32))
         return fly_dispatch<double>(items, nitems, ctr, rowpid, cpid, cws, kp.pts, ws, kp, FlyK32{}, st);
-    const DfLogTab *tab = reinterpret_cast<const DfLogTab *>(logtab);
-    if (kp.dim == 3) return flydf_launch<3>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, 0.5 / kp.loga, st);
-    return flydf_launch<2>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, kp.c2d, st);
+    const float4 *tab = reinterpret_cast<const float4 *>(logtab);
+    if (kp.dim == 3) return flydf_launch<3>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, k32, 0.5 / kp.loga, st);
+    return flydf_launch<2>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, k32, kp.c2d, st);
 }
 
-// The log table of the double-FP32 form: 128 bins of [1, 2), centre
+// The table of fly_log: 128 bins for each of ne exponents from e0, (log c, 1 / c) as (hi, lo)
+// pairs of their FP64 values. 4 floats per entry.
+void fly_df_table(int e0, int ne, float *out) {
+    for (int k = 0; k < 128 * ne; ++k, out += 4) {
+        const double c = std::ldexp(1.0 + (2.0 * (k % 128) + 1.0) / 256.0, e0 + k / 128), l = std::log(c), i = 1.0 / c;
+        out[0] = (float)l;
+        out[1] = (float)(l - (double)out[0]);
+        out[2] = (float)i;
+        out[3] = (float)(i - (double)out[2]);
+    }
+}
+
+// The log table of the double-FP32 pivot search: 128 bins of [1, 2), centre
 // c_k = 1 + (2k + 1) / 256 (exact in FP32), log c_k and 1 / c_k as (hi, lo)
 // pairs of their FP64 values. 8 floats per entry.
 void fly_df_logtab(float *out) {
