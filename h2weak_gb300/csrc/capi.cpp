@@ -1670,52 +1670,75 @@ void check_phase_writers(const std::vector<int64_t> &roff, const std::vector<int
 void build_deps(const PlanBuilder &pb, int64_t ws_n, std::vector<int32_t> &cnt, std::vector<int64_t> &coff,
                 std::vector<int32_t> &cidx) {
     const size_t nt = pb.T.size();
-    std::vector<int32_t> last_nw((size_t)ws_n, -1);
-    std::vector<std::vector<int32_t>> atom((size_t)ws_n), rd((size_t)ws_n);
+    // Rows that every target reads and writes together are kept as one: blocks between the ends
+    // of all source segments and destinations (2D, 9973 points: 10 ms row by row, 0.5 so).
+    std::vector<int32_t> blk((size_t)ws_n + 1, 0);
+    for (const Target &tg : pb.T) {
+        if (!(tg.flags & T_SCATTER) || (tg.flags & T_ACCUM)) blk[(size_t)tg.dst] = blk[(size_t)(tg.dst + tg.nrows)] = 1;
+        for (int32_t q = tg.p0; q < tg.p1; ++q)
+            for (int32_t e = pb.P[(size_t)q].s0; e < pb.P[(size_t)q].s1; ++e) {
+                const Seg &sg = pb.S[(size_t)e];
+                if (!(sg.flags & S_GATHER)) blk[(size_t)sg.src] = blk[(size_t)(sg.src + sg.len)] = 1;
+            }
+    }
+    int32_t nb = 0;  // blk[r]: blocks that start before row r
+    for (int64_t r = 0; r <= ws_n; ++r) {
+        const int32_t start = blk[(size_t)r];
+        blk[(size_t)r] = nb;
+        nb += start;
+    }
+    auto first = [&](int64_t r) { return (size_t)blk[(size_t)r]; };  // the block that starts at a marked row r
+    std::vector<int32_t> last_nw((size_t)nb, -1);
+    std::vector<std::vector<int32_t>> atom((size_t)nb), rd((size_t)nb);
     std::vector<std::vector<int32_t>> prod(nt);
-    std::vector<int32_t> deps, rows_read;
+    std::vector<int32_t> deps, seen(nt, -1);
+    std::vector<size_t> read;
     for (size_t t = 0; t < nt; ++t) {
         const Target &tg = pb.T[t];
         const bool scatter = tg.flags & T_SCATTER, atomic = tg.flags & T_ATOMIC, accum = tg.flags & T_ACCUM;
         deps.clear();
-        rows_read.clear();
-        auto read_row = [&](int64_t r) {
-            if (last_nw[(size_t)r] >= 0) deps.push_back(last_nw[(size_t)r]);
-            for (int32_t a : atom[(size_t)r]) deps.push_back(a);
-            rows_read.push_back((int32_t)r);
+        read.clear();
+        seen[t] = (int32_t)t;
+        auto dep = [&](int32_t u) {
+            if (seen[(size_t)u] == (int32_t)t) return;
+            seen[(size_t)u] = (int32_t)t;
+            deps.push_back(u);
+        };
+        auto read_rows = [&](int64_t r, int64_t n) {
+            for (size_t k = first(r); k < first(r + n); ++k) {
+                if (last_nw[k] >= 0) dep(last_nw[k]);
+                for (int32_t u : atom[k]) dep(u);
+                read.push_back(k);
+            }
         };
         for (int32_t q = tg.p0; q < tg.p1; ++q) {
             const Panel &pn = pb.P[(size_t)q];
             for (int32_t e = pn.s0; e < pn.s1; ++e) {
                 const Seg &sg = pb.S[(size_t)e];
-                if (sg.flags & S_GATHER) continue;  // the input vector: no producer
-                for (int64_t r = sg.src; r < sg.src + sg.len; ++r) read_row(r);
+                if (!(sg.flags & S_GATHER)) read_rows(sg.src, sg.len);  // the input vector has no producer
             }
         }
-        if (accum)
-            for (int64_t r = tg.dst; r < tg.dst + tg.nrows; ++r) read_row(r);
-        if (!scatter)
-            for (int64_t r = tg.dst; r < tg.dst + tg.nrows; ++r) {
-                if (last_nw[(size_t)r] >= 0) deps.push_back(last_nw[(size_t)r]);
-                if (!atomic)
-                    for (int32_t a : atom[(size_t)r]) deps.push_back(a);
-                for (int32_t a : rd[(size_t)r]) deps.push_back(a);
-            }
+        if (accum) read_rows(tg.dst, tg.nrows);
+        const size_t k0 = scatter ? 0 : first(tg.dst), k1 = scatter ? 0 : first(tg.dst + tg.nrows);
+        for (size_t k = k0; k < k1; ++k) {
+            if (last_nw[k] >= 0) dep(last_nw[k]);
+            if (!atomic)
+                for (int32_t u : atom[k]) dep(u);
+            for (int32_t u : rd[k]) dep(u);
+        }
         std::sort(deps.begin(), deps.end());
-        deps.erase(std::unique(deps.begin(), deps.end()), deps.end());
-        deps.erase(std::remove(deps.begin(), deps.end(), (int32_t)t), deps.end());
         prod[t] = deps;
-        for (int32_t r : rows_read) rd[(size_t)r].push_back((int32_t)t);
-        if (!scatter)
-            for (int64_t r = tg.dst; r < tg.dst + tg.nrows; ++r) {
-                if (atomic) {
-                    atom[(size_t)r].push_back((int32_t)t);
-                } else {
-                    last_nw[(size_t)r] = (int32_t)t;
-                    atom[(size_t)r].clear();
-                    rd[(size_t)r].clear();
-                }
+        for (size_t k : read)
+            if (rd[k].empty() || rd[k].back() != (int32_t)t) rd[k].push_back((int32_t)t);
+        for (size_t k = k0; k < k1; ++k) {
+            if (atomic) {
+                atom[k].push_back((int32_t)t);
+            } else {
+                last_nw[k] = (int32_t)t;
+                atom[k].clear();
+                rd[k].clear();
             }
+        }
     }
     cnt.assign(nt, 0);
     coff.assign(nt + 1, 0);
