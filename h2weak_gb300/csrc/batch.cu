@@ -291,8 +291,6 @@ cudaError_t launch_scatter64(const double *x, double *y, const int64_t *idx, int
     return cudaGetLastError();
 }
 
-bool gms_attr(const GmresSeg &g) { return ((size_t)(g.m + 1) + 4 * GMS_WARPS) * 8 <= 48 * 1024; }
-
 cudaError_t gms_norms(const GmresSeg &g, const double *v, double *out, int zero_to_one, cudaStream_t st) {
     gms_colnorm_part<<<g.nblk, GMS_THREADS, 0, st>>>(g, v);
     gms_colnorm_fin<<<g.P, 32, 0, st>>>(g, out, zero_to_one);

@@ -183,6 +183,16 @@ __device__ __forceinline__ uint32_t sv_acquire(const void *p) {
     asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+// the group's producers are done: bounded, out of line as the waits above
+__device__ __noinline__ bool sv_until(const int32_t *rem, volatile int32_t *fail, int32_t *err) {
+    for (int it = 0; it <= SV_POLL; ++it) {
+        if ((int32_t)sv_acquire(rem) <= 0) return true;
+        if (*fail) return false;
+    }
+    *fail = 1;
+    atomicExch(err, 3);
+    return false;
+}
 
 template <class T, int CW>
 __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
@@ -363,7 +373,7 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
                                     atomicExch(a.err, 1);
                                 }
                         it = 0;
-                        while (good && !skip && (int32_t)sv_acquire(a.rem + sl.grp) > 0)
+                        while (good && !skip && !(sl.flags & SV_LATE) && (int32_t)sv_acquire(a.rem + sl.grp) > 0)
                             if (++it > SV_POLL || *fail) {
                                 good = false;
                                 atomicExch(a.err, 3);
@@ -389,7 +399,7 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
             const uint32_t pd = xd + (uint32_t)(max_w * (int)sizeof(T));
 #pragma unroll 1
             for (int i = lane; i < nrows; i += 32) {
-                if (flags & T_ACCUM) sv_cp(pd + (uint32_t)(i * (int)sizeof(T)), (const T *)a.ws + sl.dst + i);
+                if ((flags & T_ACCUM) && !(flags & SV_LATE)) sv_cp(pd + (uint32_t)(i * (int)sizeof(T)), (const T *)a.ws + sl.dst + i);
                 if ((flags & T_SCATTER) && a.perm)
                     sv_cp(pd + (uint32_t)(SV_MAX_ROWS * (int)sizeof(T) + 4 * i), a.perm + sl.vpos + i);
             }
@@ -495,6 +505,8 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
             int l = 0;
             while (l < 3 && (nrows << (l + 1)) <= CT) ++l;
             const int part = tid & ((1 << l) - 1), flags = sl.flags;
+            // the rows added to: only now does a target of input columns wait for the part before it
+            if ((flags & SV_LATE) && !__all_sync(0xffffffffu, lane != 0 || sv_until(a.rem + sl.grp, fail, a.err))) return;
 #pragma unroll 1
             for (int r0 = 0; r0 < nrows; r0 += CT >> l) {
                 if (r0 + (warp * 32 >> l) >= nrows) break;  // the same for the whole warp
@@ -508,7 +520,7 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
                 for (int o = 1; o < (1 << l); o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
                 if (part != 0 || r >= nrows) continue;
                 T *w = a.ws + sl.dst + r;
-                if (flags & T_ACCUM) sum += xs[max_w + r];
+                if (flags & T_ACCUM) sum += flags & SV_LATE ? __ldcg(w) : xs[max_w + r];
                 if (flags & T_SCATTER) {
                     const int32_t *pp = reinterpret_cast<const int32_t *>(xs + max_w + SV_MAX_ROWS);
                     a.yout[a.perm ? (int64_t)pp[r] : sl.vpos + r] = (double)sum;

@@ -17,6 +17,7 @@ from h2weak_gb300 import synth
 CASES = {
     "1d_tiny": (1, 0, 1, 10, 2, 37),
     "1d_semi": (1, 1, 0, 10, 5, 1111),
+    "1d_semi_parts": (1, 1, 1, 8, 7, 20001),  # block rows of three column parts, from the input alone
     "2d_few_points": (2, 0, 1, 8, 3, -90),
     "2d_odd": (2, 0, 0, 10, 3, 41),
     "2d_plain": (2, 2, 1, 8, 3, -1501),
