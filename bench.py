@@ -748,27 +748,28 @@ def main():
     ctype = {"fp32": "float, FP32", "df64": "double, double-FP32", "fp64": "double, FP64"}[top]
     rp = 16 if R <= 16 else (32 if R <= 32 else 64)
     # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from the ncu captures of the
-    # same launches on this workload: profiles/mw_flow_fp32_2d_ie_65536.md, mr_flow_df64_2d_ie_65536.md
-    kname = (("mw_flow_kernel" if top == "fp32" and op.get_option(hw.OPT_PRODUCER_WARP) else "mr_flow_kernel")
-             if op.get_option(hw.OPT_DATAFLOW) else "mr_coop_kernel")
-    ncu_traffic = {("mw_flow_kernel", "fp32"): 361.970e6 + 72.415e6, ("mr_flow_kernel", "df64"): 896.444e6 + 188.591e6}
+    # same launches on this workload: profiles/mw_flow_fp32_2d_ie_65536.md
+    kname = ("mr_coop_kernel" if not op.get_option(hw.OPT_DATAFLOW) else "mo_kernel" if top != "fp32" else
+             "mw_flow_kernel" if op.get_option(hw.OPT_PRODUCER_WARP) else "mr_flow_kernel")
+    ncu_traffic = {("mw_flow_kernel", "fp32"): 361.970e6 + 72.415e6}
     # the multi-vector kernel multiplies every packed operator entry by R vectors: one FMA per
-    # term (FP32), about twelve FP32 operations per term (double-FP32); nominal FP32 peak of
-    # 152 SMs x 128 lanes x 2 flop x 2.07 GHz
+    # term (FP32), about twelve FP32 operations per term (double-FP32 on the FP32 pipes); nominal FP32
+    # peak of 152 SMs x 128 lanes x 2 flop x 2.07 GHz. The tensor-core form (mo_kernel) multiplies 36
+    # pairs of digits a term, which the figures count as its one FMA.
     entries = op.operator_bytes(hw.PREC_FP32) / 4
     fp32_nominal = 152 * 128 * 2 * 2.07e9
-    ops_per_term = {"fp32": 2.0, "df64": 12.0, "fp64": 2.0}[top]
+    ops_per_term = 2.0 if kname == "mo_kernel" else {"fp32": 2.0, "df64": 12.0, "fp64": 2.0}[top]
     achieved_ops = ops_per_term * entries * R / (tk["us"] / 1e6)
     plan = op.plan_stats()
     plan["padding_overhead"] = plan["multiplied"] / plan["entries"] - 1.0 if plan["entries"] else None
     roof = {"bound": "hbm", "achieved": tk["gbs"], "peak": peak, "unit": "GB/s", "frac": tk["gbs"] / peak,
             # the captured kernel's DRAM bytes, only when that kernel is the one reported here
             "traffic": ncu_traffic.get((kname, top)) if args.workload == "2d_ie_65536" and R == 64 else None,
-            "compute": {"pipe": "fp64" if top == "fp64" else "fp32",
+            "compute": {"pipe": "tensor (digits)" if kname == "mo_kernel" else "fp64" if top == "fp64" else "fp32",
                         "ops_per_launch": ops_per_term * entries * R,
                         "achieved_tops": achieved_ops / 1e12,
                         "nominal_fp32_tops": fp32_nominal / 1e12,
-                        "frac_of_nominal": achieved_ops / fp32_nominal if top != "fp64" else None,
+                        "frac_of_nominal": achieved_ops / fp32_nominal if top != "fp64" and kname != "mo_kernel" else None,
                         "note": "each operator element feeds R FMAs: the pipe, not HBM, bounds this kernel",
                         # entries multiplied per column with the kernel's row and column padding
                         "plan": plan},

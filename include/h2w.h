@@ -53,9 +53,11 @@ enum { H2W_KERNEL_IE = 0, H2W_KERNEL_RBF = 1, H2W_KERNEL_HELMHOLTZ = 2, H2W_KERN
 enum { H2W_ASSEMBLE_NCA = 0, H2W_ASSEMBLE_IMPORT = 1, H2W_ASSEMBLE_LEARNED = 2 };
 /* FP64: FP64 operator and arithmetic. FP32: FP32 operator copy and arithmetic.
  * DF64 (multi-vector products only: h2w_matvec with nrhs > 1 and the batched
- * solvers): the FP64 operator with double-FP32 arithmetic (each operand split
- * into an FP32 pair, products and sums carried as FP32 pairs), about 2^-44
- * relative per term, on the FP32 pipes. */
+ * solvers): the FP64 operator, at least about 2^-44 relative per term. Products of many
+ * vectors in FP64 and DF64 run on the tensor cores (operands in base-256 digits, exact
+ * digit products, an FP64 result) where the operator's digits, 16 bytes an entry, fit twice into the
+ * free memory at the first such product; otherwise, and with H2W_OPT_DATAFLOW or
+ * H2W_OPT_COOP 0, FP64 on the FP64 pipe and DF64 as FP32 pairs on the FP32 pipes. */
 enum { H2W_PREC_FP64 = 0, H2W_PREC_FP32 = 1, H2W_PREC_DF64 = 2 };
 /* pointer-location flags for vectors */
 enum { H2W_HOST = 0, H2W_DEVICE = 1 };
@@ -244,7 +246,7 @@ int h2w_gmres_ir_batch(h2w_handle *h, const double *b, double *x, int nrhs, int 
  *                 their orthogonalisation in FP32 (Hessenberg, rotations and
  *                 block sums in FP64); 0: FP64 Krylov vectors.
  *  H2W_OPT_DATAFLOW  1 (default): the products (single-vector FP64 / FP32,
- *                 multi-vector FP32 / FP64 / double-FP32) run as one
+ *                 multi-vector FP32 / FP64 / double-FP32, batches) run as one
  *                 cooperative launch without grid barriers: each target waits
  *                 for the targets that produce the workspace rows it uses
  *                 (dependencies derived on the host from the rows each target
