@@ -80,11 +80,12 @@ template <class T> struct DBuf {
 struct MoStream {
     DBuf<MoHdr> hdr;
     DBuf<uint32_t> idx, cons, blist, zrow;
-    DBuf<uint2> grp;
+    DBuf<uint2> grp, plist;
     DBuf<int32_t> cnt, rem, ctr, xb, sa, mx;
-    DBuf<int64_t> s0, slices;
+    DBuf<int64_t> s0, slices, col;
     DBuf<char> img;  // made on the first product
     int64_t bytes = 0;
+    double entries = 0, chunks = 0, chain = 0;  // chunks of 32 columns; in the longest sequence of column parts
     int32_t list[3][2] = {{0, 0}, {0, 0}, {0, 0}};
     int32_t share = 0, ngrp = 0, nwb = 0, nxb = 0, nzrow = 0;
     bool fused = true, ready = false, refused = false;
@@ -1788,12 +1789,14 @@ struct SvHost {
     std::vector<int32_t> cnt;
     std::vector<int64_t> slices;  // operator pieces to copy (slice_records)
     std::vector<int64_t> s0;      // the slices of each target
-    // the tensor-core form (mo.cu): source block lists and blocks of the written rows per
-    // target, block starts (the workspace's, then the input's), rows nobody writes
-    std::vector<uint32_t> blist, bl0, ob0, zrow;
-    std::vector<uint16_t> nbl, nob;
+    // the tensor-core form (mo.cu): source block lists of each part of a target's columns, its first
+    // part, blocks of its written rows, block starts (the workspace's, then the input's), rows nobody writes
+    std::vector<uint32_t> blist, p0, ob0, zrow;
+    std::vector<uint2> plist;
+    std::vector<uint16_t> nob;
     std::vector<int64_t> blocks;
     int32_t nwb = 0;
+    double chain = 0;  // chunks of 32 columns in the longest sequence of column parts
     int64_t opn = 0;
     int max_w = 1;
     bool fused = true;  // the leaf pass writes the result itself
@@ -1867,7 +1870,7 @@ void group_deps(const std::vector<const PlanBuilder::LTarget *> &groups, const s
 constexpr int SV_CUT_CTAS = 608;
 constexpr int64_t SV_CUT_MIN = 2048;
 // tiles: the tensor-core form's cut, tiles of 64 rows and at most MO_XW columns.
-constexpr int64_t MO_XW = 2048;
+constexpr int64_t MO_XW = MO_MAX_W;
 void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t ws0, int64_t x0, int64_t xoff, SvHost &out,
               bool tiles = false) {
     auto bad = [](const char *what) { throw ApiError(H2W_ERR_STATE, std::string("internal: single-vector stream: ") + what); };
@@ -1905,6 +1908,7 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
             for (const auto &p : l.panels)
                 for (const Seg &sg : p.segs)
                     if (!(sg.flags & S_GATHER)) bad("a free target reads the workspace");
+        out.chain = std::max(out.chain, (double)(xw + 31) / 32);
         if (xw <= pb.xw_cap) {
             groups.push_back(&l);
             key.push_back({ls, l.hi, 0, w, 0});
@@ -2005,8 +2009,8 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
     // headers; targets of a group that read the same sources share the list of rows.
     // Every value the kernel indexes with is checked against its field.
     std::vector<uint32_t> rows, prev;
-    uint32_t prev0 = 0, blist0 = 0;
-    uint16_t nblist = 0;
+    uint32_t prev0 = 0;
+    std::vector<uint2> lists;  // of the targets' parts with these sources
     for (size_t t = 0; t + 1 < roff.size(); ++t) {
         const size_t o = (size_t)roff[t];
         const int64_t nrows = blob[o + 1] & 0xffffffff, fl = blob[o + 1] >> 32;
@@ -2042,13 +2046,16 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
         out.s0.push_back(out.s0.back() + np);
         if (rows != prev) {
             if (tiles) {
-                const size_t b0 = out.blist.size();
-                for (uint32_t r : rows)
-                    if (out.blist.size() == b0 || out.blist.back() != block[r]) out.blist.push_back(block[r]);
-                std::sort(out.blist.begin() + (long)b0, out.blist.end());
-                out.blist.erase(std::unique(out.blist.begin() + (long)b0, out.blist.end()), out.blist.end());
-                blist0 = (uint32_t)b0;
-                nblist = (uint16_t)(out.blist.size() - b0);
+                lists.clear();
+                for (size_t r0 = 0; r0 < rows.size(); r0 += (size_t)mo_part_columns()) {
+                    const size_t b0 = out.blist.size(), r1 = std::min(rows.size(), r0 + (size_t)mo_part_columns());
+                    for (size_t r = r0; r < r1; ++r)
+                        if (out.blist.size() == b0 || out.blist.back() != block[rows[r]]) out.blist.push_back(block[rows[r]]);
+                    std::sort(out.blist.begin() + (long)b0, out.blist.end());
+                    out.blist.erase(std::unique(out.blist.begin() + (long)b0, out.blist.end()), out.blist.end());
+                    lists.push_back(make_uint2((uint32_t)b0, (uint32_t)(out.blist.size() - b0)));
+                }
+                if (out.blist.size() > (size_t)UINT32_MAX) bad("too many source blocks");
             }
             prev0 = (uint32_t)out.idx.size();
             if (out.idx.size() + rows.size() > (size_t)UINT32_MAX) bad("too many sources");
@@ -2058,8 +2065,8 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
         d.idx0 = prev0;
         d.W = (uint16_t)W;
         if (tiles) {
-            out.bl0.push_back(blist0);
-            out.nbl.push_back(nblist);
+            out.p0.push_back((uint32_t)out.plist.size());
+            out.plist.insert(out.plist.end(), lists.begin(), lists.end());
             out.ob0.push_back(block[d.dst]);
             out.nob.push_back((uint16_t)(block[d.dst + (uint32_t)nrows - 1] - block[d.dst] + 1));
         }
@@ -2136,20 +2143,24 @@ void mo_upload(const SvHost &v, MoStream &d, cudaStream_t st) {
     for (int l = 0; l < 3; ++l) d.list[l][0] = d.list[l][1] = 0;
     double work[3] = {0, 0, 0};
     d.bytes = 0;
+    d.entries = d.chunks = 0;
+    d.chain = v.chain;
     for (size_t t = 0; t < hdr.size(); ++t) {
         const SvHdr &s = v.hdr[t];
         MoHdr &h = hdr[t];
+        if (s.W > MO_MAX_W || s.nrows > MR_ROWS) throw ApiError(H2W_ERR_STATE, "internal: tensor-core target out of range");
         h.img = d.bytes;
         d.bytes += mo_image_bytes(s.nrows, s.W);
+        d.entries += (double)s.nrows * s.W;
+        d.chunks += (s.W + 31) / 32;
         h.dst = s.dst;
         h.idx0 = s.idx0;
         h.grp = s.grp;
-        h.bl0 = v.bl0[t];
         h.ob0 = v.ob0[t];
+        h.p0 = v.p0[t];
         h.nrows = s.nrows;
         h.W = s.W;
         h.flags = s.flags;
-        h.nbl = v.nbl[t];
         h.nob = v.nob[t];
         ++d.list[v.list[t]][1];
         work[v.list[t]] += (double)s.nrows * s.W;
@@ -2172,6 +2183,7 @@ void mo_upload(const SvHost &v, MoStream &d, cudaStream_t st) {
     d.blist.upload(v.blist, st);
     d.zrow.upload(v.zrow, st);
     d.grp.upload(v.grp, st);
+    d.plist.upload(v.plist, st);
     d.cnt.upload(v.cnt, st);
     d.xb.upload(xb, st);
     d.s0.upload(v.s0, st);
@@ -3324,10 +3336,11 @@ bool ensure_mo(h2w_handle *h) {
     if (d.refused) return false;
     cudaStream_t st = h->stream;
     d.img.alloc((size_t)d.bytes);
-    d.sa.alloc(d.hdr.n * 64);
+    d.sa.alloc(d.plist.n * 64);
+    d.col.alloc(d.plist.n * (size_t)mo_part_columns());
     d.mx.alloc((size_t)(d.nwb + d.nxb) * MR_MAX);
     CK(cudaMemsetAsync(d.mx.p, 0, 4, st));  // the first word reports a bad entry
-    CK(launch_mo_image(d.hdr.p, d.list[2][1], d.s0.p, d.slices.p, h->d_op.p, d.img.p, d.sa.p, d.mx.p, st));
+    CK(launch_mo_image(d.hdr.p, d.list[2][1], d.s0.p, d.slices.p, h->d_op.p, d.img.p, d.sa.p, d.col.p, d.mx.p, st));
     int32_t bad = 0;
     CK(cudaMemcpyAsync(&bad, d.mx.p, 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
@@ -3340,7 +3353,21 @@ bool ensure_mo(h2w_handle *h) {
     return true;
 }
 
-MoArgs mo_args(h2w_handle *h, int rp, const double *xi, double *yi) {
+// Whether the tensor-core form is the faster one, by times in us fitted to products of operators of
+// 1e6 to 9e7 entries in 1D, 2D and 3D. It takes groups of 16 vectors one after another, each a chunk of 32
+// columns an SM at a time, 7 us a dependent pass, and the column parts of a block row in sequence; the
+// FP32 pairs 1.74e6 entries and vectors a us and 19 a pass for all vectors at once, FP64 multiply-adds a third
+// of that and 30. So FP32 pairs stay where passes or a long row rule: 64 vectors, 1D, 16384 points on 8
+// levels 394 us (650 on the tensor cores), 1D semi-nested, rows of 16384 columns, 820 (1670); 2D, 65536
+// points 2280 (1440).
+bool mo_pays(const h2w_handle *h, int prec, int rp, int nrhs) {
+    const MoStream &d = h->mo;
+    const double passes = h->nph_total, terms = d.entries * rp;
+    const double mo = (nrhs + 15) / 16 * (std::max(d.chunks / 152.0, 0.8 * d.chain) + 7.0 * passes);
+    return mo < (prec == H2W_PREC_DF64 ? terms / 1.74e6 + 19.0 * passes : terms / 0.576e6 + 30.0 * passes);
+}
+
+MoArgs mo_args(h2w_handle *h, int prec, int rp, int nrhs, const double *xi, double *yi) {
     MoStream &d = h->mo;
     MoArgs a{};
     a.hdr = d.hdr.p;
@@ -3352,6 +3379,9 @@ MoArgs mo_args(h2w_handle *h, int rp, const double *xi, double *yi) {
     a.sa = d.sa.p;
     a.xb = d.xb.p;
     a.img = d.img.p;
+    a.op = h->d_op.p;
+    a.col = d.col.p;
+    a.plist = d.plist.p;
     for (int l = 0; l < 3; ++l) {
         a.l0[l] = d.list[l][0];
         a.l1[l] = d.list[l][1];
@@ -3363,6 +3393,8 @@ MoArgs mo_args(h2w_handle *h, int rp, const double *xi, double *yi) {
     a.nzrow = d.nzrow;
     a.xoff = (uint32_t)h->xoff();
     a.ld = rp;
+    a.ncg = (nrhs + 15) / 16;
+    a.guard = prec == H2W_PREC_DF64 ? 28 : 20;
     a.rows = h->xoff() + h->nv();
     a.mx = d.mx.p;
     a.ws = h->m_wsd.p;
@@ -3376,8 +3408,9 @@ MoArgs mo_args(h2w_handle *h, int rp, const double *xi, double *yi) {
     return a;
 }
 
-// Y = A X for an interleaved leaf-order block of rp vectors (xi, yi: N x rp).
-void run_matvec_multi(h2w_handle *h, int prec, int rp, const double *xi, double *yi, cudaStream_t st) {
+// Y = A X for an interleaved leaf-order block of rp vectors (xi, yi: N x rp), nrhs of
+// them in use and the others zero.
+void run_matvec_multi(h2w_handle *h, int prec, int rp, int nrhs, const double *xi, double *yi, cudaStream_t st) {
     if (h->fly_active)
         throw ApiError(H2W_ERR_STATE, "multi-vector products need the stored far field (H2W_OPT_FAR_ON_THE_FLY is on)");
     const int nph = (int)h->mphases.size();
@@ -3414,10 +3447,10 @@ void run_matvec_multi(h2w_handle *h, int prec, int rp, const double *xi, double 
         });
         if (!h->fused_scatter_m) CK(launch_mr_widen_f32(h->m_wsf.p + (size_t)h->yperm_off * rp, yi, h->tree.N * rp, st));
     } else {
-        if (h->dataflow && h->coop && ensure_mo(h)) {
+        if (h->dataflow && h->coop && mo_pays(h, prec, rp, nrhs) && ensure_mo(h)) {
             const size_t need = (size_t)(h->xoff() + h->nv()) * (size_t)rp;
             if (h->m_wsd.n < need) h->m_wsd.alloc(need);
-            const MoArgs a = mo_args(h, rp, xi, yi);
+            const MoArgs a = mo_args(h, prec, rp, nrhs, xi, yi);
             mr_prof(h, prec, rp, st, [&] { return launch_mo(a, st); });
             if (!h->mo.fused) CK(launch_mo_unplane(a, h->yperm_off, h->tree.N, yi, st));
             return;
@@ -3561,7 +3594,7 @@ int gmres_batch_run_t(h2w_handle *h, const double *bi, double *xi, int rp, int n
     // w = A vcur: the FP32 basis feeds the FP32 product directly (no conversions)
     auto product = [&](cudaStream_t s) {
         if constexpr (F32) run_matvec_multi_f32io(h, rp, g.vcur, g.w, s);
-        else run_matvec_multi(h, prec, rp, g.vcur, g.w, s);
+        else run_matvec_multi(h, prec, rp, nrhs, g.vcur, g.w, s);
     };
     const int kind = F32 ? 2 : 1;
     cudaStream_t st = h->stream;
@@ -3572,7 +3605,7 @@ int gmres_batch_run_t(h2w_handle *h, const double *bi, double *xi, int rp, int n
         if (F32) throw ApiError(H2W_ERR_ARG, "batched GMRES: the FP32 basis starts from x0 = 0");
         CK(gmb_norms(g, bi, g.normb, 1, st));
         if (h->m_ri.n < (size_t)h->tree.N * rp) h->m_ri.alloc((size_t)h->tree.N * MR_MAX);
-        run_matvec_multi(h, prec, rp, xi, h->m_ri.p, st);
+        run_matvec_multi(h, prec, rp, nrhs, xi, h->m_ri.p, st);
         CK(gmb_start(g, bi, h->m_ri.p, tol, st));
     }
     std::vector<int32_t> conv((size_t)rp);
@@ -3757,8 +3790,8 @@ double fp32_error_multi(h2w_handle *h, const GmbT<T> &g, int rp, cudaStream_t st
     if (h->m_dn.n < (size_t)2 * MR_MAX) h->m_dn.alloc((size_t)2 * MR_MAX);
     double *z = h->m_di.p, *y32 = h->m_ri.p, *y = h->m_ti.p;
     CK(launch_calib_fill(z, N, rp, 0, st));
-    run_matvec_multi(h, H2W_PREC_FP32, rp, z, y32, st);
-    run_matvec_multi(h, h->ir_resid_prec, rp, z, y, st);
+    run_matvec_multi(h, H2W_PREC_FP32, rp, rp, z, y32, st);
+    run_matvec_multi(h, h->ir_resid_prec, rp, rp, z, y, st);
     CK(vec_axpby(1.0, y32, -1.0, y, y32, (int64_t)len, st));
     CK(gmb_norms(g, y32, h->m_dn.p, 0, st));
     CK(gmb_norms(g, z, h->m_dn.p + MR_MAX, 0, st));
@@ -4894,7 +4927,7 @@ int h2w_matvec(h2w_handle *h, const double *x, double *y, int nrhs, int precisio
                 } else {
                     ensure_multi_vectors(h);
                     CK(launch_mr_pack(xc, N, h->m_xi.p, h->d_perm.p, N, nc, rp, st));
-                    run_matvec_multi(h, precision, rp, h->m_xi.p, h->m_yi.p, st);
+                    run_matvec_multi(h, precision, rp, nc, h->m_xi.p, h->m_yi.p, st);
                     CK(launch_mr_unpack(h->m_yi.p, out, N, h->d_perm.p, N, nc, rp, st));
                 }
                 if (where == H2W_HOST)
@@ -5139,13 +5172,13 @@ int h2w_gmres_ir_batch(h2w_handle *h, const double *b, double *x, int nrhs, int 
                     for (int c = 0; c < nc; ++c)
                         drift[(size_t)c] += IR_UPDATE_SAFETY * IR_UPDATE_ARNOLDI * eta * nd[(size_t)c];
                 } else if (upd) {
-                    run_matvec_multi(h, H2W_PREC_FP32, rp, h->m_di.p, h->m_ti.p, st);
+                    run_matvec_multi(h, H2W_PREC_FP32, rp, nc, h->m_di.p, h->m_ti.p, st);
                     CK(vec_axpby(1.0, h->m_ri.p, -1.0, h->m_ti.p, h->m_ri.p, (int64_t)len, st));
                     for (int c = 0; c < nc; ++c) drift[(size_t)c] += IR_UPDATE_SAFETY * eta * nd[(size_t)c];
                 } else if (o == 0 && x0_zero) {
                     CK(cudaMemcpyAsync(h->m_ri.p, bi, len * 8, cudaMemcpyDeviceToDevice, st));
                 } else {
-                    run_matvec_multi(h, o == 0 ? H2W_PREC_FP32 : h->ir_resid_prec, rp, xi, h->m_ri.p, st);
+                    run_matvec_multi(h, o == 0 ? H2W_PREC_FP32 : h->ir_resid_prec, rp, nc, xi, h->m_ri.p, st);
                     CK(vec_axpby(1.0, bi, -1.0, h->m_ri.p, h->m_ri.p, (int64_t)len, st));
                     std::fill(drift.begin(), drift.end(), o == 0 ? HUGE_VAL : 0.0);
                     if (o == 1 && h->ir_update) {
@@ -5329,9 +5362,9 @@ int h2w_autotune(h2w_handle *h, int nrhs, int precision, int reps, int64_t *chos
                 else realize_single(h, c);
                 auto once = [&] {
                     if (mix) {  // the batched refinement's mix: four FP32 products per DF64 residual
-                        for (int q = 0; q < 4; ++q) run_matvec_multi(h, H2W_PREC_FP32, rp, h->m_xi.p, h->m_yi.p, st);
-                        run_matvec_multi(h, H2W_PREC_DF64, rp, h->m_xi.p, h->m_yi.p, st);
-                    } else if (multi) run_matvec_multi(h, precision, rp, h->m_xi.p, h->m_yi.p, st);
+                        for (int q = 0; q < 4; ++q) run_matvec_multi(h, H2W_PREC_FP32, rp, rp, h->m_xi.p, h->m_yi.p, st);
+                        run_matvec_multi(h, H2W_PREC_DF64, rp, rp, h->m_xi.p, h->m_yi.p, st);
+                    } else if (multi) run_matvec_multi(h, precision, rp, rp, h->m_xi.p, h->m_yi.p, st);
                     else if (precision == H2W_PREC_FP32) run_matvec_f32(h, h->d_x.p, h->d_y.p, st, true);
                     else run_matvec_f64(h, h->d_x.p, h->d_y.p, st, true);
                 };

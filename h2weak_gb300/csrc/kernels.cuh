@@ -386,29 +386,34 @@ cudaError_t launch_mr_f64_flow(int rp, bool df, const int64_t *roff, const int64
                                int32_t *rem, const int64_t *coff, const int32_t *cidx, const double *A, double *ws,
                                const double *xin, double *yout, int32_t *err, cudaStream_t st);
 // FP64 product of many vectors on the tensor cores (mo.cu): the dataflow stream of
-// 64-row targets, A as digits in the MMA's layout (img + hdr.img), a scale for each row
-// (sa, 64 a target). Rows are numbered as in SvArgs ([0, xoff) the workspace, then
-// the input), in blocks that no target reads or writes a part of: blist the blocks of a
-// target's sources, ob0 .. ob0 + nob those of its rows; mx (blocks x ld) the largest
+// 64-row targets of at most MO_MAX_W columns, in parts of mo_part_columns() (a target's from p0 on): A as
+// digits in the MMA's layout (img + hdr.img), a scale for each row in each part (sa, 64 a part), the
+// addresses in op of a part's columns (col). Rows are numbered as in SvArgs ([0, xoff) the workspace, then
+// the input), in blocks that no target reads or writes a part of: plist the blocks of a
+// part's sources (start and count in blist), ob0 .. ob0 + nob those of its rows; mx (blocks x ld) the largest
 // magnitude of each column of a block (high words), workspace blocks [0, nwb), then the
 // nxb input blocks with rows xb[b] .. xb[b + 1). zrow: workspace rows that are read but
-// never written (zero). ld = 16, 32 or 64 vectors; the input and the result interleaved as
-// in launch_mr_f64_flow, the workspace in planes of 16 (ld 16) or 32 columns, rows (=
-// xoff + N) x 16 or 32 each, which hold the input from row xoff.
+// never written (zero). ld = 16, 32 or 64 vectors, of which the first ncg groups of 16 are
+// multiplied and the others are zero; the input and the result interleaved as in launch_mr_f64_flow, the
+// workspace in planes of 16 columns, rows (= xoff + N) x 16 each, which hold the input from row xoff. Results of
+// a part below 2^-guard of its largest entry times its largest source are formed by multiply-adds.
 struct alignas(8) MoHdr {
     int64_t img;
-    uint32_t dst, idx0, grp, bl0, ob0;
-    uint16_t nrows, W, flags, nbl, nob, pad;
+    uint32_t dst, idx0, grp, ob0, p0;
+    uint16_t nrows, W, flags, nob;
 };
+constexpr int MO_MAX_W = 2048;  // columns of a target
 struct MoArgs {
     const MoHdr *hdr;
     const uint32_t *idx, *cons, *blist, *zrow;
-    const uint2 *grp;
+    const uint2 *grp, *plist;
     const int32_t *sa, *xb;
     const char *img;
+    const double *op;
+    const int64_t *col;
     int32_t l0[3], l1[3], na, ngrp, nwb, nxb, nzrow;
     uint32_t xoff;
-    int32_t ld;
+    int32_t ld, ncg, guard;
     int64_t rows;
     int32_t *mx;
     double *ws;
@@ -420,9 +425,10 @@ struct MoArgs {
     int32_t *err;
 };
 int64_t mo_image_bytes(int nrows, int W);
+int mo_part_columns();
 // s0: the slices (as launch_slice_copy_f32) of each target; *bad set if an entry is not finite
 cudaError_t launch_mo_image(const MoHdr *hdr, int64_t nt, const int64_t *s0, const int64_t *slices, const double *op,
-                            char *img, int32_t *sa, int32_t *bad, cudaStream_t st);
+                            char *img, int32_t *sa, int64_t *col, int32_t *bad, cudaStream_t st);
 cudaError_t launch_mo(const MoArgs &a, cudaStream_t st);
 // the first n rows of the workspace planes as an interleaved block
 cudaError_t launch_mo_unplane(const MoArgs &a, int64_t r0, int64_t n, double *y, cudaStream_t st);

@@ -55,7 +55,8 @@ enum { H2W_ASSEMBLE_NCA = 0, H2W_ASSEMBLE_IMPORT = 1, H2W_ASSEMBLE_LEARNED = 2 }
  * DF64 (multi-vector products only: h2w_matvec with nrhs > 1 and the batched
  * solvers): the FP64 operator, at least about 2^-44 relative per term. Products of many
  * vectors in FP64 and DF64 run on the tensor cores (operands in base-256 digits, exact
- * digit products, an FP64 result) where the operator's digits, 16 bytes an entry, fit twice into the
+ * digit products, multiply-adds where the digits would hold less than FP64, or DF64, of a row's own
+ * terms) where that is the faster form and the operator's digits, 20 bytes an entry, fit twice into the
  * free memory at the first such product; otherwise, and with H2W_OPT_DATAFLOW or
  * H2W_OPT_COOP 0, FP64 on the FP64 pipe and DF64 as FP32 pairs on the FP32 pipes. */
 enum { H2W_PREC_FP64 = 0, H2W_PREC_FP32 = 1, H2W_PREC_DF64 = 2 };
