@@ -433,25 +433,18 @@ __global__ void __launch_bounds__(BRG_THREADS, 4)
     }
 }
 
-static int g_num_sms = 0;
-
 template <class T>
 static cudaError_t launch_brg_t(const int64_t *roff, const int64_t *blob, int64_t t0, int64_t t1, const T *A, T *ws,
                                 const double *xin, double *yout, const int32_t *perm, cudaStream_t st) {
     if (t1 <= t0) return cudaSuccess;
-    static int per_sm = 0;
-    if (g_num_sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-        if (g_num_sms <= 0) g_num_sms = 1;
-    }
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
     if (per_sm == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, brg_kernel<T>, BRG_THREADS, 0);
         if (per_sm <= 0) per_sm = 1;
     }
     const int64_t nt = t1 - t0;
-    const int64_t cap = (int64_t)g_num_sms * per_sm;
+    const int64_t cap = (int64_t)device_sms() * per_sm;
     const int grid = (int)(nt < cap ? nt : cap);
     brg_kernel<T><<<grid, BRG_THREADS, 0, st>>>(roff, blob, t0, t1, A, ws, xin, yout, perm);
     count_launch();
@@ -464,18 +457,13 @@ static cudaError_t launch_coop_t(const int64_t *roff, const int64_t *blob, const
                                  unsigned *bar, int32_t *err, long long spin, cudaStream_t st) {
     if (nphase <= 0) return cudaSuccess;
     if (spin <= 0) spin = GRID_SPIN_LIMIT;
-    static int per_sm = 0;
-    if (g_num_sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-        if (g_num_sms <= 0) g_num_sms = 1;
-    }
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
     if (per_sm == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, brg_coop_kernel<T>, BRG_THREADS, 0);
         if (per_sm <= 0) return cudaErrorCooperativeLaunchTooLarge;
     }
-    const int grid = g_num_sms * per_sm;
+    const int grid = device_sms() * per_sm;
     void *args[] = {(void *)&roff, (void *)&blob, (void *)&pstart, (void *)&nphase, (void *)&A, (void *)&ws,
                     (void *)&xin, (void *)&yout, (void *)&perm, (void *)&bar, (void *)&err, (void *)&spin};
     cudaError_t e = cudaLaunchCooperativeKernel((const void *)brg_coop_kernel<T>, dim3(grid), dim3(BRG_THREADS), args,
@@ -500,18 +488,13 @@ static cudaError_t launch_brgb_t(const int64_t *roff, const int64_t *blob, const
                                  const BatchProb *probs, const int32_t *active, const double *xin, double *yout,
                                  unsigned *bar, int32_t *err, cudaStream_t st) {
     if (nphase <= 0) return cudaSuccess;
-    static int per_sm = 0;
-    if (g_num_sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-        if (g_num_sms <= 0) g_num_sms = 1;
-    }
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
     if (per_sm == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, brgb_coop_kernel<T>, BRG_THREADS, 0);
         if (per_sm <= 0) return cudaErrorCooperativeLaunchTooLarge;
     }
-    const int grid = g_num_sms * per_sm;
+    const int grid = device_sms() * per_sm;
     void *args[] = {(void *)&roff, (void *)&blob, (void *)&pstart, (void *)&nphase, (void *)&probs,
                     (void *)&active, (void *)&xin, (void *)&yout,  (void *)&bar,    (void *)&err};
     cudaError_t e = cudaLaunchCooperativeKernel((const void *)brgb_coop_kernel<T>, dim3(grid), dim3(BRG_THREADS), args,
@@ -786,7 +769,8 @@ int gmres_blocks(int64_t N) {
 // One-time function attributes of the Arnoldi kernels (done before any
 // stream capture of an Arnoldi step).
 void gmres_prepare() {
-    static bool cfg = false;
+    static PerDevice<bool> cfg_of;
+    bool &cfg = cfg_of.here();
     if (!cfg) {
         cudaFuncSetAttribute(gm_step, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         cudaFuncSetAttribute(gm_backsub, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);

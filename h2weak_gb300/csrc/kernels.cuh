@@ -8,6 +8,31 @@
 
 namespace h2w {
 
+// What a launcher remembers of a device (function attributes and occupancy belong to a device, and
+// handles of several devices may share a process): here() is the current device's entry, at first
+// zero. Beyond MAX devices nothing is remembered.
+template <class T> struct PerDevice {
+    static constexpr int MAX = 64;
+    T v[MAX + 1] = {};
+    T &here() {
+        int d = -1;
+        if (cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < MAX) return v[d];
+        return v[MAX] = T();
+    }
+};
+// Streaming multiprocessors of the current device
+inline int device_sms() {
+    static PerDevice<int> sms;
+    int &n = sms.here();
+    if (n == 0) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (n <= 0) n = 1;
+    }
+    return n;
+}
+
 // Number of kernel launches issued by this library (all kernels).
 int64_t launch_count();
 void count_launch(int64_t n = 1);

@@ -184,7 +184,8 @@ __global__ void __launch_bounds__(LT) mlp_forward_kernel(const float *__restrict
 
 cudaError_t launch_mlp_forward(const float *params, const float *X, int64_t n, float *logits, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    static bool attr = false;
+    static PerDevice<bool> attr_of;
+    bool &attr = attr_of.here();
     if (!attr) {
         cudaError_t e = cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(MlpSmem));
@@ -307,7 +308,8 @@ __global__ void __launch_bounds__(LT) mlp_grad_kernel(const float *__restrict__ 
 cudaError_t launch_mlp_grad(const float *params, const float *X, const uint8_t *y, int64_t n, float pos_weight,
                             float *grads, float *loss, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    static bool attr = false;
+    static PerDevice<bool> attr_of;
+    bool &attr = attr_of.here();
     if (!attr) {
         cudaError_t e = cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)sizeof(MlpGradSmem));
@@ -409,7 +411,8 @@ __global__ void __launch_bounds__(LT)
 cudaError_t launch_learn_propose(const LearnProb *probs, int nprob, const float *logits, float calib, int margin,
                                  int32_t *prop_r, int32_t *prop_c, LearnState *lst, int mask_words, cudaStream_t st) {
     const size_t sm = (size_t)mask_words * 4;
-    static size_t set = 0;
+    static PerDevice<size_t> set_of;
+    size_t &set = set_of.here();
     if (sm > 48 * 1024 && sm > set) {
         cudaError_t e = cudaFuncSetAttribute(learn_propose_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
@@ -615,7 +618,8 @@ __global__ void __launch_bounds__(LT)
 cudaError_t launch_learn_aca(const LearnProb *probs, int nprob, double tol, double *scr, int32_t *ordI,
                              int32_t *ordJ, LearnState *lst, int mask_words, cudaStream_t st) {
     const size_t sm = (size_t)mask_words * 4;
-    static size_t set = 0;
+    static PerDevice<size_t> set_of;
+    size_t &set = set_of.here();
     if (sm > 48 * 1024 && sm > set) {
         cudaError_t e = cudaFuncSetAttribute(learn_aca_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;
@@ -890,7 +894,8 @@ cudaError_t launch_learn_test(const LearnProb *probs, int nprob, const int32_t *
                               LearnState *lst, double *scr, int32_t *prow, int32_t *pcol, int mask_words,
                               cudaStream_t st) {
     const size_t sm = (size_t)mask_words * 4;
-    static size_t set = 0;
+    static PerDevice<size_t> set_of;
+    size_t &set = set_of.here();
     if (sm > 48 * 1024 && sm > set) {
         cudaError_t e = cudaFuncSetAttribute(learn_test_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         if (e != cudaSuccess) return e;

@@ -384,27 +384,17 @@ __global__ void __launch_bounds__(FLY_THREADS)
     }
 }
 
-static int fly_sms() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 template <class T, int DIM, int CH>
 static cudaError_t fly_launch_t(const FlyItem *items, int64_t nitems, unsigned long long *ctr, const int32_t *rowpid,
                                 const int32_t *cpid, const int32_t *cws, const T *pts, T *ws, const KParams &kp,
                                 const FlyK32 &k32, cudaStream_t st) {
-    static int per_sm = 0;
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
     if (per_sm == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m2l_fly_kernel<T, DIM, CH>, FLY_THREADS, 0);
         if (per_sm <= 0) per_sm = 1;
     }
-    const int64_t cap = (int64_t)fly_sms() * per_sm;
+    const int64_t cap = (int64_t)device_sms() * per_sm;
     const int grid = (int)(nitems < cap ? nitems : cap);
     cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
@@ -436,12 +426,13 @@ template <int DIM, int CH>
 static cudaError_t fly32_sep_launch(const FlyItem *items, int64_t nitems, unsigned long long *ctr,
                                     const int32_t *rowpid, const int32_t *cpid, const int32_t *cws, const float *pts4,
                                     float *ws, float scale, cudaStream_t st) {
-    static int per_sm = 0;
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
     if (per_sm == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m2l_fly32_sep_kernel<DIM, CH>, FLY_THREADS, 0);
         if (per_sm <= 0) per_sm = 1;
     }
-    const int64_t cap = (int64_t)fly_sms() * per_sm;
+    const int64_t cap = (int64_t)device_sms() * per_sm;
     const int grid = (int)(nitems < cap ? nitems : cap);
     cudaError_t e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
@@ -480,7 +471,7 @@ static cudaError_t flydf_launch(const FlyItem *items, int64_t nitems, unsigned l
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, m2l_flydf_kernel<DIM>, FLY_THREADS, smem);
     if (e != cudaSuccess) return e;
-    const int64_t cap = (int64_t)fly_sms() * std::max(per_sm, 1);
+    const int64_t cap = (int64_t)device_sms() * std::max(per_sm, 1);
     const int grid = (int)(nitems < cap ? nitems : cap);
     e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
@@ -549,7 +540,7 @@ __global__ void ptsdf_kernel(const double *__restrict__ pts, int dim, int64_t n,
 }
 
 cudaError_t launch_ptsdf(const double *pts, int dim, int64_t n, float *out, cudaStream_t st) {
-    ptsdf_kernel<<<fly_sms() * 4, 256, 0, st>>>(pts, dim, n, out);
+    ptsdf_kernel<<<device_sms() * 4, 256, 0, st>>>(pts, dim, n, out);
     count_launch();
     return cudaGetLastError();
 }
@@ -564,7 +555,7 @@ __global__ void pts4_kernel(const double *__restrict__ pts, int dim, int64_t n, 
 }
 
 cudaError_t launch_pts4(const double *pts, int dim, int64_t n, float *out, cudaStream_t st) {
-    pts4_kernel<<<fly_sms() * 4, 256, 0, st>>>(pts, dim, n, out);
+    pts4_kernel<<<device_sms() * 4, 256, 0, st>>>(pts, dim, n, out);
     count_launch();
     return cudaGetLastError();
 }

@@ -919,11 +919,12 @@ __global__ void mo_image_kernel(const MoHdr *__restrict__ hdr, const int64_t *__
 
 cudaError_t mo_launch(const MoArgs &args, cudaStream_t st) {
     using L = MoLay;
-    int dev = 0, sms = 0;  // attributes belong to the device, so both are set and asked for at every call
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(mo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::smem);
+    static PerDevice<bool> attr_of;
+    bool &attr = attr_of.here();
+    cudaError_t e = attr ? cudaSuccess : cudaFuncSetAttribute(mo_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::smem);
     if (e != cudaSuccess) return e;
+    attr = true;
+    const int sms = device_sms();
     int64_t n[3];
     for (int l = 0; l < 3; ++l) n[l] = args.l1[l] - args.l0[l];
     const int64_t want = std::max<int64_t>(n[0] + n[1] + n[2], 1);

@@ -410,24 +410,17 @@ __global__ void __launch_bounds__(TC_NT, 1)
     tc_teardown<RP>(tmem);
 }
 
-int tc_num_sms() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 template <int RP, class YT>
 cudaError_t mrt_launch(const int64_t *roff, const int64_t *blob, const int64_t *pstart, int nphase,
                        const MrPhases *phased, int32_t *ctr, const float *A, float *ws, const float *xin, YT *yout,
                        unsigned *bar, int32_t *err, cudaStream_t st) {
     using L = TcLayout<RP>;
-    static int per_sm_coop = 0, per_sm = 0;
-    static bool attr = false;
+    static PerDevice<int> per_sm_coop_of;
+    int &per_sm_coop = per_sm_coop_of.here();
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
+    static PerDevice<bool> attr_of;
+    bool &attr = attr_of.here();
     if (!attr) {
         cudaError_t e = cudaFuncSetAttribute(mrt_coop_kernel<RP, YT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::smem);
         if (e != cudaSuccess) return e;
@@ -438,7 +431,7 @@ cudaError_t mrt_launch(const int64_t *roff, const int64_t *blob, const int64_t *
         cudaFuncSetAttribute(mrt_kernel<RP, YT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         attr = true;
     }
-    const int nsm = tc_num_sms();
+    const int nsm = device_sms();
     if (phased) {
         if (per_sm == 0) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mrt_kernel<RP, YT>, TC_NT, L::smem);

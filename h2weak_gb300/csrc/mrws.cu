@@ -408,23 +408,13 @@ __global__ void __launch_bounds__(MwLayout<RP>::NT, 3)
     else mw_consume<RP, YT>(mw_smem, coff, cidx, rem, ws, yout, err);
 }
 
-int mw_num_sms() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 template <int RP, class YT>
 cudaError_t mw_launch(const int64_t *roff, const int64_t *blob, int64_t nt, int32_t *ctr, int32_t *rem,
                       const int64_t *coff, const int32_t *cidx, const float *A, float *ws, const float *xin, YT *yout,
                       int32_t *err, cudaStream_t st) {
     using Lay = MwLayout<RP>;
-    static int per_sm = 0;
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
     if (per_sm == 0) {
         if (cudaFuncSetAttribute(mw_flow_kernel<RP, YT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)Lay::smem) != cudaSuccess)
@@ -432,7 +422,7 @@ cudaError_t mw_launch(const int64_t *roff, const int64_t *blob, int64_t nt, int3
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mw_flow_kernel<RP, YT>, Lay::NT, Lay::smem);
         if (per_sm <= 0) return cudaErrorCooperativeLaunchTooLarge;
     }
-    const int grid = mw_num_sms() * per_sm;
+    const int grid = device_sms() * per_sm;
     void *args[] = {(void *)&roff, (void *)&blob, (void *)&nt, (void *)&ctr, (void *)&rem, (void *)&coff,
                     (void *)&cidx, (void *)&A, (void *)&ws, (void *)&xin, (void *)&yout, (void *)&err};
     cudaError_t e = cudaLaunchCooperativeKernel((const void *)mw_flow_kernel<RP, YT>, dim3(grid), dim3(Lay::NT), args,

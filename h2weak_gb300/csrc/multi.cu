@@ -519,17 +519,6 @@ __global__ void __launch_bounds__(4 * RP)
     }
 }
 
-static int mr_num_sms() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 // Dataflow form of mr_coop_kernel: no grid barriers. Targets are claimed in
 // their stored order (a topological order: every producer of a target
 // precedes it), first blockIdx.x, then from a global counter; a CTA waits
@@ -583,7 +572,8 @@ static cudaError_t mr_flow_launch(const int64_t *roff, const int64_t *blob, int6
                                   YT *yout, int32_t *err, cudaStream_t st) {
     using Lay = MrLayout<T, RP>;
     constexpr size_t SMEM = (std::is_same<T, float>::value && !DF) ? Lay::smem_async : Lay::smem;
-    static int per_sm = 0;
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
     if (per_sm == 0) {
         if (cudaFuncSetAttribute(mr_flow_kernel<T, RP, DF, YT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)SMEM) != cudaSuccess)
@@ -591,7 +581,7 @@ static cudaError_t mr_flow_launch(const int64_t *roff, const int64_t *blob, int6
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mr_flow_kernel<T, RP, DF, YT>, Lay::NT, SMEM);
         if (per_sm <= 0) return cudaErrorCooperativeLaunchTooLarge;
     }
-    const int grid = mr_num_sms() * per_sm;
+    const int grid = device_sms() * per_sm;
     void *args[] = {(void *)&roff, (void *)&blob, (void *)&nt, (void *)&ctr, (void *)&rem, (void *)&coff,
                     (void *)&cidx, (void *)&A, (void *)&ws, (void *)&xin, (void *)&yout, (void *)&err};
     cudaError_t e = cudaLaunchCooperativeKernel((const void *)mr_flow_kernel<T, RP, DF, YT>, dim3(grid), dim3(Lay::NT),
@@ -633,8 +623,12 @@ static cudaError_t mr_launch_t(const int64_t *roff, const int64_t *blob, const i
                                YT *yout, unsigned *bar, int32_t *err, cudaStream_t st) {
     using Lay = MrLayout<T, RP>;
     constexpr size_t SMEM = (std::is_same<T, float>::value && !DF) ? Lay::smem_async : Lay::smem;
-    static int per_sm_coop = 0, per_sm = 0;
-    static bool attr = false;
+    static PerDevice<int> per_sm_coop_of;
+    int &per_sm_coop = per_sm_coop_of.here();
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
+    static PerDevice<bool> attr_of;
+    bool &attr = attr_of.here();
     if (!attr) {
         cudaError_t e = cudaFuncSetAttribute(mr_coop_kernel<T, RP, DF, YT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)SMEM);
@@ -643,7 +637,7 @@ static cudaError_t mr_launch_t(const int64_t *roff, const int64_t *blob, const i
         if (e != cudaSuccess) return e;
         attr = true;
     }
-    const int nsm = mr_num_sms();
+    const int nsm = device_sms();
     if (phased) {
         if (per_sm == 0) {
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mr_kernel<T, RP, DF, YT>, Lay::NT, SMEM);

@@ -648,23 +648,12 @@ __global__ void __launch_bounds__(NG_THREADS, 2)
     }
 }
 
-static int ng_sms() {
-    static int n = 0;
-    if (n == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        if (n <= 0) n = 1;
-    }
-    return n;
-}
-
 int nca_group_grid(int dcap, bool df) {
     (void)dcap;  // shared memory no longer depends on the rank
     int per_sm = 0;
     if (df) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nca_group_kernel<float2>, NG_THREADS, 0);
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nca_group_kernel<double>, NG_THREADS, 0);
-    return per_sm > 0 ? ng_sms() * per_sm : 0;
+    return per_sm > 0 ? device_sms() * per_sm : 0;
 }
 
 cudaError_t launch_nca_group(const NcaProb *probs, const int64_t *moff, int nprob, int G, int grid,
