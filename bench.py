@@ -749,12 +749,13 @@ def main():
     rp = 16 if R <= 16 else (32 if R <= 32 else 64)
     # DRAM bytes per launch (dram__bytes_read.sum + dram__bytes_write.sum) from the ncu captures of the
     # same launches on this workload: profiles/mw_flow_fp32_2d_ie_65536.md
-    kname = ("mr_coop_kernel" if not op.get_option(hw.OPT_DATAFLOW) else "mo_kernel" if top != "fp32" else
-             "mw_flow_kernel" if op.get_option(hw.OPT_PRODUCER_WARP) else "mr_flow_kernel")
+    digits = top != "fp32" and op.get_option(hw.OPT_COPIES_MADE) & 2  # the tensor-core form ran
+    kname = ("mr_coop_kernel" if not op.get_option(hw.OPT_DATAFLOW) else "mo_kernel" if digits else
+             "mw_flow_kernel" if top == "fp32" and op.get_option(hw.OPT_PRODUCER_WARP) else "mr_flow_kernel")
     ncu_traffic = {("mw_flow_kernel", "fp32"): 361.970e6 + 72.415e6}
     # the multi-vector kernel multiplies every packed operator entry by R vectors: one FMA per
     # term (FP32), about twelve FP32 operations per term (double-FP32 on the FP32 pipes); nominal FP32
-    # peak of 152 SMs x 128 lanes x 2 flop x 2.07 GHz. The tensor-core form (mo_kernel) multiplies 36
+    # peak of 152 SMs x 128 lanes x 2 flop x 2.07 GHz. The tensor-core form (mo_kernel) multiplies 60
     # pairs of digits a term, which the figures count as its one FMA.
     entries = op.operator_bytes(hw.PREC_FP32) / 4
     fp32_nominal = 152 * 128 * 2 * 2.07e9

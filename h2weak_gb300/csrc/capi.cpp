@@ -11,6 +11,7 @@
 #include <cstring>
 #include <deque>
 #include <memory>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -44,6 +45,50 @@ struct ApiError : std::runtime_error {
 // pointers and is rebuilt when the generation moved.
 std::atomic<uint64_t> g_alloc_gen{0};
 
+// What holds copies of an operator that it could do without (other layouts of the same entries, for
+// faster products): when an allocation on the device fails, the idle owners give theirs back.
+// An owner is idle when no call on it is in progress (`busy` is free, or held by the allocating call itself,
+// which reads a copy's address only after its allocations), and keeps its copies once a stream capture of the
+// caller's has taken their addresses.
+struct CopyOwner {
+    std::recursive_mutex busy;
+    bool captured = false;
+    virtual int copies_device() const = 0;
+    virtual bool give_back() = 0;  // true if it had any
+    void enlist();
+    void strike();
+    virtual ~CopyOwner() {}
+};
+std::mutex g_owners_lock;
+std::vector<CopyOwner *> g_owners;
+void CopyOwner::enlist() {
+    std::lock_guard<std::mutex> l(g_owners_lock);
+    g_owners.push_back(this);
+}
+void CopyOwner::strike() {
+    std::lock_guard<std::mutex> l(g_owners_lock);
+    g_owners.erase(std::remove(g_owners.begin(), g_owners.end(), this), g_owners.end());
+}
+// One owner's copies on the current device; false if there are none left to give
+bool give_back_copies() {
+    int dev = -1;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    std::lock_guard<std::mutex> l(g_owners_lock);
+    for (CopyOwner *o : g_owners) {
+        std::unique_lock<std::recursive_mutex> b(o->busy, std::try_to_lock);
+        if (b.owns_lock() && !o->captured && o->copies_device() == dev && o->give_back()) return true;
+    }
+    return false;
+}
+// This thread captures a step of its own (the graph is made again when a buffer goes)
+thread_local bool t_own_capture = false;
+void note_capture(CopyOwner &o, cudaStream_t st) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (t_own_capture || o.captured) return;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess) cudaGetLastError();
+    if (c != cudaStreamCaptureStatusNone) o.captured = true;
+}
+
 template <class T> struct DBuf {
     T *p = nullptr;
     size_t n = 0;
@@ -64,6 +109,12 @@ template <class T> struct DBuf {
         if (cnt == 0) cnt = 1;
         g_alloc_gen.fetch_add(1);
         cudaError_t e = cudaMalloc(&p, cnt * sizeof(T));
+        while (e == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            p = nullptr;
+            if (!give_back_copies()) break;
+            e = cudaMalloc(&p, cnt * sizeof(T));
+        }
         if (e != cudaSuccess) {
             p = nullptr;
             throw ApiError(H2W_ERR_NOMEM, "cudaMalloc of " + std::to_string(cnt * sizeof(T)) + " bytes failed");
@@ -89,6 +140,7 @@ struct MoStream {
     int32_t list[3][2] = {{0, 0}, {0, 0}, {0, 0}};
     int32_t share = 0, ngrp = 0, nwb = 0, nxb = 0, nzrow = 0;
     bool fused = true, ready = false, refused = false;
+    bool bad = false;  // an entry is not finite
 };
 
 // Device state of the lockstep GMRES for one Krylov-vector type T
@@ -124,7 +176,7 @@ namespace {
 struct PlanBuilder;
 }
 
-struct h2w_handle {
+struct h2w_handle : CopyOwner {
     h2w_config cfg{};
     std::string err;
     std::vector<double> pts;
@@ -232,6 +284,10 @@ struct h2w_handle {
     bool producer_warp = true;  // the FP32 dataflow product's warp-specialised form (H2W_OPT_PRODUCER_WARP)
     DBuf<int32_t> d_mdep0, d_mdep, d_mcidx;
     DBuf<int64_t> d_mcoff;
+    // the same for the single-vector stream on the packed operator, made when an FP64 product has no copy
+    DBuf<int32_t> d_sdep0, d_sdep, d_scidx, d_sctr;
+    DBuf<int64_t> d_scoff;
+    bool copies = true;  // H2W_OPT_COPIES
     int64_t mflow_edges = 0;
     // multi-vector plan: targets, panels, operator entries per column, entries
     // the kernel multiplies (rows to warp granularity, each panel's columns to
@@ -266,6 +322,19 @@ struct h2w_handle {
     double learn_rhat = 0.0, learn_r1 = 0.0;
     double learn_ms = 0.0;
     cudaStream_t stream = nullptr;
+
+    int copies_device() const override { return cfg.device; }
+    bool give_back() override {
+        if (!d_op64s.p && !mo.ready) return false;
+        cudaDeviceSynchronize();  // products on callers' streams
+        d_op64s.reset();
+        if (mo.ready) {
+            mo.img.reset();
+            mo.ready = false;
+            mo.refused = true;
+        }
+        return true;
+    }
 
     KParams kparams() const {
         KParams k;
@@ -2191,10 +2260,24 @@ void mo_upload(const SvHost &v, MoStream &d, cudaStream_t st) {
     d.rem.alloc(v.cnt.size());
     if (!d.ctr.p) d.ctr.alloc(SV_CTRS);
     d.img.reset();
-    d.ready = d.refused = false;
+    d.ready = d.refused = d.bad = false;
     CK(cudaStreamSynchronize(st));
 }
 
+// The FP64 operator in the single-vector stream's slices, a second one in memory: only where that
+// leaves the room of the FP32 copies and of a double-FP32 one (three times as much again); else FP64
+// products run on the packed operator (run_matvec_f64).
+void copy_f64s(h2w_handle *h) {
+    size_t fr = 0, tot = 0;
+    const size_t need = (size_t)std::max<int64_t>(h->ops_n, 4) * 8;
+    h->d_op64s.reset();
+    CK(cudaMemGetInfo(&fr, &tot));
+    if (!h->copies || fr / 4 < need) return;
+    h->d_op64s.alloc(need / 8);
+    CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 6, h->d_op64s.p, h->stream));
+}
+
+// (Re)cut the single-vector target stream from the handle's logical targets, with the figures
 // for the profiling statistics.
 void realize_single(h2w_handle *h, int64_t row_split) {
     if (!h->plan) throw ApiError(H2W_ERR_STATE, "operator not assembled");
@@ -2252,17 +2335,8 @@ void realize_single(h2w_handle *h, int64_t row_split) {
         h->op32s_ready = false;
         h->d_op32s.reset();
         sv_upload(sv, {0}, h->sv, st);
-        // The FP64 copy is made with the operator, a second one in memory: only where that
-        // leaves the room of the FP32 copies and of a double-FP32 one (three times as much
-        // again); else FP64 products stay on the packed operator and the cooperative launch.
-        size_t fr = 0, tot = 0;
-        const size_t need = (size_t)std::max<int64_t>(h->ops_n, 4) * 8;
-        h->d_op64s.reset();
-        CK(cudaMemGetInfo(&fr, &tot));
-        if (fr / 4 >= need) {
-            h->d_op64s.alloc(need / 8);
-            CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 6, h->d_op64s.p, st));
-        }
+        h->d_sdep0.reset();
+        copy_f64s(h);
     }
     CK(cudaStreamSynchronize(st));
 }
@@ -3096,6 +3170,36 @@ void sv_product(h2w_handle *h, int prec, SvArgs<T> a, cudaStream_t st, F &&far) 
     prof_launch(h, prec, nph, st, [&] { return sv_run(h, a, st); });
 }
 
+// The dependency lists of the single-vector stream on the packed operator, for FP64 dataflow products
+// without a copy. False where they cannot be made now (they need allocations, which a caller's stream
+// capture forbids): such a product takes the launch with grid barriers.
+bool flow_lists(h2w_handle *h, cudaStream_t st) {
+    if (h->d_sdep0.p) return true;
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    PlanBuilder &pb = *h->plan;
+    std::vector<Phase> ph;
+    bool fused = true;
+    pb.realize(h->row_split, 4, XW_CAP);  // as realize_single
+    assign_phases(h, pb, h->nph_total, ph, fused);
+    std::vector<int32_t> cnt, cidx;
+    std::vector<int64_t> coff;
+    build_deps(pb, h->ws_n, cnt, coff, cidx);
+    pb.T = std::vector<Target>();
+    pb.P = std::vector<Panel>();
+    pb.S = std::vector<Seg>();
+    h->d_sdep.alloc(cnt.size());
+    h->d_scoff.upload(coff, h->stream);
+    h->d_scidx.upload(cidx, h->stream);
+    if (!h->d_sctr.p) h->d_sctr.alloc(1);
+    h->d_sdep0.upload(cnt, h->stream);
+    CK(cudaStreamSynchronize(h->stream));  // products may run on a caller's stream
+    return true;
+}
+
 // y = A x. permuted: x and y in leaf order (GMRES works there: no gather or
 // scatter per product); otherwise original point order.
 // df: with the far field on the fly, its M2L in double-FP32 arithmetic
@@ -3105,7 +3209,7 @@ void run_matvec_f64(h2w_handle *h, const double *dx, double *dy, cudaStream_t st
                     bool df = false) {
     const int32_t *perm = permuted ? nullptr : h->d_perm.p;
     const int nph = (int)h->phases.size();
-    const bool flow = h->coop && h->dataflow && h->d_op64s.p;
+    const bool flow = h->coop && h->dataflow && h->copies && h->d_op64s.p;
     auto far = [&] {
         prof_launch(h, df ? H2W_PREC_DF64 : H2W_PREC_FP64, FLY_PHASE, st, [&] {
             if (df)
@@ -3117,7 +3221,16 @@ void run_matvec_f64(h2w_handle *h, const double *dx, double *dy, cudaStream_t st
         });
     };
     if (flow) {
+        note_capture(*h, st);
         sv_product(h, H2W_PREC_FP64, sv_args<double>(h, h->d_op64s.p, h->d_ws.p, dx, dy, perm), st, far);
+    } else if (h->coop && h->dataflow && !h->fly_active && flow_lists(h, st)) {
+        CK(cudaMemsetAsync(h->d_ws.p, 0, (size_t)h->ws_n * 8, st));
+        CK(cudaMemcpyAsync(h->d_sdep.p, h->d_sdep0.p, h->d_sdep0.n * 4, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemsetAsync(h->d_sctr.p, 0, 4, st));
+        prof_launch(h, H2W_PREC_FP64, nph, st, [&] {
+            return launch_brg_flow_f64(h->d_roff.p, h->d_blob.p, (int64_t)h->d_roff.n - 1, h->d_sctr.p, h->d_sdep.p,
+                                       h->d_scoff.p, h->d_scidx.p, h->d_op.p, h->d_ws.p, dx, dy, perm, h->d_err.p, st);
+        });
     } else {
         CK(cudaMemsetAsync(h->d_ws.p, 0, (size_t)h->ws_n * 8, st));
         auto stored = [&](int a, int b) {  // phases [a, b)
@@ -3231,6 +3344,10 @@ bool capture_loop(cudaStream_t st, cudaGraph_t &graph, cudaGraphExec_t &exec, in
     exec = nullptr;
     const int64_t c0 = launch_count();
     bool capturing = false;
+    t_own_capture = true;
+    struct Done {
+        ~Done() { t_own_capture = false; }
+    } done;
     try {
         CK(cudaGraphCreate(&graph, 0));
         cudaGraphConditionalHandle cond;
@@ -3329,23 +3446,30 @@ void mr_prof(h2w_handle *h, int prec, int rp, cudaStream_t st, F &&launch) {
 // FP32 pipes.
 bool ensure_mo(h2w_handle *h) {
     MoStream &d = h->mo;
-    if (d.ready || d.refused) return d.ready;
+    if (!h->copies || d.refused) return false;
+    if (d.ready) return true;
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
     d.refused = d.bytes <= 0 || fr / 2 < (size_t)d.bytes || h->xoff() + h->nv() >= (int64_t)INT32_MAX;
     if (d.refused) return false;
     cudaStream_t st = h->stream;
-    d.img.alloc((size_t)d.bytes);
-    d.sa.alloc(d.plist.n * 64);
-    d.col.alloc(d.plist.n * (size_t)mo_part_columns());
-    d.mx.alloc((size_t)(d.nwb + d.nxb) * MR_MAX);
+    try {
+        d.img.alloc((size_t)d.bytes);
+        d.sa.alloc(d.plist.n * 64);
+        d.col.alloc(d.plist.n * (size_t)mo_part_columns());
+        d.mx.alloc((size_t)(d.nwb + d.nxb) * MR_MAX);
+    } catch (const ApiError &) {  // the room went meanwhile
+        d.refused = true;
+        d.img.reset();
+        return false;
+    }
     CK(cudaMemsetAsync(d.mx.p, 0, 4, st));  // the first word reports a bad entry
     CK(launch_mo_image(d.hdr.p, d.list[2][1], d.s0.p, d.slices.p, h->d_op.p, d.img.p, d.sa.p, d.col.p, d.mx.p, st));
     int32_t bad = 0;
     CK(cudaMemcpyAsync(&bad, d.mx.p, 4, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (bad) {
-        d.refused = true;
+        d.refused = d.bad = true;
         d.img.reset();
         return false;
     }
@@ -3447,15 +3571,16 @@ void run_matvec_multi(h2w_handle *h, int prec, int rp, int nrhs, const double *x
         });
         if (!h->fused_scatter_m) CK(launch_mr_widen_f32(h->m_wsf.p + (size_t)h->yperm_off * rp, yi, h->tree.N * rp, st));
     } else {
-        if (h->dataflow && h->coop && mo_pays(h, prec, rp, nrhs) && ensure_mo(h)) {
-            const size_t need = (size_t)(h->xoff() + h->nv()) * (size_t)rp;
-            if (h->m_wsd.n < need) h->m_wsd.alloc(need);
+        const bool digits = h->dataflow && h->coop && !h->mo.refused && mo_pays(h, prec, rp, nrhs);
+        const size_t need = digits ? (size_t)(h->xoff() + h->nv()) * (size_t)rp : wsz;
+        if (h->m_wsd.n < need) h->m_wsd.alloc(need);  // first: it may take the copies back
+        if (digits && ensure_mo(h)) {
+            note_capture(*h, st);
             const MoArgs a = mo_args(h, prec, rp, nrhs, xi, yi);
             mr_prof(h, prec, rp, st, [&] { return launch_mo(a, st); });
             if (!h->mo.fused) CK(launch_mo_unplane(a, h->yperm_off, h->tree.N, yi, st));
             return;
         }
-        if (h->m_wsd.n < wsz) h->m_wsd.alloc(wsz);
         CK(cudaMemsetAsync(h->m_wsd.p, 0, wsz * 8, st));
         if (prec == H2W_PREC_DF64) {  // operator split once; the input block split per product
             if (!h->d_opdf.p) {
@@ -3889,7 +4014,7 @@ void check_device_error(h2w_handle *h) {
 // launch per product; the solvers run every problem's GMRES in lockstep over
 // concatenated vectors. The handles must outlive the batch and must not be
 // re-assembled while it exists.
-struct h2w_batch {
+struct h2w_batch : CopyOwner {
     std::vector<h2w_handle *> hs;
     std::string err;
     int device = 0;
@@ -3930,6 +4055,15 @@ struct h2w_batch {
     DBuf<int32_t> conv, iter, bprob, pblk;
     DBuf<int64_t> brow;
     int g_m = -1, nblk = 0;
+
+    int copies_device() const override { return device; }
+    bool give_back() override {
+        if (!A64.p) return false;
+        cudaDeviceSynchronize();
+        A64.reset();
+        op64.clear();
+        return true;
+    }
 };
 
 namespace {
@@ -3937,6 +4071,7 @@ namespace {
 template <class F>
 int bguarded(h2w_batch *b, F &&f) {
     if (!b) return H2W_ERR_ARG;
+    std::lock_guard<std::recursive_mutex> in_use(b->busy);
     try {
         if (cudaSetDevice(b->device) != cudaSuccess) {
             b->err = "cudaSetDevice failed";
@@ -4001,51 +4136,6 @@ cudaError_t batch_sv(h2w_batch *b, const T *const *A, T *ws, const SvConf &conf,
     return launch_sv(a, conf, b->stream);
 }
 
-// y = A x for every problem: x, y concatenated, leaf order (leaf) or each
-// problem's original point order.
-void run_batch(h2w_batch *b, int prec, const double *x, double *y, bool leaf, const int32_t *active = nullptr) {
-    cudaStream_t st = b->stream;
-    const bool f32 = prec == H2W_PREC_FP32;
-    const int P = (int)b->hs.size();
-    if (f32 && b->op32.empty()) {
-        std::vector<std::unique_ptr<DBuf<float>>> op((size_t)P);
-        std::vector<const float *> tab((size_t)P);
-        for (int p = 0; p < P; ++p) {
-            op[(size_t)p].reset(new DBuf<float>());
-            op[(size_t)p]->alloc((size_t)std::max<int64_t>(b->opn[(size_t)p], 4));
-            CK(launch_sv_slices(b->hs[(size_t)p]->d_op.p, b->slices[(size_t)p].p, (int64_t)b->slices[(size_t)p].n / 6,
-                                op[(size_t)p]->p, st));
-            tab[(size_t)p] = op[(size_t)p]->p;
-        }
-        b->ws32.alloc((size_t)(b->xoff + b->Ntot));
-        b->A32.upload(tab, st);
-        CK(cudaStreamSynchronize(st));
-        b->op32.swap(op);
-    }
-    const std::vector<int> *unfused = &b->unfused;
-    if (f32) {
-        CK(batch_sv<float>(b, b->A32.p, b->ws32.p, b->sv.f32, x, y, leaf, active));
-    } else if (b->A64.p) {
-        CK(batch_sv<double>(b, b->A64.p, b->ws64.p, b->sv.f64, x, y, leaf, active));
-    } else {
-        CK(cudaMemsetAsync(b->ws64.p, 0, (size_t)b->wsoff[(size_t)P] * 8, st));
-        CK(launch_brgb_f64(b->roff.p, b->blob.p, b->pstart.p, b->nphase, leaf ? b->tab64_leaf.p : b->tab64_orig.p,
-                           active, x, y, b->bar.p, b->errf.p, st));
-        unfused = &b->unfused_ph;
-    }
-    for (int p : *unfused) {
-        h2w_handle *h = b->hs[(size_t)p];
-        const int64_t N = h->tree.N, o = b->off[(size_t)p], w0 = b->wsoff[(size_t)p] + h->yperm_off;
-        if (f32) {
-            if (leaf) CK(vec_f32_to_f64(b->ws32.p + w0, y + o, N, st));
-            else CK(launch_scatter_f32(b->ws32.p + w0, y + o, h->d_perm.p, N, st));
-        } else {
-            if (leaf) CK(cudaMemcpyAsync(y + o, b->ws64.p + w0, (size_t)N * 8, cudaMemcpyDeviceToDevice, st));
-            else CK(launch_scatter_f64(b->ws64.p + w0, y + o, h->d_perm.p, N, st));
-        }
-    }
-}
-
 // The merged stream of a batch's FP64 products by phases: records with the problem
 // index in the flags, phases aligned at the leaf end.
 void batch_phased(h2w_batch *b) {
@@ -4056,6 +4146,7 @@ void batch_phased(h2w_batch *b) {
     std::vector<size_t> nph((size_t)P);
     for (int p = 0; p < P; ++p) {
         h2w_handle *h = b->hs[(size_t)p];
+        std::lock_guard<std::recursive_mutex> in_use(h->busy);  // its plan is cut again
         PlanBuilder &pb = *h->plan;
         std::vector<Phase> ph;
         bool fused = true;
@@ -4097,7 +4188,6 @@ void batch_phased(h2w_batch *b) {
         }
     }
     pstart.push_back((int64_t)roff.size() - 1);
-    b->nphase = (int)maxph;
     cudaStream_t st = b->stream;
     b->roff.upload(roff, st);
     b->blob.upload(blob, st);
@@ -4111,6 +4201,54 @@ void batch_phased(h2w_batch *b) {
     }
     b->tab64_orig.upload(to, st);
     b->tab64_leaf.upload(tl, st);
+    CK(cudaStreamSynchronize(st));  // the host arrays end here
+    b->nphase = (int)maxph;
+}
+
+// y = A x for every problem: x, y concatenated, leaf order (leaf) or each
+// problem's original point order.
+void run_batch(h2w_batch *b, int prec, const double *x, double *y, bool leaf, const int32_t *active = nullptr) {
+    cudaStream_t st = b->stream;
+    const bool f32 = prec == H2W_PREC_FP32;
+    const int P = (int)b->hs.size();
+    if (f32 && b->op32.empty()) {
+        std::vector<std::unique_ptr<DBuf<float>>> op((size_t)P);
+        std::vector<const float *> tab((size_t)P);
+        for (int p = 0; p < P; ++p) {
+            op[(size_t)p].reset(new DBuf<float>());
+            op[(size_t)p]->alloc((size_t)std::max<int64_t>(b->opn[(size_t)p], 4));
+            CK(launch_sv_slices(b->hs[(size_t)p]->d_op.p, b->slices[(size_t)p].p, (int64_t)b->slices[(size_t)p].n / 6,
+                                op[(size_t)p]->p, st));
+            tab[(size_t)p] = op[(size_t)p]->p;
+        }
+        b->ws32.alloc((size_t)(b->xoff + b->Ntot));
+        b->A32.upload(tab, st);
+        CK(cudaStreamSynchronize(st));
+        b->op32.swap(op);
+    }
+    const std::vector<int> *unfused = &b->unfused;
+    if (f32) {
+        CK(batch_sv<float>(b, b->A32.p, b->ws32.p, b->sv.f32, x, y, leaf, active));
+    } else if (b->A64.p) {
+        CK(batch_sv<double>(b, b->A64.p, b->ws64.p, b->sv.f64, x, y, leaf, active));
+    } else {
+        if (b->nphase == 0) batch_phased(b);
+        CK(cudaMemsetAsync(b->ws64.p, 0, (size_t)b->wsoff[(size_t)P] * 8, st));
+        CK(launch_brgb_f64(b->roff.p, b->blob.p, b->pstart.p, b->nphase, leaf ? b->tab64_leaf.p : b->tab64_orig.p,
+                           active, x, y, b->bar.p, b->errf.p, st));
+        unfused = &b->unfused_ph;
+    }
+    for (int p : *unfused) {
+        h2w_handle *h = b->hs[(size_t)p];
+        const int64_t N = h->tree.N, o = b->off[(size_t)p], w0 = b->wsoff[(size_t)p] + h->yperm_off;
+        if (f32) {
+            if (leaf) CK(vec_f32_to_f64(b->ws32.p + w0, y + o, N, st));
+            else CK(launch_scatter_f32(b->ws32.p + w0, y + o, h->d_perm.p, N, st));
+        } else {
+            if (leaf) CK(cudaMemcpyAsync(y + o, b->ws64.p + w0, (size_t)N * 8, cudaMemcpyDeviceToDevice, st));
+            else CK(launch_scatter_f64(b->ws64.p + w0, y + o, h->d_perm.p, N, st));
+        }
+    }
 }
 
 GmresSeg gms_state(h2w_batch *b, int m) {
@@ -4304,6 +4442,7 @@ int fail(h2w_handle *h, int code, const std::string &m) {
 template <class F>
 int guarded(h2w_handle *h, F &&f) {
     if (!h) return H2W_ERR_ARG;
+    std::lock_guard<std::recursive_mutex> in_use(h->busy);
     try {
         if (h->cfg.device >= 0 && cudaSetDevice(h->cfg.device) != cudaSuccess)
             return fail(h, H2W_ERR_CUDA, "cudaSetDevice failed");
@@ -4534,6 +4673,7 @@ int h2w_create(const h2w_config *cfg, h2w_handle **out) {
             delete h;
             return H2W_ERR_CUDA;
         }
+        h->enlist();
     } else {
         // host-only handle: points, tree and lists, no device work
         h = new h2w_handle;
@@ -4546,6 +4686,7 @@ int h2w_create(const h2w_config *cfg, h2w_handle **out) {
 
 int h2w_destroy(h2w_handle *h) {
     if (!h) return H2W_OK;
+    h->strike();
     if (h->cfg.device >= 0) cudaSetDevice(h->cfg.device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (auto &r : h->prof_recs) {
@@ -5283,6 +5424,15 @@ int h2w_set_option(h2w_handle *h, int option, int64_t value) {
         } else if (option == H2W_OPT_FAR_ON_THE_FLY) {
             if (value != 0) require_real(h, "the far field on the fly");
             h->far_fly = value != 0;  // takes effect at the next h2w_assemble
+        } else if (option == H2W_OPT_COPIES) {
+            h->copies = value != 0;
+            if (!h->copies && !h->captured) h->give_back();
+            if (h->copies && h->has_op && !h->d_op64s.p) copy_f64s(h);
+            h->mo.refused = h->mo.bad;  // asked again at the next product
+            h->eta_multi = h->eta_single = -1.0;  // other sums, other rounding
+            CK(cudaStreamSynchronize(h->stream));
+        } else if (option == H2W_OPT_COPIES_MADE) {
+            throw ApiError(H2W_ERR_ARG, "H2W_OPT_COPIES_MADE is read only");
         } else if (option == H2W_OPT_COOP) {
             h->coop = value != 0;
             for (auto &g : h->loops) {  // captured steps hold the other launch form
@@ -5314,6 +5464,8 @@ int h2w_get_option(h2w_handle *h, int option, int64_t *value) {
         else if (option == H2W_OPT_FAR_ON_THE_FLY) *value = h->far_fly ? 1 : 0;
         else if (option == H2W_OPT_NCA_DF) *value = h->nca_df ? 1 : 0;
         else if (option == H2W_OPT_COMPLEX_ARNOLDI) *value = h->cgm_hermitian ? 1 : 0;
+        else if (option == H2W_OPT_COPIES) *value = h->copies ? 1 : 0;
+        else if (option == H2W_OPT_COPIES_MADE) *value = (h->d_op64s.p ? 1 : 0) | (h->mo.ready ? 2 : 0);
         else throw ApiError(H2W_ERR_ARG, "unknown option");
         return H2W_OK;
     });
@@ -5462,7 +5614,9 @@ int h2w_batch_create(h2w_handle *const *handles, int n, h2w_batch **out) {
         int64_t all = 0;
         for (int64_t v : b->opn) all += std::max<int64_t>(v, 4);
         CK(cudaMemGetInfo(&fr, &tot));
-        if (fr / 2 >= (size_t)all * 8) {
+        bool copies = true;
+        for (h2w_handle *h : b->hs) copies = copies && h->copies;
+        if (copies && fr / 2 >= (size_t)all * 8) {
             std::vector<const double *> tab((size_t)P);
             for (int p = 0; p < P; ++p) {
                 b->op64.emplace_back(new DBuf<double>());
@@ -5473,8 +5627,6 @@ int h2w_batch_create(h2w_handle *const *handles, int n, h2w_batch **out) {
             }
             b->A64.upload(tab, st);
             CK(cudaStreamSynchronize(st));
-        } else {
-            batch_phased(b);
         }
         std::vector<int64_t> pa((size_t)b->Ntot);
         for (int p = 0; p < P; ++p) {
@@ -5517,12 +5669,14 @@ int h2w_batch_create(h2w_handle *const *handles, int n, h2w_batch **out) {
         delete b;
         return rc;
     }
+    b->enlist();
     *out = b;
     return H2W_OK;
 }
 
 int h2w_batch_destroy(h2w_batch *b) {
     if (!b) return H2W_OK;
+    b->strike();
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     for (auto &L : b->loops) {

@@ -407,6 +407,46 @@ __global__ void __launch_bounds__(BRG_THREADS, 4)
     }
 }
 
+// Dataflow form of brg_coop_kernel (no grid barriers), for FP64 products of operators without room for
+// the copy that sv.cu streams: targets claimed in stored (topological) order from a
+// global counter; each waits until its producer count rem[t] is zero (bounded spin: on timeout
+// *err = 3 and the CTA proceeds), runs, fences its writes and decrements the counts of its
+// consumers cidx[coff[t] .. coff[t+1]). Cooperative launch: every CTA is resident, so the
+// producers of a waiting target are all claimed and running. 2D integral equation, 65536 points: 218 us,
+// 320 with grid barriers (154 on the copy); 3D semi-nested RBF, 20011 points: 667, 752 (472).
+__global__ void __launch_bounds__(BRG_THREADS, 4)
+    brg_flow_kernel(const int64_t *__restrict__ roff, const int64_t *__restrict__ blob, int64_t nt, int32_t *ctr,
+                    int32_t *rem, const int64_t *__restrict__ coff, const int32_t *__restrict__ cidx,
+                    const double *__restrict__ A, double *ws, const double *__restrict__ xin, double *yout,
+                    const int32_t *__restrict__ perm, int32_t *err) {
+    __shared__ BrgShared<double> sh;
+    __shared__ int64_t s_next;
+    int64_t t = blockIdx.x;
+    while (t < nt) {
+        if (threadIdx.x == 0) {
+            long long it = 0;
+            while (*((volatile int32_t *)(rem + t)) > 0) {
+                if (++it > (1LL << 20)) {  // about 0.1 s
+                    atomicExch(err, 3);
+                    break;
+                }
+                __nanosleep(32);
+            }
+            __threadfence();
+        }
+        __syncthreads();
+        brg_target<double>(sh, t, roff, blob, A, ws, xin, yout, perm);
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            __threadfence();  // this CTA's results are visible before its consumers are released
+            for (int64_t e = coff[t] + threadIdx.x; e < coff[t + 1]; e += 32) atomicSub(rem + cidx[e], 1);
+            if (threadIdx.x == 0) s_next = gridDim.x + atomicAdd(ctr, 1);
+        }
+        __syncthreads();
+        t = s_next;
+    }
+}
+
 // Many independent problems in one cooperative launch: the problem index of
 // a target sits in bits 8.. of its record's flag word, and the target runs
 // on that problem's operator, workspace, point permutation and vector
@@ -468,6 +508,24 @@ static cudaError_t launch_coop_t(const int64_t *roff, const int64_t *blob, const
                     (void *)&xin, (void *)&yout, (void *)&perm, (void *)&bar, (void *)&err, (void *)&spin};
     cudaError_t e = cudaLaunchCooperativeKernel((const void *)brg_coop_kernel<T>, dim3(grid), dim3(BRG_THREADS), args,
                                                 0, st);
+    count_launch();
+    return e;
+}
+
+cudaError_t launch_brg_flow_f64(const int64_t *roff, const int64_t *blob, int64_t nt, int32_t *ctr, int32_t *rem,
+                                const int64_t *coff, const int32_t *cidx, const double *A, double *ws,
+                                const double *xin, double *yout, const int32_t *perm, int32_t *err, cudaStream_t st) {
+    if (nt <= 0) return cudaSuccess;
+    static PerDevice<int> per_sm_of;
+    int &per_sm = per_sm_of.here();
+    if (per_sm == 0) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, brg_flow_kernel, BRG_THREADS, 0);
+        if (per_sm <= 0) return cudaErrorCooperativeLaunchTooLarge;
+    }
+    const int grid = device_sms() * per_sm;
+    void *args[] = {(void *)&roff, (void *)&blob, (void *)&nt, (void *)&ctr, (void *)&rem,  (void *)&coff, (void *)&cidx,
+                    (void *)&A,    (void *)&ws,   (void *)&xin, (void *)&yout, (void *)&perm, (void *)&err};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void *)brg_flow_kernel, dim3(grid), dim3(BRG_THREADS), args, 0, st);
     count_launch();
     return e;
 }

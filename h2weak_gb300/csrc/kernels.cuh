@@ -152,6 +152,12 @@ cudaError_t launch_sv(const SvArgs<float> &a, const SvConf &c, cudaStream_t st);
 // the slices of an FP64 operator (as launch_slice_copy_f32) copied or converted
 cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, double *dst, cudaStream_t st);
 cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, float *dst, cudaStream_t st);
+// Dataflow form of the FP64 product on the packed operator: the nt targets in stored order, ctr a zeroed
+// claim counter, rem the producer counts (reset before every launch), consumers in
+// cidx[coff[t] .. coff[t+1])
+cudaError_t launch_brg_flow_f64(const int64_t *roff, const int64_t *blob, int64_t nt, int32_t *ctr, int32_t *rem,
+                                const int64_t *coff, const int32_t *cidx, const double *A, double *ws,
+                                const double *xin, double *yout, const int32_t *perm, int32_t *err, cudaStream_t st);
 // The whole matvec as one cooperative launch: phase p covers targets
 // [pstart[p], pstart[p+1]); bar (2 unsigned, zero) is the grid barrier state;
 // spin bounds each grid-barrier wait in polls (<= 0: the built-in limit).

@@ -304,11 +304,25 @@ int h2w_gmres_ir_batch(h2w_handle *h, const double *b, double *x, int nrhs, int 
  *                 not the true residual (iteration counts and results match
  *                 the reference's). 1: Hermitian projections sum conj(v_k) w
  *                 and unitary rotations: GMRES proper, whose stopping test
- *                 bounds the true residual. */
+ *                 bounds the true residual.
+ *  H2W_OPT_COPIES  1 (default): where the memory free at the time allows,
+ *                 copies of the FP64 operator in other layouts are kept for
+ *                 faster products: one (8 bytes an entry, made with the
+ *                 operator where it fits four times) for FP64 products of one
+ *                 vector, one (20 bytes, made by the first such product) for
+ *                 products of several vectors on the tensor cores, and one (8)
+ *                 for each problem of a batch. When a later allocation of any
+ *                 handle or batch of the process on the device fails, idle
+ *                 ones give theirs back; a handle whose products a caller has
+ *                 captured into a graph keeps them. 0: none are made and the
+ *                 handle's are given back: the same products in other orders
+ *                 of summation, on the packed operator.
+ *  H2W_OPT_COPIES_MADE  read only: the copies a handle holds now (1: one
+ *                 vector, 2: tensor cores). */
 enum { H2W_OPT_GRAPH = 0, H2W_OPT_COOP = 1, H2W_OPT_IR_RESIDUAL = 2, H2W_OPT_MULTI_XW = 3, H2W_OPT_ROW_SPLIT = 4,
        H2W_OPT_IR_UPDATE = 5, H2W_OPT_TENSOR = 6, H2W_OPT_F32_BASIS = 7, H2W_OPT_DATAFLOW = 8,
        H2W_OPT_PRODUCER_WARP = 9, H2W_OPT_SPIN_LIMIT = 10, H2W_OPT_FAR_ON_THE_FLY = 11, H2W_OPT_NCA_DF = 12,
-       H2W_OPT_COMPLEX_ARNOLDI = 13 };
+       H2W_OPT_COMPLEX_ARNOLDI = 13, H2W_OPT_COPIES = 14, H2W_OPT_COPIES_MADE = 15 };
 int h2w_set_option(h2w_handle *h, int option, int64_t value);
 int h2w_get_option(h2w_handle *h, int option, int64_t *value);
 
