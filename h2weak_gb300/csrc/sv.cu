@@ -46,8 +46,8 @@
 // Measured against one kernel whose CTAs gathered, multiplied and released a target
 // at a time: 2D integral equation, 65536 points (62e6 entries): FP64 207 -> 153 us,
 // FP32 138 -> 80; 3D semi-nested RBF, 20011 points (2e8): FP64 665 -> 471 (FP64 pipe 67 %
-// busy), FP32 330 -> 165 (5.0 TB/s); 1D RBF, 4096 points: 69 -> 50, back to back on
-// several streams 18.
+// busy), FP32 330 -> 165 (5.0 TB/s); 1D RBF, 4096 points, waited for: 92 -> 75, calls on
+// several streams 69 -> 18 each.
 #include <algorithm>
 
 #include "kernels.cuh"
@@ -544,7 +544,10 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
             while (l < 3 && (nrows << (l + 1)) <= CT) ++l;
             const int part = tid & ((1 << l) - 1), flags = sl.flags;
             // the rows added to: only now does a target of input columns wait for the part before it
-            if ((flags & SV_LATE) && !__all_sync(0xffffffffu, lane != 0 || sv_until(a.rem + sl.grp, fail, a.err))) return;
+            if (flags & SV_LATE) {
+                if (!__all_sync(0xffffffffu, lane != 0 || sv_until(a.rem + sl.grp, fail, a.err))) return;
+                __syncwarp();  // lane 0's acquire, for the rows that the other lanes read
+            }
 #pragma unroll 1
             for (int r0 = 0; r0 < nrows; r0 += CT >> l) {
                 if (r0 + (warp * 32 >> l) >= nrows) break;  // the same for the whole warp
