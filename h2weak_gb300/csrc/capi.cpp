@@ -3215,7 +3215,7 @@ void run_matvec_f64(h2w_handle *h, const double *dx, double *dy, cudaStream_t st
             if (df)
                 return launch_fly_df64(h->d_fly_items.p, (int64_t)h->d_fly_items.n, h->d_fly_ctr.p, h->d_fly_rowpid.p,
                                        h->d_fly_cpid.p, h->d_fly_cws.p, h->d_ptsdf.p, h->d_logtab.p, h->d_ws.p,
-                                       h->kparams(), h->k32, st);
+                                       h->kparams(), h->k32, h->d_err.p, st);
             return launch_fly_f64(h->d_fly_items.p, (int64_t)h->d_fly_items.n, h->d_fly_ctr.p, h->d_fly_rowpid.p,
                                   h->d_fly_cpid.p, h->d_fly_cws.p, h->d_ws.p, h->kparams(), st);
         });
@@ -3998,6 +3998,7 @@ void check_device_error(h2w_handle *h) {
     if (e) {
         CK(cudaMemsetAsync(h->d_err.p, 0, 4, h->stream));
         CK(cudaMemsetAsync(h->d_bar.p, 0, 8, h->stream));
+        if (e == 5) throw ApiError(H2W_ERR_CUDA, "far field: a distance lies outside the logarithm's table (device error flag 5)");
         static const char *what[] = {"", "a grid-barrier wait", "a tensor-pipeline wait", "a dependency wait",
                                      "a stage (mbarrier or counter) wait"};
         throw ApiError(H2W_ERR_CUDA, std::string("matvec: ") + (e >= 1 && e <= 4 ? what[e] : "a device wait") +

@@ -199,11 +199,12 @@ cudaError_t launch_pts4(const double *pts, int dim, int64_t n, float *out, cudaS
 // The FP64-accurate form on the FP32 pipes (double-FP32 arithmetic) for the
 // kernels built on log(R^2) when every far pair is farther apart than a (else
 // the FP64 form): ptsdf = (hi, lo) FP32 quadruples of the points
-// (launch_ptsdf, 8 floats per point), logtab = fly_df_table's entries.
+// (launch_ptsdf, 8 floats per point), logtab = fly_df_table's entries; *err = 5 if a pair's R^2
+// lies outside the table.
 bool fly_df_supported(const KParams &kp, const FlyK32 &k32);
 cudaError_t launch_fly_df64(const FlyItem *items, int64_t nitems, unsigned long long *ctr, const int32_t *rowpid,
                             const int32_t *cpid, const int32_t *cws, const float *ptsdf, const void *logtab,
-                            double *ws, const KParams &kp, const FlyK32 &k32, cudaStream_t st);
+                            double *ws, const KParams &kp, const FlyK32 &k32, int32_t *err, cudaStream_t st);
 void fly_df_table(int e0, int ne, float *out);  // 128 ne x 4 floats
 void fly_df_logtab(float *out);                 // of the pivot search, 128 x 8 floats
 cudaError_t launch_ptsdf(const double *pts, int dim, int64_t n, float *out, cudaStream_t st);

@@ -274,10 +274,12 @@ __global__ void __launch_bounds__(FLY_THREADS)
 // others keep the FP64 form.
 
 // log of r.h + r.l > 0 within the table's range (a pair, not renormalised); tab: n entries from
-// the bin of bits `base`, (log c, 1 / c) pairs
-__device__ __forceinline__ Df fly_log(Df r, const float4 *tab, unsigned base, unsigned n) {
-    const unsigned bits = __float_as_uint(r.h);
-    const float4 t = tab[min((bits >> 16) - base, n - 1u)];
+// the bin of bits `base`, (log c, 1 / c) pairs; far: the largest entry asked for, n or more
+// (below `base` too) where the range was left
+__device__ __forceinline__ Df fly_log(Df r, const float4 *tab, unsigned base, unsigned n, unsigned &far) {
+    const unsigned bits = __float_as_uint(r.h), bin = (bits >> 16) - base;
+    far = max(far, bin);
+    const float4 t = tab[min(bin, n - 1u)];
     const float d = __fsub_rn(r.h, __uint_as_float((bits & 0xffff0000u) | 0x8000u));  // r.h - c, exact
     const float u0 = __fmul_rn(d, t.z);
     float e = __fmaf_rn(d, t.z, -u0);
@@ -301,17 +303,21 @@ __global__ void __launch_bounds__(FLY_THREADS)
     m2l_flydf_kernel(const FlyItem *__restrict__ items, int64_t nitems, unsigned long long *ctr,
                      const int32_t *__restrict__ rowpid, const int32_t *__restrict__ cpid,
                      const int32_t *__restrict__ cws, const float *__restrict__ ptsdf, double *ws,
-                     const float4 *__restrict__ gtab, unsigned base, unsigned ntab, double scale) {
+                     const float4 *__restrict__ gtab, unsigned base, unsigned ntab, double scale, int32_t *err) {
     extern __shared__ __align__(16) float4 fly_tab[];
     __shared__ __align__(16) float sc[FLY_TILE][8];  // x, y, z hi; x, y, z lo; value hi, lo
     __shared__ long long s_it;
     for (unsigned i = threadIdx.x; i < ntab; i += FLY_THREADS) fly_tab[i] = gtab[i];
+    unsigned far = 0;
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) s_it = (long long)atomicAdd(ctr, 1ull);
         __syncthreads();
         const long long it = s_it;
-        if (it >= nitems) return;
+        if (it >= nitems) {
+            if (far >= ntab) atomicExch(err, 5);
+            return;
+        }
         const FlyItem m = items[it];
         const int lt = m.nrows > 16 ? 2 : m.nrows > 8 ? 3 : m.nrows > 4 ? 4 : 5, tpr = 1 << lt;
         const int row = threadIdx.x >> lt, sub = threadIdx.x & (tpr - 1);
@@ -356,7 +362,7 @@ __global__ void __launch_bounds__(FLY_THREADS)
                             r2 = Df{t.h, __fadd_rn(__fadd_rn(r2.l, e), t.l)};
                         }
                     }
-                    const Df lg = fly_log(df_fast(r2.h, r2.l), fly_tab, base, ntab);
+                    const Df lg = fly_log(df_fast(r2.h, r2.l), fly_tab, base, ntab, far);
                     // sum += lg * v
                     const float ph = __fmul_rn(lg.h, p1.z);
                     float pe = __fmaf_rn(lg.h, p1.z, -ph);
@@ -464,7 +470,7 @@ cudaError_t launch_fly_f32(const FlyItem *items, int64_t nitems, unsigned long l
 template <int DIM>
 static cudaError_t flydf_launch(const FlyItem *items, int64_t nitems, unsigned long long *ctr, const int32_t *rowpid,
                                 const int32_t *cpid, const int32_t *cws, const float *ptsdf, double *ws,
-                                const float4 *tab, const FlyK32 &k32, double scale, cudaStream_t st) {
+                                const float4 *tab, const FlyK32 &k32, double scale, int32_t *err, cudaStream_t st) {
     const size_t smem = (size_t)k32.ntab * sizeof(float4);
     int per_sm = 0;
     cudaError_t e = cudaFuncSetAttribute(m2l_flydf_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
@@ -476,7 +482,7 @@ static cudaError_t flydf_launch(const FlyItem *items, int64_t nitems, unsigned l
     e = cudaMemsetAsync(ctr, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;
     m2l_flydf_kernel<DIM><<<grid, FLY_THREADS, smem, st>>>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab,
-                                                           (unsigned)(127 + k32.tab_e0) << 7, (unsigned)k32.ntab, scale);
+                                                           (unsigned)(127 + k32.tab_e0) << 7, (unsigned)k32.ntab, scale, err);
     count_launch();
     return cudaGetLastError();
 }
@@ -487,13 +493,13 @@ bool fly_df_supported(const KParams &kp, const FlyK32 &k32) {
 
 cudaError_t launch_fly_df64(const FlyItem *items, int64_t nitems, unsigned long long *ctr, const int32_t *rowpid,
                             const int32_t *cpid, const int32_t *cws, const float *ptsdf, const void *logtab,
-                            double *ws, const KParams &kp, const FlyK32 &k32, cudaStream_t st) {
+                            double *ws, const KParams &kp, const FlyK32 &k32, int32_t *err, cudaStream_t st) {
     if (nitems <= 0) return cudaSuccess;
     if (!fly_df_supported(kp, k32))
         return fly_dispatch<double>(items, nitems, ctr, rowpid, cpid, cws, kp.pts, ws, kp, FlyK32{}, st);
     const float4 *tab = reinterpret_cast<const float4 *>(logtab);
-    if (kp.dim == 3) return flydf_launch<3>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, k32, 0.5 / kp.loga, st);
-    return flydf_launch<2>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, k32, kp.c2d, st);
+    if (kp.dim == 3) return flydf_launch<3>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, k32, 0.5 / kp.loga, err, st);
+    return flydf_launch<2>(items, nitems, ctr, rowpid, cpid, cws, ptsdf, ws, tab, k32, kp.c2d, err, st);
 }
 
 // The table of fly_log: 128 bins for each of ne exponents from e0, (log c, 1 / c) as (hi, lo)
