@@ -2977,7 +2977,7 @@ void build_plan(h2w_handle *h) {
         h->plan = pbp;
         realize_single(h, h->row_split);
         realize_multi(h, h->mr_xw);
-        if (!h->fly_active) {
+        if (!h->fly_active && !h->cplx) {  // the complex kernels have products of one vector only
             SvHost mo;
             sv_build(h, h->row_split, SV_CUT_CTAS, 0, 0, 0, h->xoff(), mo, true);
             mo_upload(mo, h->mo, st);
