@@ -1856,7 +1856,7 @@ struct SvHost {
     std::vector<uint32_t> idx, cons;
     std::vector<uint2> grp;
     std::vector<int32_t> cnt;
-    std::vector<int64_t> slices;  // operator pieces to copy (slice_records)
+    std::vector<int64_t> slices;  // operator pieces to copy (launch_sv_slices; tiles: slice_records)
     std::vector<int64_t> s0;      // the slices of each target
     // the tensor-core form (mo.cu): source block lists of each part of a target's columns, its first
     // part, blocks of its written rows, block starts (the workspace's, then the input's), rows nobody writes
@@ -2075,6 +2075,7 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
         out.blocks.push_back(nr);
     }
     out.s0.assign(1, 0);
+    std::vector<int64_t> panels;
     // headers; targets of a group that read the same sources share the list of rows.
     // Every value the kernel indexes with is checked against its field.
     std::vector<uint32_t> rows, prev;
@@ -2112,6 +2113,15 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
             W += w;
         }
         if (W < 1 || W > BRG_XS_ELEMS || ws0 + blob[o] + nrows > (int64_t)UINT32_MAX) bad("target out of range");
+        bool own = false;  // the rows' own points among the sources: the diagonal
+        if (!tiles)
+            for (uint32_t r : rows) own = own || r - (uint32_t)(xoff + x0) - (d.dst - (uint32_t)ws0) < (uint32_t)nrows;
+        if (!tiles && !own) d.flags |= SV_NEIGHBOURS;
+        for (int64_t q = 0, c = 0; !tiles && q < np; ++q) {
+            const int64_t *p = out.slices.data() + 6 * (out.s0.back() + q);
+            panels.insert(panels.end(), {p[0], p[1], p[2], p[3], d.a, p[5], c, own ? -W : W});
+            c += p[3];
+        }
         out.s0.push_back(out.s0.back() + np);
         if (rows != prev) {
             if (tiles) {
@@ -2141,6 +2151,7 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
         }
         out.max_w = std::max(out.max_w, (int)W);
     }
+    if (!tiles) out.slices.swap(panels);
     pb.T = std::vector<Target>();
     pb.P = std::vector<Panel>();
     pb.S = std::vector<Seg>();
@@ -2274,7 +2285,7 @@ void copy_f64s(h2w_handle *h) {
     CK(cudaMemGetInfo(&fr, &tot));
     if (!h->copies || fr / 4 < need) return;
     h->d_op64s.alloc(need / 8);
-    CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 6, h->d_op64s.p, h->stream));
+    CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 8, h->sv.f64, h->d_op64s.p, h->stream));
 }
 
 // (Re)cut the single-vector target stream from the handle's logical targets, with the figures
@@ -3112,7 +3123,7 @@ void ensure_f32s(h2w_handle *h) {
     if (h->op32s_ready) return;
     h->d_op32s.reset();
     h->d_op32s.alloc((size_t)std::max<int64_t>(h->ops_n, 4));
-    CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 6, h->d_op32s.p, h->stream));
+    CK(launch_sv_slices(h->d_op.p, h->d_sslices.p, (int64_t)h->d_sslices.n / 8, h->sv.f32, h->d_op32s.p, h->stream));
     CK(cudaStreamSynchronize(h->stream));  // products may run on a caller's stream
     h->op32s_ready = true;
 }
@@ -4218,8 +4229,8 @@ void run_batch(h2w_batch *b, int prec, const double *x, double *y, bool leaf, co
         for (int p = 0; p < P; ++p) {
             op[(size_t)p].reset(new DBuf<float>());
             op[(size_t)p]->alloc((size_t)std::max<int64_t>(b->opn[(size_t)p], 4));
-            CK(launch_sv_slices(b->hs[(size_t)p]->d_op.p, b->slices[(size_t)p].p, (int64_t)b->slices[(size_t)p].n / 6,
-                                op[(size_t)p]->p, st));
+            CK(launch_sv_slices(b->hs[(size_t)p]->d_op.p, b->slices[(size_t)p].p, (int64_t)b->slices[(size_t)p].n / 8,
+                                b->sv.f32, op[(size_t)p]->p, st));
             tab[(size_t)p] = op[(size_t)p]->p;
         }
         b->ws32.alloc((size_t)(b->xoff + b->Ntot));
@@ -5622,8 +5633,8 @@ int h2w_batch_create(h2w_handle *const *handles, int n, h2w_batch **out) {
             for (int p = 0; p < P; ++p) {
                 b->op64.emplace_back(new DBuf<double>());
                 b->op64.back()->alloc((size_t)std::max<int64_t>(b->opn[(size_t)p], 4));
-                CK(launch_sv_slices(b->hs[(size_t)p]->d_op.p, b->slices[(size_t)p].p, (int64_t)b->slices[(size_t)p].n / 6,
-                                    b->op64.back()->p, st));
+                CK(launch_sv_slices(b->hs[(size_t)p]->d_op.p, b->slices[(size_t)p].p, (int64_t)b->slices[(size_t)p].n / 8,
+                                    b->sv.f64, b->op64.back()->p, st));
                 tab[(size_t)p] = b->op64.back()->p;
             }
             b->A64.upload(tab, st);

@@ -100,6 +100,7 @@ constexpr int SV_CTRS = 12;       // claim counters (three per launch of a produ
 // The column parts of a wide block row then multiply side by side and only add in turn (1D
 // semi-nested, parts of 4096 columns: FP64 31823 points 98 -> 73 us, FP32 65536 points 137 -> 90).
 constexpr int SV_LATE = 8;
+constexpr int SV_NEIGHBOURS = 16;  // FP64: a thread has neighbouring columns (sv_slice_kernel)
 struct alignas(16) SvHdr {
     int64_t a;
     uint32_t dst, idx0, grp, pid;
@@ -149,9 +150,11 @@ struct SvConf {
 cudaError_t sv_configure(int max_w, SvConf &f64, SvConf &f32);
 cudaError_t launch_sv(const SvArgs<double> &a, const SvConf &c, cudaStream_t st);
 cudaError_t launch_sv(const SvArgs<float> &a, const SvConf &c, cudaStream_t st);
-// the slices of an FP64 operator (as launch_slice_copy_f32) copied or converted
-cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, double *dst, cudaStream_t st);
-cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, float *dst, cudaStream_t st);
+// The targets' matrices of an FP64 operator as the launch with configuration c reads them: n panels of 8 words
+// (source offset, leading dimension, rows, columns, the matrix's offset and leading dimension, the panel's first
+// column in it, its columns in all, negative without SV_NEIGHBOURS)
+cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, const SvConf &c, double *dst, cudaStream_t st);
+cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, const SvConf &c, float *dst, cudaStream_t st);
 // Dataflow form of the FP64 product on the packed operator: the nt targets in stored order, ctr a zeroed
 // claim counter, rem the producer counts (reset before every launch), consumers in
 // cidx[coff[t] .. coff[t+1])

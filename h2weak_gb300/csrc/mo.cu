@@ -26,8 +26,9 @@
 // target and no guard it took 0.81 and 0.67 ms, but a term of 2^-k of the largest kept 62 - k bits: 1e-12 of a
 // near-field entry for a unit vector. The guard costs 3 to 9 % on vectors without structure; unit
 // vectors take up to twice as long as those.
-// What bounds it is issue slots: reading 160 accumulator columns a part out of tensor memory,
-// adding them up as integers, and forming digits.
+// What bounds it is latency: digits, MMAs and read-out (160 accumulator columns a part, added up as
+// integers) follow one another through the rings of one CTA an SM; issue slots are 36 % busy, the
+// tensor pipe 21 %, the FP64 pipe 19 % (2D, 64 vectors).
 //
 // Accumulators: digits 2p+1 and 2p+2 of eight rows each alternate in the 128 rows of an
 // MMA (A_p, p = 0 .. 4), so A_p times digit j adds weight 2p+1+j in one half of the

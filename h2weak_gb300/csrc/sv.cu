@@ -21,6 +21,15 @@
 //  * R (release): fences the written rows and decrements the producer counts
 //    of the groups that wait for them, whose list it read in advance.
 //
+// Which columns a thread adds up decides how much is lost to rounding. In FP64 a thread has neighbouring
+// ones, for terms that cancel are mostly neighbours (the matrix is stored so that the threads read neighbouring
+// vectors of it all the same, sv_slice_kernel); only the rows of a leaf's own points, whose diagonal outweighs the
+// rest and stands among the last columns, take every CG-th column, so that little is added after it. Against
+// every CG-th column everywhere, error of a product, quadratic mean over 64 vectors: 1D integral equation, 32768
+// points, 7.0e-14 and 3.5e-14 of the result (3.5e-14 in the launch by phases), 2D RBF 9973 3.5e-16 and 1.9e-16 (2.5e-16);
+// neighbouring columns everywhere: 2D integral equation 65536 2.7e-16, 1.6e-16 so. In FP32 every CG-th
+// column with SvSum does best.
+//
 // Two kinds of CTA share an SM: some take the chain of dependent passes first and
 // mostly wait, so that each pass starts at once when its producers are done; the
 // others stream the work that depends on the input alone meanwhile (SvArgs).
@@ -45,8 +54,8 @@
 // chain of dependent passes (2 L + 1, about 3 us each) for small problems.
 // Measured against one kernel whose CTAs gathered, multiplied and released a target
 // at a time: 2D integral equation, 65536 points (62e6 entries): FP64 207 -> 153 us,
-// FP32 138 -> 80; 3D semi-nested RBF, 20011 points (2e8): FP64 665 -> 471 (FP64 pipe 67 %
-// busy), FP32 330 -> 165 (5.0 TB/s); 1D RBF, 4096 points, waited for: 92 -> 75, calls on
+// FP32 138 -> 80; 3D semi-nested RBF, 20011 points (2e8): FP64 665 -> 471, FP32 330 -> 168
+// (4.8 TB/s); the FP64 pipe is 79 % busy in the 2D product; 1D RBF, 4096 points, waited for: 92 -> 75, calls on
 // several streams 69 -> 18 each.
 #include <algorithm>
 
@@ -111,6 +120,7 @@ struct SvSlot {  // one target in preparation
     uint32_t dst, idx0, grp;
     int32_t nrows, W, flags, skip;
     int32_t RQ, CG, cpc;  // row vectors, column groups of the consumer threads, columns a stage
+    int32_t per, rem, xs;  // group cg's sources: from cg per + min(cg, rem), xs apart
     uint32_t inv;         // thread / RQ = thread * inv >> 16
     int64_t vpos;         // its rows' position in the output vector (scatter targets)
 };
@@ -293,6 +303,10 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
                     sl.RQ = RQ;
                     sl.CG = CG;
                     sl.cpc = cpc;
+                    const bool near = sizeof(T) == 8 && (h.flags & SV_NEIGHBOURS);
+                    sl.per = near ? h.W / CG : 1;
+                    sl.rem = near ? h.W - sl.per * CG : 0;
+                    sl.xs = near ? 1 : CG;
                     sl.inv = (65536u + (uint32_t)RQ - 1) / (uint32_t)RQ;  // exact for thread numbers below 512
                     sl.vpos = (int64_t)h.dst - (a.vshift ? a.vshift[h.pid] : 0);
                 } else {
@@ -489,6 +503,7 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
         if (!sl.skip) {
             const int nrows = sl.nrows, W = sl.W, RQ = sl.RQ, CG = sl.CG, cpc = sl.cpc;
             const T *xs = reinterpret_cast<const T *>(src0 + sr.i * slot_b);
+            const int xstep = sizeof(T) == 8 ? sl.xs : CG;
             // thread = row slice q (VN rows, one 16-byte vector a column) x column group cg
             const int cg = (int)((uint32_t)tid * sl.inv >> 16), q = tid - cg * RQ;
             // FP32: four stages' terms (16 at most) summed apart before they go to the total. One sum of a
@@ -498,26 +513,28 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
 #pragma unroll
             for (int v = 0; v < VN; ++v) acc[v] = tot[v] = T(0);
             int done = 0;
+            const T *x0 = xs + (sizeof(T) == 8 ? cg * sl.per + min(cg, sl.rem) : cg);  // the group's sources
 #pragma unroll 1
             for (int c = 0; c < W; c += cpc) {
                 if (!sv_wait_warp(full + fr.i, fr.par, fail, a.err)) return;
                 const int nc = min(cpc, W - c);
                 if (cg < CG) {
                     const V *As = reinterpret_cast<const V *>(stages + fr.i * STAGE) + cg * RQ + q;
-                    const T *xc = xs + c + cg;
                     const int step = CG * RQ;
+                    const T *xc = sizeof(T) == 8 ? x0 : x0 + c;
                     int j = cg;
 #pragma unroll 1
-                    for (; j + 3 * CG < nc; j += 4 * CG, As += 4 * step, xc += 4 * CG) {
+                    for (; j + 3 * CG < nc; j += 4 * CG, As += 4 * step, xc += 4 * xstep) {
                         const V v0 = As[0], v1 = As[step], v2 = As[2 * step], v3 = As[3 * step];
-                        const T x0 = xc[0], x1 = xc[CG], x2 = xc[2 * CG], x3 = xc[3 * CG];
-                        sv_fma(acc, v0, x0);
-                        sv_fma(acc, v1, x1);
-                        sv_fma(acc, v2, x2);
-                        sv_fma(acc, v3, x3);
+                        const T y0 = xc[0], y1 = xc[xstep], y2 = xc[2 * xstep], y3 = xc[3 * xstep];
+                        sv_fma(acc, v0, y0);
+                        sv_fma(acc, v1, y1);
+                        sv_fma(acc, v2, y2);
+                        sv_fma(acc, v3, y3);
                     }
 #pragma unroll 1
-                    for (; j < nc; j += CG, As += step, xc += CG) sv_fma(acc, As[0], xc[0]);
+                    for (; j < nc; j += CG, As += step, xc += xstep) sv_fma(acc, As[0], xc[0]);
+                    if (sizeof(T) == 8) x0 = xc;
                 }
                 __syncwarp();
                 if (lane == 0) sv_arrive(empty + fr.i);
@@ -553,10 +570,12 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
                 if (r0 + (warp * 32 >> l) >= nrows) break;  // the same for the whole warp
                 const int r = r0 + (tid >> l);
                 SvSum<T> sum;
+                constexpr bool near = sizeof(T) == 8;  // neighbouring groups together
                 const T *p = rb + (r % VN) * CT + r / VN;
                 if (r < nrows)
 #pragma unroll 1
-                    for (int e = part; e < CG; e += 1 << l) sum.add(p[e * RQ]);
+                    for (int e = near ? part * CG >> l : part; e < (near ? (part + 1) * CG >> l : CG); e += near ? 1 : 1 << l)
+                        sum.add(p[e * RQ]);
 #pragma unroll 1
                 for (int o = 1; o < (1 << l); o <<= 1) sum.join(o);
                 if (part != 0 || r >= nrows) continue;
@@ -640,19 +659,31 @@ template <class T> cudaError_t sv_launch(const SvArgs<T> &args, const SvConf &c,
     return e;
 }
 
-// one CTA per slice, as launch_slice_copy_f32
-template <class S, class D> __global__ void sv_slice_kernel(const S *__restrict__ src, const int64_t *__restrict__ sl, D *dst) {
-    const int64_t *d = sl + 6 * (int64_t)blockIdx.x;
-    const int64_t a = d[0], lda = d[1], rows = d[2], w = d[3], o = d[4], ld = d[5];
-    for (int64_t e = threadIdx.x; e < ld * w; e += blockDim.x) {
-        const int64_t c = e / ld, r = e - c * ld;
-        dst[o + e] = r < rows ? (D)src[a + c * lda + r] : D(0);
+// One CTA per slice, a panel of a target's matrix: source offset, leading dimension, rows, columns, the matrix's
+// offset and leading dimension, the panel's first column in it, its columns in all (negative: columns stay in
+// order). In FP64 column j of the matrix goes where its consumer group reads it: groups take W / CG neighbouring
+// columns each, and position k CG + cg holds the k-th of group cg.
+template <class D> __global__ void sv_slice_kernel(const double *__restrict__ src, const int64_t *__restrict__ sl, D *dst, int ct) {
+    const int64_t *d = sl + 8 * (int64_t)blockIdx.x;
+    const int64_t a = d[0], lda = d[1], o = d[4];
+    const int rows = (int)d[2], w = (int)d[3], ld = (int)d[5], c0 = (int)d[6], W = abs((int)d[7]);
+    const bool near = sizeof(D) == 8 && d[7] > 0;
+    const int CG = ct / (ld / SvVec<D>::n), per = W / CG, rem = W - per * CG, more = rem * (per + 1);
+    for (int e = threadIdx.x; e < ld * w; e += blockDim.x) {
+        const int c = e / ld, r = e - c * ld, j = c0 + c;
+        int to = j;
+        if (near) {
+            const int cg = j < more ? j / (per + 1) : rem + (j - more) / per;
+            to = (j - cg * per - min(cg, rem)) * CG + cg;
+        }
+        dst[o + (int64_t)to * ld + r] = r < rows ? (D)src[a + (int64_t)c * lda + r] : D(0);
     }
 }
-template <class D> cudaError_t sv_slices(const double *src, const int64_t *slices, int64_t n, D *dst, cudaStream_t st) {
+template <class D>
+cudaError_t sv_slices(const double *src, const int64_t *slices, int64_t n, const SvConf &conf, D *dst, cudaStream_t st) {
     for (int64_t b = 0; b < n; b += 1 << 30) {
         const int64_t m = n - b < (1 << 30) ? n - b : 1 << 30;
-        sv_slice_kernel<double, D><<<(unsigned)m, 256, 0, st>>>(src, slices + 6 * b, dst);
+        sv_slice_kernel<D><<<(unsigned)m, 256, 0, st>>>(src, slices + 8 * b, dst, 32 * conf.cw);
         count_launch();
     }
     return cudaGetLastError();
@@ -666,11 +697,11 @@ cudaError_t sv_configure(int max_w, SvConf &f64, SvConf &f32) {
 }
 cudaError_t launch_sv(const SvArgs<double> &a, const SvConf &c, cudaStream_t st) { return sv_launch<double>(a, c, st); }
 cudaError_t launch_sv(const SvArgs<float> &a, const SvConf &c, cudaStream_t st) { return sv_launch<float>(a, c, st); }
-cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, double *dst, cudaStream_t st) {
-    return sv_slices(src, slices, n, dst, st);
+cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, const SvConf &c, double *dst, cudaStream_t st) {
+    return sv_slices(src, slices, n, c, dst, st);
 }
-cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, float *dst, cudaStream_t st) {
-    return sv_slices(src, slices, n, dst, st);
+cudaError_t launch_sv_slices(const double *src, const int64_t *slices, int64_t n, const SvConf &c, float *dst, cudaStream_t st) {
+    return sv_slices(src, slices, n, c, dst, st);
 }
 
 }  // namespace h2w
