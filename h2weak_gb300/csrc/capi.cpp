@@ -1934,10 +1934,18 @@ void group_deps(const std::vector<const PlanBuilder::LTarget *> &groups, const s
 // (an FP64 target of 16384 elements takes one SM's FP64 pipe 4 us). Large operators
 // have whole rows to spare and keep at least 8, 16 or 32 rows a target: its sources are
 // gathered once for all its rows (3D semi-nested, 2e8 entries, FP32: 262 us at 4 rows,
-// 196 at 16, 166 at 32). A block row wider than XW_CAP is cut into column parts, each
-// adding to the rows of the one before: the sums come in the same order on every run.
+// 196 at 16, 166 at 32). A wide block row is cut into column parts, each adding to the rows of the
+// one before: the sums come in the same order on every run.
 constexpr int SV_CUT_CTAS = 608;
 constexpr int64_t SV_CUT_MIN = 2048;
+// Entries below which an operator counts as small: a chain of column parts that starts late ends
+// last there, where a large one has work enough to hide it. So in a small one parts are as wide as the kernel takes
+// them and the longest chains are claimed first, in a large one they have 2048 columns, which leaves
+// room for more stages. Parts: 1D semi-nested, 31823 points, 1.6e7 entries, FP64 72 us and FP32 46 (2048 columns: 81
+// and 54); 2D semi-nested, 8.2e7, 236 and 127 at 2048 (3072: 240 and 136), 3D semi-nested, 1.9e8, 426 and 171 (432
+// and 178). Order: 1D semi-nested FP64, 9.4e6 entries, 82 -> 69 us, 2D semi-nested, 5.7e7, 240 -> 232;
+// 3D, 2e8, FP32 174 us, 187 so, 6.3e7 1770 and 1816 a solve.
+constexpr double SV_SMALL = 60e6;
 // tiles: the tensor-core form's cut, tiles of 64 rows and at most MO_XW columns.
 constexpr int64_t MO_XW = MO_MAX_W;
 void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t ws0, int64_t x0, int64_t xoff, SvHost &out,
@@ -1958,20 +1966,22 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
     pb.S.clear();
     pb.win.clear();
     pb.fused = true;
-    pb.xw_cap = tiles ? MO_XW : (int64_t)XW_CAP;
+    double all = 0;
+    for (const auto &l : pb.logical) all += elems(l);
+    const bool small = all < SV_SMALL;
+    pb.xw_cap = tiles ? MO_XW : small ? (int64_t)SV_MAX_W : 2048;
     pb.max_rows = tiles ? MR_ROWS : (int64_t)SV_MAX_ROWS;
     std::vector<const PlanBuilder::LTarget *> groups;
     std::deque<PlanBuilder::LTarget> cut;  // the column parts and what changes its flags
     struct Key { int list, hi, part; double work; int behind; };
     std::vector<Key> key;
-    double pass[3][2 * 64] = {}, all = 0;
+    double pass[3][2 * 64] = {};
     for (const auto &l : pb.logical) {
         int64_t xw = 0;
         for (const auto &p : l.panels) xw += pad4(p.w);
         if (xw == 0 || l.nrows <= 0) continue;
         const double w = elems(l);
         const int ls = list_of(l);
-        all += w;
         pass[ls][std::min(l.hi, 127)] += w;
         if (ls == 1)
             for (const auto &p : l.panels)
@@ -1990,11 +2000,9 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
             key.push_back({ls, l.hi, (int)i, w, (int)(parts.size() - 1 - i)});
         }
     }
-    // Of a deadline's targets, first parts come first. In a small operator those with the most parts
-    // behind them do: a chain of parts that starts late ends last (1D semi-nested FP64, 28385 points,
-    // 9.4e6 entries: 82 -> 69 us; 2D semi-nested, 5.7e7: 240 -> 232), where a large one has work
-    // enough to hide it (3D, 2e8 entries, FP32: 174 us, 187 so; 6.3e7: 1770 and 1816 a solve).
-    if (!tiles && all < 60e6)
+    // Of a deadline's targets, first parts come first; in a small operator those with the most parts
+    // behind them do.
+    if (!tiles && small)
         for (Key &k : key) k.part = -k.behind;
     {
         std::vector<size_t> ord(groups.size());
@@ -2112,7 +2120,7 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
             if (c != w) bad("columns without a source");
             W += w;
         }
-        if (W < 1 || W > BRG_XS_ELEMS || ws0 + blob[o] + nrows > (int64_t)UINT32_MAX) bad("target out of range");
+        if (W < 1 || W > (tiles ? (int64_t)MO_MAX_W : (int64_t)SV_MAX_W) || ws0 + blob[o] + nrows > (int64_t)UINT32_MAX) bad("target out of range");
         bool own = false;  // the rows' own points among the sources: the diagonal
         if (!tiles)
             for (uint32_t r : rows) own = own || r - (uint32_t)(xoff + x0) - (d.dst - (uint32_t)ws0) < (uint32_t)nrows;

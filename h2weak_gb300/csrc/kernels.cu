@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(BRG_THREADS, 4)
 // *err = 3 and the CTA proceeds), runs, fences its writes and decrements the counts of its
 // consumers cidx[coff[t] .. coff[t+1]). Cooperative launch: every CTA is resident, so the
 // producers of a waiting target are all claimed and running. 2D integral equation, 65536 points: 218 us,
-// 320 with grid barriers (154 on the copy); 3D semi-nested RBF, 20011 points: 667, 752 (472).
+// 320 with grid barriers (154 on the copy); 3D semi-nested RBF, 20011 points: 667, 752 (428).
 __global__ void __launch_bounds__(BRG_THREADS, 4)
     brg_flow_kernel(const int64_t *__restrict__ roff, const int64_t *__restrict__ blob, int64_t nt, int32_t *ctr,
                     int32_t *rem, const int64_t *__restrict__ coff, const int32_t *__restrict__ cidx,

@@ -99,6 +99,7 @@ constexpr int SV_CTRS = 12;       // claim counters (three per launch of a produ
 // earlier writers at its last step, not before its sources (in SvHdr::flags, beside T_ACCUM).
 // The column parts of a wide block row then multiply side by side and only add in turn (1D
 // semi-nested, parts of 4096 columns: FP64 31823 points 98 -> 73 us, FP32 65536 points 137 -> 90).
+constexpr int SV_MAX_W = 3072;  // columns of a target: two CTAs fit an SM (sv_configure)
 constexpr int SV_LATE = 8;
 constexpr int SV_NEIGHBOURS = 16;  // FP64: a thread has neighbouring columns (sv_slice_kernel)
 struct alignas(16) SvHdr {

@@ -54,7 +54,7 @@
 // chain of dependent passes (2 L + 1, about 3 us each) for small problems.
 // Measured against one kernel whose CTAs gathered, multiplied and released a target
 // at a time: 2D integral equation, 65536 points (62e6 entries): FP64 207 -> 153 us,
-// FP32 138 -> 80; 3D semi-nested RBF, 20011 points (2e8): FP64 665 -> 471, FP32 330 -> 168
+// FP32 138 -> 80; 3D semi-nested RBF, 20011 points (2e8): FP64 665 -> 428, FP32 330 -> 169
 // (4.8 TB/s); the FP64 pipe is 79 % busy in the 2D product; 1D RBF, 4096 points, waited for: 92 -> 75, calls on
 // several streams 69 -> 18 each.
 #include <algorithm>
@@ -64,12 +64,12 @@
 namespace h2w {
 namespace {
 
-// CW consumer warps: 4, or 8 or 16 where few CTAs fit an SM (wide targets)
+// CW consumer warps: 4, or 8 where few CTAs fit an SM (wide targets)
 template <int CW> struct SvDim {
     static constexpr int CT = 32 * CW;                         // consumer threads
     static constexpr int NT = CT + 128;                        // + P, two G, R
     static constexpr int STAGE = CW == 4 ? 8192 : 16384;       // bytes of one operator stage
-    static constexpr int PER_SM = CW == 4 ? 5 : CW == 8 ? 3 : 1;
+    static constexpr int PER_SM = CW == 4 ? 5 : 3;
 };
 constexpr int SV_GW = 2;                      // G warps, taking targets in turn
 constexpr int SV_MAX_SLOTS = 4, SV_MAX_STAGES = 24;
@@ -598,8 +598,10 @@ __global__ void __launch_bounds__(SvDim<CW>::NT, SvDim<CW>::PER_SM)
 // columns. Four slots when they are small, two when one holds thousands of
 // sources; as many CTAs as fit with at least three stages each (five at most: 40
 // warps), the remaining shared memory to the stages. With fewer than four CTAs an
-// SM each has 8 consumer warps instead of 4, and one alone has 16, so that the FP64
-// pipe and the shared memory always see 16 or more of them.
+// SM each has 8 consumer warps instead of 4, so that the FP64 pipe and the shared memory
+// always see 16 or more of them. SV_MAX_W columns leave room for two CTAs: one alone, with 16 warps, had
+// nothing to do while they met at the end of a target (2D semi-nested FP64, 13908 points: 165 us with
+// targets of 3535 columns, 93 with two CTAs; 3D, 13824 points: 225 and 195).
 template <class T, int CW> cudaError_t sv_configure_cw(int per, int sms, SvConf &s) {
     using Lay = SvLayout<T, CW>;
     const size_t each = (size_t)(SV_SM_BYTES / per - 1024), base = Lay::smem(s.max_w, s.nslots, 0);
@@ -619,16 +621,14 @@ template <class T, int CW> cudaError_t sv_configure_cw(int per, int sms, SvConf 
 template <class T> cudaError_t sv_configure_t(int max_w, SvConf &s) {
     s = SvConf{};
     s.max_w = (max_w + 3) & ~3;  // keeps the slots and stages 16-byte aligned
-    if (max_w < 1 || max_w > BRG_XS_ELEMS) return cudaErrorInvalidValue;
+    if (max_w < 1 || max_w > SV_MAX_W) return cudaErrorInvalidValue;
     const size_t sb = SvLayout<T, 4>::slot_bytes(s.max_w);
     s.nslots = sb <= 8192 ? 4 : sb <= 16384 ? 3 : 2;
     int dev = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    for (int per = 5; e == cudaSuccess && per >= 1 && s.ctas == 0; --per)
-        e = per >= 4   ? sv_configure_cw<T, 4>(per, sms, s)
-            : per >= 2 ? sv_configure_cw<T, 8>(per, sms, s)
-                       : sv_configure_cw<T, 16>(per, sms, s);
+    for (int per = 5; e == cudaSuccess && per >= 2 && s.ctas == 0; --per)
+        e = per >= 4 ? sv_configure_cw<T, 4>(per, sms, s) : sv_configure_cw<T, 8>(per, sms, s);
     if (e == cudaSuccess && s.ctas == 0) e = cudaErrorCooperativeLaunchTooLarge;
     return e;
 }
@@ -650,10 +650,8 @@ template <class T> cudaError_t sv_launch(const SvArgs<T> &args, const SvConf &c,
     a.na = na;
     int max_w = c.max_w, nslots = c.nslots, nst = c.nst;
     void *pv[] = {(void *)&a, (void *)&max_w, (void *)&nslots, (void *)&nst};
-    const void *f = c.cw == 4   ? (const void *)sv_flow_kernel<T, 4>
-                    : c.cw == 8 ? (const void *)sv_flow_kernel<T, 8>
-                                : (const void *)sv_flow_kernel<T, 16>;
-    const int nt = c.cw == 4 ? SvDim<4>::NT : c.cw == 8 ? SvDim<8>::NT : SvDim<16>::NT;
+    const void *f = c.cw == 4 ? (const void *)sv_flow_kernel<T, 4> : (const void *)sv_flow_kernel<T, 8>;
+    const int nt = c.cw == 4 ? SvDim<4>::NT : SvDim<8>::NT;
     const cudaError_t e = cudaLaunchCooperativeKernel(f, dim3(grid), dim3(nt), pv, c.smem, st);
     count_launch();
     return e;
