@@ -2102,6 +2102,7 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
         d.flags = (uint16_t)(fl & (T_ACCUM | T_SCATTER));
         if (!tiles && out.list[t] == 1 && d.flags == T_ACCUM) d.flags |= SV_LATE;
         rows.clear();
+        bool own = false;  // the rows' own points among the sources: the diagonal
         int64_t W = 0, e = 0;
         for (int64_t q = 0; q < np; ++q) {  // padded panel offsets become columns of the one matrix
             const int64_t w = blob[o + 4 + 3 * (size_t)q] >> 32, px = blob[o + 5 + 3 * (size_t)q];
@@ -2113,6 +2114,7 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
                 if ((code >> 1) >= px + w) break;  // the next panel's
                 if ((code >> 1) != px + c || len < 0 || c + len > w) bad("segments do not cover the columns in order");
                 const int64_t row = (code & 1) ? xoff + x0 + src : ws0 + src;
+                own = own || ((code & 1) && src < blob[o] + nrows && src + len > blob[o]);
                 if (row < 0 || row + len > (int64_t)UINT32_MAX) bad("source rows out of range");
                 for (int64_t i = 0; i < len; ++i) rows.push_back((uint32_t)(row + i));
                 c += len;
@@ -2121,9 +2123,6 @@ void sv_build(h2w_handle *h, int64_t row_split, int ctas, int32_t pid, int64_t w
             W += w;
         }
         if (W < 1 || W > (tiles ? (int64_t)MO_MAX_W : (int64_t)SV_MAX_W) || ws0 + blob[o] + nrows > (int64_t)UINT32_MAX) bad("target out of range");
-        bool own = false;  // the rows' own points among the sources: the diagonal
-        if (!tiles)
-            for (uint32_t r : rows) own = own || r - (uint32_t)(xoff + x0) - (d.dst - (uint32_t)ws0) < (uint32_t)nrows;
         if (!tiles && !own) d.flags |= SV_NEIGHBOURS;
         for (int64_t q = 0, c = 0; !tiles && q < np; ++q) {
             const int64_t *p = out.slices.data() + 6 * (out.s0.back() + q);
