@@ -53,8 +53,8 @@
 // multiply-adds a clock and SM, 5.0 TB/s of operator) for FP64 ones, and the
 // chain of dependent passes (2 L + 1, about 3 us each) for small problems.
 // Measured against one kernel whose CTAs gathered, multiplied and released a target
-// at a time: 2D integral equation, 65536 points (62e6 entries): FP64 207 -> 153 us,
-// FP32 138 -> 80; 3D semi-nested RBF, 20011 points (2e8): FP64 665 -> 428, FP32 330 -> 169
+// at a time: 2D integral equation, 65536 points (62e6 entries): FP64 207 -> 152 us,
+// FP32 138 -> 80; 3D semi-nested RBF, 20011 points (2e8): FP64 665 -> 428, FP32 330 -> 168
 // (4.8 TB/s); the FP64 pipe is 79 % busy in the 2D product; 1D RBF, 4096 points, waited for: 92 -> 75, calls on
 // several streams 69 -> 18 each.
 #include <algorithm>
